@@ -90,7 +90,6 @@ struct Level {
   // (the reference's coarse solve), row-major, and lu_free, the inverse of the
   // unpinned matrix used inside FGMRES unless it was singular (device flag)
   DBuf<double> lu, lu_free;
-  DBuf<int> piv;                   // two permutations of n
 };
 
 // Solver state of the device-driven FGMRES (amg_cycle.cu), read by the host
@@ -181,6 +180,8 @@ struct AMG {
 void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const double* val,
                cudaStream_t s);
 void amg_update(AMG& h, const double* val, cudaStream_t s);
+// amg_dense.cu: inverses of the coarsest matrix (n <= 500), pinned and unpinned
+void coarse_factor(AMG& h, Level& L, cudaStream_t s, bool from_fp32 = false);
 // amg_cycle.cu
 void amg_vcycle(AMG& h, int lvl, bool zero_x, int precision, cudaStream_t s);
 void amg_solve_vcycles(AMG& h, const double* b, double* x, double tol, int max_cycles,
@@ -200,7 +201,6 @@ void amg_fgmres_capture(AMG& h, const double* b, double* x, const impes_krylov_p
 // shared kernels (amg_cycle.cu)
 void spmv(const Level& L, const double* x, double* y, cudaStream_t s);
 double dot_host(AMG& h, const double* a, const double* b, int n, cudaStream_t s);
-void coarse_factor(AMG& h, Level& L, cudaStream_t s, bool from_fp32 = false);
 // Times the CSR kernels of every level with each lanes-per-row choice and keeps
 // the fastest (amg_cycle.cu); choices are cached per level shape for the process.
 void amg_autotune(AMG& h, cudaStream_t s);

@@ -1019,182 +1019,6 @@ __global__ void k_scale_by_inv_sqrt(long long n, const double* in, double* out, 
 }
 
 // --------------------------------------------------- coarsest dense solve
-// Dense copy of the coarsest matrix with DOF 0 pinned (classical_amg.py:1045-1055).
-__global__ void k_dense_pinned(int n, const int* rowptr, const int* col, const double* val, double* M) {
-  GRID_LOOP(t, (long long)n * n) M[t] = 0.0;
-}
-template <typename TV>
-__global__ void k_dense_fill(int n, const int* rowptr, const int* col, const TV* val, double* M,
-                             int pin) {
-  GRID_LOOP(i, n) {
-    for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
-      int j = col[e];
-      if (pin && (i == 0 || j == 0)) continue;
-      M[(long long)i * n + j] = val[e];
-    }
-    if (pin && i == 0) M[0] = 1.0;
-  }
-}
-// In-place Gauss-Jordan inversion with partial pivoting: block b inverts M[b]
-// (the pinned and the unpinned coarsest matrix in one launch).  With SMEM the
-// n x n matrix lives in shared memory for the whole elimination (n <= 168 in
-// 227 KB); otherwise it stays in global memory.  Pivot ties go to the lower row.
-constexpr int kGJ = 1024;
-struct GJArgs {
-  double* M[2];
-  int* perm[2];
-  int* singular[2];
-};
-template <bool SMEM, int NT = kGJ>
-__global__ void __launch_bounds__(NT) k_gauss_jordan(int n, GJArgs args) {
-  __shared__ double s_val[NT / 32];
-  __shared__ int s_idx[NT / 32];
-  __shared__ int s_p;
-  __shared__ double s_inv;
-  __shared__ int s_perm[512];        // row interchanges (n <= 500), kept on chip
-  extern __shared__ double s_dyn[];
-  double* s_row = s_dyn;             // n (pivot row)
-  double* s_col = s_row + n;         // n (pivot column)
-  double* G = args.M[blockIdx.x];
-  int* perm = args.perm[blockIdx.x];
-  double* M = SMEM ? s_col + n : G;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (SMEM) {
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) M[t] = G[t];
-    __syncthreads();
-  }
-  for (int k = 0; k < n; ++k) {
-    double best = -1.0;
-    int bi = k;
-    for (int i = k + threadIdx.x; i < n; i += blockDim.x) {
-      const double v = fabs(M[i * n + k]);
-      if (v > best) { best = v; bi = i; }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ov = __shfl_down_sync(0xffffffffu, best, o);
-      const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    if (lane == 0) { s_val[warp] = best; s_idx[warp] = bi; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double bv = -1.0;
-      int b = k;
-      for (int w = 0; w < nw; ++w)
-        if (s_val[w] > bv || (s_val[w] == bv && s_idx[w] < b)) { bv = s_val[w]; b = s_idx[w]; }
-      s_p = b;
-      s_perm[k] = b;
-      if (!(bv > 0.0)) *args.singular[blockIdx.x] = 1;
-      const double piv = M[b * n + k];
-      s_inv = piv != 0.0 ? 1.0 / piv : 0.0;
-    }
-    __syncthreads();
-    const int p = s_p;
-    const double inv = s_inv;
-    // swap rows k and p, scale the pivot row, keep it and the pivot column
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-      const double rk = M[k * n + j], rp = M[p * n + j];
-      if (p != k) M[p * n + j] = rk;
-      const double v = (j == k) ? inv : rp * inv;
-      M[k * n + j] = v;
-      s_row[j] = v;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) s_col[i] = M[i * n + k];
-    __syncthreads();
-    for (int i = warp; i < n; i += nw) {
-      if (i == k) continue;
-      const double f = s_col[i];
-      for (int j = lane; j < n; j += 32) {
-        if (j == k) M[i * n + j] = -f * s_row[k];
-        else M[i * n + j] -= f * s_row[j];
-      }
-    }
-    __syncthreads();
-  }
-  // undo the row interchanges as column interchanges, last first
-  for (int k = threadIdx.x; k < n; k += blockDim.x) perm[k] = s_perm[k];
-  for (int k = n - 1; k >= 0; --k) {
-    const int p = s_perm[k];
-    if (p != k)
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double a = M[i * n + k];
-        M[i * n + k] = M[i * n + p];
-        M[i * n + p] = a;
-      }
-    __syncthreads();
-  }
-  if (SMEM)
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) G[t] = M[t];
-}
-// k_gauss_jordan for n <= kGJPingPong with one block barrier per pivot step:
-// every warp finds the pivot itself (column k of the previous matrix, same rule:
-// largest |value|, ties to the lower row) and step k writes a second copy of
-// the matrix from the first (rows k and p swapped, the pivot row scaled, the
-// others updated), so no row is read after it is rewritten.  Each element gets
-// the same operations in the same order as in k_gauss_jordan.
-constexpr int kGJPingPong = 64;
-__global__ void __launch_bounds__(256) k_gauss_jordan_pp(int n, GJArgs args) {
-  extern __shared__ double s_dyn[];
-  __shared__ int s_perm[kGJPingPong];
-  double* A = s_dyn;                 // n x n, even steps read here
-  double* B = A + (size_t)n * n;     // n x n, odd steps read here
-  double* G = args.M[blockIdx.x];
-  int* perm = args.perm[blockIdx.x];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int t = threadIdx.x; t < n * n; t += blockDim.x) A[t] = G[t];
-  __syncthreads();
-  bool singular = false;
-  for (int k = 0; k < n; ++k) {
-    const double* M = (k & 1) ? B : A;
-    double* W = (k & 1) ? A : B;
-    double best = -1.0;
-    int bi = k;
-    for (int i = k + lane; i < n; i += 32) {
-      const double v = fabs(M[i * n + k]);
-      if (v > best) { best = v; bi = i; }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ov = __shfl_down_sync(0xffffffffu, best, o);
-      const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    const int p = __shfl_sync(0xffffffffu, bi, 0);
-    best = __shfl_sync(0xffffffffu, best, 0);
-    if (!(best > 0.0)) singular = true;
-    if (threadIdx.x == 0) s_perm[k] = p;
-    const double piv = M[p * n + k];
-    const double inv = piv != 0.0 ? 1.0 / piv : 0.0;
-    for (int i = warp; i < n; i += nw) {
-      // row i of the swapped matrix: old row p at k, old row k at p
-      const int src = (i == k) ? p : (i == p ? k : i);
-      if (i == k) {
-        for (int j = lane; j < n; j += 32) W[k * n + j] = (j == k) ? inv : M[p * n + j] * inv;
-      } else {
-        const double f = M[src * n + k];
-        for (int j = lane; j < n; j += 32) {
-          const double sr = (j == k) ? inv : M[p * n + j] * inv;
-          W[i * n + j] = (j == k) ? -f * sr : M[src * n + j] - f * sr;
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (singular && threadIdx.x == 0) *args.singular[blockIdx.x] = 1;
-  double* M = (n & 1) ? B : A;       // the last step wrote here
-  for (int k = threadIdx.x; k < n; k += blockDim.x) perm[k] = s_perm[k];
-  for (int k = n - 1; k >= 0; --k) {
-    const int p = s_perm[k];
-    if (p != k)
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double a = M[i * n + k];
-        M[i * n + k] = M[i * n + p];
-        M[i * n + p] = a;
-      }
-    __syncthreads();
-  }
-  for (int t = threadIdx.x; t < n * n; t += blockDim.x) G[t] = M[t];
-}
 // x = Ainv * b with b[0] pinned to 0 (the reference's coarsest solve), or, in
 // Krylov mode while the unpinned matrix was invertible, x = Afree^-1 * b.
 template <typename T>
@@ -1229,45 +1053,6 @@ bool amg_level_tiled(const AMG& h, int l, int slot) {
 }
 
 // =================================================================== host
-void coarse_factor(AMG& h, Level& L, cudaStream_t s, bool from_fp32) {
-  if (L.n > 500 || L.n == 0) return;
-  const int n = L.n;
-  // the reference's pinned matrix (row/column 0 replaced by e_0) and the
-  // unpinned one used inside FGMRES (the pinned solve would freeze x[0] there)
-  L.lu.ensure((size_t)n * n);
-  L.lu_free.ensure((size_t)n * n);
-  L.piv.ensure(2 * (size_t)n);
-  double* mats[2] = {L.lu.p, L.lu_free.p};
-  for (int q = 0; q < 2; ++q) {
-    k_dense_pinned<<<grid_for((size_t)n * n, TB), TB, 0, s>>>(n, L.rowptr.p, L.col.p, L.val.p, mats[q]); ::impes::count_launch();
-    if (from_fp32) {
-      k_dense_fill<float><<<grid_for(n, TB), TB, 0, s>>>(n, L.rowptr.p, L.col.p, L.valf.p, mats[q], q == 0 ? 1 : 0); ::impes::count_launch();
-    } else {
-      k_dense_fill<double><<<grid_for(n, TB), TB, 0, s>>>(n, L.rowptr.p, L.col.p, L.val.p, mats[q], q == 0 ? 1 : 0); ::impes::count_launch();
-    }
-  }
-  IMPES_CHECK_LAUNCH();
-  IMPES_CUDA(cudaMemsetAsync(h.iflag.p + 2, 0, 2 * sizeof(int), s));
-  GJArgs args{{L.lu.p, L.lu_free.p}, {L.piv.p, L.piv.p + n}, {h.iflag.p + 2, h.iflag.p + 3}};
-  const size_t smem_full = sizeof(double) * ((size_t)n * n + 2 * (size_t)n);
-  if (n <= kGJPingPong) {
-    const size_t smem_pp = sizeof(double) * 2 * (size_t)n * n;
-    raise_smem_limit((const void*)k_gauss_jordan_pp, smem_pp);
-    k_gauss_jordan_pp<<<2, 256, smem_pp, s>>>(n, args); ::impes::count_launch();
-  } else if (n <= 128) {
-    // small coarsest matrices: 8 warps keep each of the n pivot steps' block
-    // barriers short (the elimination has at most 128 rows to share out)
-    raise_smem_limit((const void*)k_gauss_jordan<true, 256>, smem_full);
-    k_gauss_jordan<true, 256><<<2, 256, smem_full, s>>>(n, args); ::impes::count_launch();
-  } else if (smem_full <= (size_t)(224u << 10)) {
-    raise_smem_limit((const void*)k_gauss_jordan<true>, smem_full);
-    k_gauss_jordan<true><<<2, kGJ, smem_full, s>>>(n, args); ::impes::count_launch();
-  } else {
-    k_gauss_jordan<false><<<2, kGJ, 2 * n * sizeof(double), s>>>(n, args); ::impes::count_launch();
-  }
-  IMPES_CHECK_LAUNCH();
-}
-
 void spmv(const Level& L, const double* x, double* y, cudaStream_t s) {
   launch_csr<double, Y_AX>(L.n, L.avg_row, L.rowptr.p, L.col.p, L.val.p, x, nullptr, nullptr, y, s);
 }

@@ -27,6 +27,7 @@ SOURCES = {
     "physics.cu": ["-fmad=false"],
     "amg_setup.cu": [],
     "amg_cycle.cu": [],
+    "amg_dense.cu": [],
     "adjoint.cu": [],
     "ensemble.cu": [],
     "pcg.cu": [],
