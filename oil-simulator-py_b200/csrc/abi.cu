@@ -177,9 +177,11 @@ bool step_graph_run(Model& m, AMG& a, double* p, double* sw, double* sg, double*
       cudaGetLastError();
       count_launches(-(long long)(thread_launches() - before));
       a.fp64_stale = stale_before;
+      a.dense_invalidate();
       a.step_graph_failed = true;
       return false;
     }
+    a.dense_invalidate();                      // captured, not run
     IMPES_CUDA(cudaStreamEndCapture(cs, &graph));
     AMG::StepGraph e;
     e.model = &m; e.p = p; e.sw = sw; e.sg = sg; e.so = so; e.dt = dt;
@@ -205,6 +207,8 @@ bool step_graph_run(Model& m, AMG& a, double* p, double* sw, double* sg, double*
   }
   IMPES_CUDA(cudaGraphLaunch(g->exec, s));
   a.fp64_stale = g->fp64_stale_after;
+  a.dense_invalidate();
+  a.dense_valid[kp.precision == 1 ? 1 : 0][1] = a.dense_level >= 0;
   FgState* hs = reinterpret_cast<FgState*>(a.hbuf.p);
   static_assert(sizeof(FgState) <= 64 * sizeof(double), "state must fit the pinned scratch");
   IMPES_CUDA(cudaMemcpyAsync(hs, a.fgst.p, sizeof(FgState), cudaMemcpyDeviceToHost, s));

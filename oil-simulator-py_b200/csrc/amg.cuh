@@ -153,6 +153,14 @@ struct AMG {
   bool use_step_graph = true;           // whole IMPES steps as graphs (IMPES_NO_STEP_GRAPH=1: off)
   bool use_tail = false;                // fused V-cycle tail (IMPES_TAIL=1: on)
   bool use_dia_tile = false;            // level-0 grid-tile sweeps (IMPES_DIA_TILE=1: on)
+  // The V-cycle of levels dense_level and below as one dense operator (row-major,
+  // leading dimension dense_ld), per [fp32 values][Krylov mode]; valid while the
+  // values it was formed from are the hierarchy's (amg_dense.cu)
+  int dense_level = -1;                 // -1: none
+  int dense_ld = 0;
+  DBuf<double> dense_op[2][2], dense_work;
+  bool dense_valid[2][2] = {{false, false}, {false, false}};
+  void dense_invalidate() { for (auto& a : dense_valid) a[0] = a[1] = false; }
   int tail_level = -1;                  // first level of the fused tail, -1: none
   int tail_cluster = 0;                 // CTAs in the tail's cluster (16 or 8)
   int stail_level = -1;                 // first level of the shared-memory fp32 tail, -1: none
@@ -182,6 +190,12 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
 void amg_update(AMG& h, const double* val, cudaStream_t s);
 // amg_dense.cu: inverses of the coarsest matrix (n <= 500), pinned and unpinned
 void coarse_factor(AMG& h, Level& L, cudaStream_t s, bool from_fp32 = false);
+// The coarse V-cycle's dense operator: which levels (after the tails were chosen),
+// forming it from the current values, and x = Op b on level h.dense_level.
+void amg_dense_setup(AMG& h);
+void amg_dense_form(AMG& h, int slot, bool krylov, cudaStream_t s);
+template <typename T>
+void dense_apply(const AMG& h, bool krylov, const T* b, T* x, cudaStream_t s);
 // amg_cycle.cu
 void amg_vcycle(AMG& h, int lvl, bool zero_x, int precision, cudaStream_t s);
 void amg_solve_vcycles(AMG& h, const double* b, double* x, double tol, int max_cycles,

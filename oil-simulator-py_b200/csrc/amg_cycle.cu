@@ -1202,6 +1202,10 @@ double vcycle_bytes(const AMG& h, int l) {
   double tot = 0.0;
   for (size_t q = l; q < h.levels.size(); ++q) {
     const Level& L = *h.levels[q];
+    if ((int)q == h.dense_level) {
+      tot += 8.0 * L.n * (double)L.n + 2.0 * sz * L.n;
+      break;
+    }
     if (L.coarsest) {
       tot += L.n <= 500 ? 8.0 * L.n * (double)L.n + 2.0 * sz * L.n : 50.0 * sweep_bytes(sz, L.nnz, L.n);
       break;
@@ -1681,6 +1685,10 @@ T* vcycle(AMG& h, int l, bool zero_x, cudaStream_t s, bool first_sweep_done = fa
       return LV<T>::x(L);
     }
   }
+  if (l > 0 && zero_x && l == h.dense_level) {
+    dense_apply<T>(h, h.krylov_mode, LV<T>::b(L), LV<T>::x(L), s);
+    return LV<T>::x(L);
+  }
   if (L.coarsest) {
     if (L.n <= 500) {
       const int n = L.n;
@@ -1727,7 +1735,7 @@ T* vcycle(AMG& h, int l, bool zero_x, cudaStream_t s, bool first_sweep_done = fa
   if (!tiled) launch_a<T, Y_B_MINUS_AX>(L, LV<T>::slot, x, LV<T>::b(L), nullptr, LV<T>::r(L), s);
   // the restriction also takes the coarse level's first sweep from zero when
   // that level smooths with l1-Jacobi through the per-level kernels
-  const bool fuse_s0 = !Nc.coarsest && L.r_avg <= 96 && !(l + 1 == h.tail_level) &&
+  const bool fuse_s0 = !Nc.coarsest && L.r_avg <= 96 && !(l + 1 == h.tail_level) && l + 1 != h.dense_level &&
                        !(sizeof(T) == 4 && l + 1 == h.stail_level) &&
                        !(h.prm.smoother == IMPES_SMOOTHER_CHEBYSHEV && Nc.cheb_lmax.p);
   if (fuse_s0) {
@@ -1752,10 +1760,17 @@ T* vcycle(AMG& h, int l, bool zero_x, cudaStream_t s, bool first_sweep_done = fa
   return out;
 }
 
+// Forms the coarse levels' dense operator where the values changed since.
+template <typename T>
+void dense_ensure(AMG& h, cudaStream_t s) {
+  if (h.dense_level >= 0 && !h.dense_valid[LV<T>::slot][h.krylov_mode]) amg_dense_form(h, LV<T>::slot, h.krylov_mode, s);
+}
+
 // One V-cycle from level 0 (input in LV<T>::b(L0), initial iterate in
 // LV<T>::x(L0) unless zero_x), replayed from a CUDA graph captured on first use.
 template <typename T>
 T* vcycle_top(AMG& h, bool zero_x, cudaStream_t s) {
+  dense_ensure<T>(h, s);
   if (!h.use_graphs) return vcycle<T>(h, 0, zero_x, s);
   PhaseTimers& tm = timers();
   AMG::VGraph& g = h.vgraph[sizeof(T) == 4][zero_x][h.krylov_mode][tm.on];
@@ -2907,6 +2922,8 @@ void amg_fgmres_prepare(AMG& h, const impes_krylov_params& kp) {
 
 void amg_fgmres_capture(AMG& h, const double* b, double* x, const impes_krylov_params& kp, cudaStream_t s) {
   KrylovModeGuard guard(h);
+  // part of the captured work: every replay follows an update of the values
+  amg_dense_form(h, kp.precision == 1 ? 1 : 0, true, s);
   Level& L0 = *h.levels[0];
   const long long n = L0.n;
   const int m = h.krylov_m;
@@ -3109,6 +3126,7 @@ void solve_vcycles_noalloc(AMG& h, const double* b, double* x, double tol, int m
   double* bs = base;
   double* r = base + kNoAllocMaxRows;
   double* wb = base + 2 * (size_t)kNoAllocMaxRows;
+  dense_ensure<double>(h, s);
   launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.dhalf_inv.p, b, bs);
   IMPES_CHECK_LAUNCH();
   const bool jac = norm == IMPES_NORM_JACOBI;

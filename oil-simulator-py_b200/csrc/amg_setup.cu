@@ -1524,6 +1524,8 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
     h.use_dia_tile = eg && eg[0] == '1';
   }
   h.levels.clear();
+  h.dense_level = -1;
+  h.dense_invalidate();
   h.built = false;
   h.fp64_stale = false;
   h.iflag.ensure(8);
@@ -1799,6 +1801,7 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
     }
   }
   h.tail_level = amg_tail_level(h);
+  amg_dense_setup(h);
   h.built = true;
 }
 
@@ -1876,6 +1879,7 @@ void amg_update(AMG& h, const double* val, cudaStream_t s) {
     bytes += 12.0 * L.nnz + 24.0 * L.pnnz + 8.0 * h.levels[l + 1]->nnz;
     if (!L.coarsest && !L.planned) all_planned = false;
   }
+  h.dense_invalidate();
   equilibrate_level0(h, val, s);
   if (h.prm.mixed_precision && all_planned && h.levels.size() > 1) {
     update_fp32_chain(h, s);

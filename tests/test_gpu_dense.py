@@ -40,3 +40,75 @@ def test_coarsest_inverse(n):
         # the unpinned inverse is an exact preconditioner of the whole system
         xs, st = amg.fgmres(torch.from_numpy(b).cuda(), tol=1e-10, norm="equilibrated")
         assert st["converged"] and st["iterations"] <= 2
+
+
+def _plain_vcycle(levels, l, b, light_rows):
+    """The V-cycle from zero on level l in numpy, from the exported levels."""
+    L = levels[l]
+    A, n = L["A"], L["n"]
+    w = 0.7 * L["inv"]
+    if L["is_coarsest"]:
+        bp = b.copy()
+        bp[0] = 0.0
+        if n <= 500:
+            P = A.copy()
+            P[0, :] = 0.0
+            P[:, 0] = 0.0
+            P[0, 0] = 1.0
+            return np.linalg.solve(P, bp)
+        x = np.zeros(n)
+        for _ in range(50):
+            x = x + w * (bp - A @ x)
+        return x
+    light = n <= light_rows
+    x = np.zeros(n)
+    for _ in range(1 if light else 3):
+        x = x + w * (b - A @ x)
+    x = x + L["P"] @ _plain_vcycle(levels, l + 1, L["P"].T @ (b - A @ x), light_rows)
+    for _ in range(1 if light else 2):
+        x = x + w * (b - A @ x)
+    return x
+
+
+def _export(amg):
+    out = []
+    for L in amg.levels:
+        out.append({"A": L["A"].to_dense().cpu().numpy(), "n": L["n"], "is_coarsest": L["is_coarsest"],
+                    "inv": L["inv_relax"].cpu().numpy(),
+                    "P": None if L["P"] is None else L["P"].to_dense().cpu().numpy()})
+    return out
+
+
+# short rows (sparse products), long rows (dense products), one sweep a side on the coarse levels, a capped
+# interpolation, and a coarsest level of more than 500 rows (fifty sweeps)
+@pytest.mark.parametrize("dims,kw", [((45, 45, 1), {}), ((15, 13, 11), {}), ((15, 13, 11), {"light_sweep_rows": 2000}),
+                                     ((16, 16, 9), {"p_max_elements": 2}), ((17, 15, 11), {"max_levels": 2}),
+                                     ((40, 44, 1), {"max_levels": 1})])
+def test_coarse_operator_vcycle(dims, kw):
+    from impes_b200 import scenarios
+    from impes_b200.amg import ClassicalAMG
+    from impes_b200.simulator import build_from_config
+    cfg, f = scenarios.two_phase_2d(seed=5, nx=dims[0], ny=dims[1], nz=dims[2])
+    cfg["wells"] = cfg["wells"][:1]
+    _, _, _, sim = build_from_config(cfg, f)
+    rowptr, col, val, _ = sim.assemble(86400.0)
+    n = dims[0] * dims[1] * dims[2]
+    amg = ClassicalAMG((rowptr, col, val, (n, n)), coarsest_size=60, mixed_precision=True, **kw)
+    rng = np.random.default_rng(3)
+    b = rng.standard_normal(n)
+    bt = torch.from_numpy(b).cuda()
+    for scale in (1.0, 1.7):       # the operator follows the values
+        if scale != 1.0:
+            d = torch.linspace(1.0, scale, val.numel(), dtype=torch.float64, device=val.device)
+            sym = 0.5 * (d + d.mean())          # keeps the matrix an M-matrix
+            amg.update_values(val * sym)
+        x64 = amg.vcycle_scaled(bt, precision="fp64").cpu().numpy()
+        x32 = amg.vcycle_scaled(bt, precision="mixed").cpu().numpy()
+        levels = _export(amg)
+        ref = _plain_vcycle(levels, 0, b, kw.get("light_sweep_rows", 0))
+        # the coarsest solve's rounding (n eps cond of a scaled matrix of at most ~1e5) bounds the first
+        assert np.linalg.norm(x64 - ref) <= 1e-9 * np.linalg.norm(ref)
+        # fp32 level values: eps32 times the same condition on the coarsest level
+        assert np.linalg.norm(x32 - ref) <= 2e-2 * np.linalg.norm(ref)
+        x, st = amg.fgmres(bt, tol=1e-10, precision="mixed", max_iters=400)
+        assert st["converged"]
