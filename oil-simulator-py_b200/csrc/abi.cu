@@ -189,9 +189,8 @@ bool step_graph_run(Model& m, AMG& a, double* p, double* sw, double* sg, double*
     e.have_prev2 = quad; e.dt_prev2 = quad ? m.dt_prev2 : 0.0;
     e.fp64_stale_after = a.fp64_stale;
     e.kernels_body = a.fg_body_kernels;
-    e.kernels_reorth = a.fg_reorth_kernels;
     e.kernels_end = a.fg_end_kernels;
-    e.kernels_fixed = (long long)(thread_launches() - before) - e.kernels_body - e.kernels_reorth - e.kernels_end;
+    e.kernels_fixed = (long long)(thread_launches() - before) - e.kernels_body - e.kernels_end;
     count_launches(-(long long)(thread_launches() - before));
     a.fp64_stale = stale_before;
     cudaError_t ie = cudaGraphInstantiate(&e.exec, graph, 0);
@@ -213,8 +212,7 @@ bool step_graph_run(Model& m, AMG& a, double* p, double* sw, double* sg, double*
   static_assert(sizeof(FgState) <= 64 * sizeof(double), "state must fit the pinned scratch");
   IMPES_CUDA(cudaMemcpyAsync(hs, a.fgst.p, sizeof(FgState), cudaMemcpyDeviceToHost, s));
   IMPES_CUDA(cudaStreamSynchronize(s));
-  count_launches(g->kernels_fixed + (long long)hs->total * g->kernels_body + (long long)hs->reorths * g->kernels_reorth +
-                 (long long)hs->restarts * g->kernels_end);
+  count_launches(g->kernels_fixed + (long long)hs->total * g->kernels_body + (long long)hs->restarts * g->kernels_end);
   st = impes_krylov_stats{hs->total, hs->restarts, hs->converged && !hs->nan ? 1 : 0, hs->rel, hs->true_rel};
   if (hs->nan) throw Error(IMPES_ERR_NAN, "NaN in FGMRES");
   if (!st.converged) return true;            // p was restored by the graph

@@ -95,7 +95,7 @@ struct Level {
 // Solver state of the device-driven FGMRES (amg_cycle.cu), read by the host
 // after the captured solve has run.
 struct FgState {
-  int j, total, restarts, converged, done, cycle_end, reorth, bzero, nan;
+  int j, total, restarts, converged, done, reorth, bzero, nan;
   int reorths;                          // second Gram-Schmidt passes taken
   int gs_count;                         // blocks of a Gram-Schmidt launch done (last block reduces)
   double bnorm, beta, wn2, rel, true_rel;
@@ -130,12 +130,11 @@ struct AMG {
   };
   VGraph vgraph[2][2][2][2];
   cudaStream_t cap_stream = nullptr;
-  cudaStream_t body_stream = nullptr;   // captures the device FGMRES's loop body
-  cudaStream_t if_stream = nullptr;     // captures the IF blocks inside that body
+  cudaStream_t body_stream = nullptr;   // captures a cycle of the device FGMRES
+  cudaStream_t inner_stream = nullptr;  // captures an iteration inside it
   DBuf<FgState> fgst;                   // device FGMRES state
   long long fg_body_kernels = 0;        // kernels of one device-FGMRES iteration
-  long long fg_reorth_kernels = 0;      // ... of its second Gram-Schmidt pass (IF node)
-  long long fg_end_kernels = 0;         // ... of its cycle-end block (IF node)
+  long long fg_end_kernels = 0;         // ... of a cycle's start and end
   // whole IMPES steps captured as graphs (abi.cu), keyed by the step's inputs
   struct StepGraph {
     cudaGraphExec_t exec = nullptr;
@@ -145,7 +144,7 @@ struct AMG {
     bool have_prev = false, have_prev2 = false;
     impes_krylov_params kp{};
     bool fp64_stale_after = false;
-    long long kernels_fixed = 0, kernels_body = 0, kernels_reorth = 0, kernels_end = 0;
+    long long kernels_fixed = 0, kernels_body = 0, kernels_end = 0;
   };
   std::vector<StepGraph> step_graphs;
   bool step_graph_failed = false;       // capture refused once: keep the host-driven path
@@ -180,7 +179,7 @@ struct AMG {
     drop_graphs();
     if (cap_stream) cudaStreamDestroy(cap_stream);
     if (body_stream) cudaStreamDestroy(body_stream);
-    if (if_stream) cudaStreamDestroy(if_stream);
+    if (inner_stream) cudaStreamDestroy(inner_stream);
   }
 };
 

@@ -16,6 +16,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 
 // handle accessors (abi.cu)
 bool impes_amg_handle_built(impes_amg* h);
@@ -2464,20 +2465,25 @@ void amg_fgmres(AMG& h, const double* b, double* x, const impes_krylov_params& k
 // The FGMRES above with its control on the device, for capture into a CUDA
 // graph: the iteration count, the Arnoldi index j, the convergence test and
 // the restart decision live in FgState, every kernel reads j from there, and a
-// conditional WHILE node repeats the iteration body until the last kernel of
-// an iteration clears the node's condition.  One body pass is one iteration
-// (preconditioner application, operator product, Gram-Schmidt with the
-// optional second pass, Givens rotation); at the end of a cycle (converged,
-// j == restart or the iteration cap) the same pass also back-solves, updates
+// two conditional WHILE nodes, one inside the other, hold the loops: a pass of
+// the inner one is one iteration (preconditioner application, operator product,
+// Gram-Schmidt with the optional second pass, Givens rotation) and its last
+// kernel ends it at the end of a cycle (converged, j == restart or the iteration
+// cap), after back-solving; a pass of the outer one is a cycle, which updates
 // x_s and recomputes the true residual, which decides whether to stop or to
-// restart.  Same arithmetic and order as amg_fgmres; no host synchronisation
-// until the caller reads the state after the graph.
+// restart.  The algorithm of amg_fgmres; no host synchronisation until the
+// caller reads the state after the graph.
 namespace {
 __global__ void k_fg_init(FgState* st, const double* part_b, const double* part_r, int nb, double tol,
                           int max_iters, int m1, double* g, cudaGraphConditionalHandle cond) {
   pdl_wait_release();
   double b2 = 0.0, r2 = 0.0;
-  for (int q = 0; q < nb; ++q) { b2 += part_b[q]; r2 += part_r[q]; }
+  for (int q = threadIdx.x; q < nb; q += 32) { b2 += part_b[q]; r2 += part_r[q]; }
+  b2 = warp_sum(b2);
+  r2 = warp_sum(r2);
+  for (int i = threadIdx.x; i < m1; i += 32) g[i] = 0.0;
+  __syncwarp();
+  if (threadIdx.x != 0) return;
   FgState t{};
   t.bnorm = sqrt(b2);
   t.beta = sqrt(r2);
@@ -2488,26 +2494,24 @@ __global__ void k_fg_init(FgState* st, const double* part_b, const double* part_
   t.converged = t.bzero || t.rel < tol;
   t.done = t.bzero || t.nan || t.rel < tol || max_iters <= 0;
   *st = t;
-  for (int i = 0; i < m1; ++i) g[i] = 0.0;
   g[0] = t.beta;
   cudaGraphSetConditional(cond, t.done ? 0u : 1u);
 }
-// V[0] /= beta while the solve goes on (after k_fg_init or a restart)
-__global__ void k_fg_scale_v0(long long n, double* V, const FgState* st, int after_restart) {
+// a cycle's start: V[0] /= beta, and the inner loop runs
+__global__ void k_fg_scale_v0(long long n, double* V, const FgState* st, cudaGraphConditionalHandle inner) {
   pdl_wait_release();
-  if (st->done || (after_restart && !st->cycle_end)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(inner, 1u);
   const double inv = 1.0 / st->beta;
   GRID_LOOP(i, n) V[i] *= inv;
 }
-// preconditioner input: V[j] ./ wt in the V-cycle's precision; a new pass
-// clears the cycle-end flag of the previous one
+// preconditioner input: V[j] ./ wt in the V-cycle's precision
 template <typename T>
 __global__ void k_fg_prec_in(long long n, double* __restrict__ V, const double* __restrict__ wt,
-                             T* __restrict__ out, FgState* st) {
+                             T* __restrict__ out, const FgState* st) {
   pdl_wait_release();
   const long long j = st->j;
   // V[j] (j > 0) still holds the orthogonalised w of the last iteration: it is
-  // normalised here, times 1 / ||w|| (||w||^2 from k_fg_update), and written back
+  // normalised here, times 1 / ||w|| (||w||^2 from k_fg_gs), and written back
   const bool sc = j > 0;
   const double inv = sc ? 1.0 / sqrt(st->wn2) : 1.0;
   GRID_LOOP(i, n) {
@@ -2518,13 +2522,13 @@ __global__ void k_fg_prec_in(long long n, double* __restrict__ V, const double* 
     }
     out[i] = (T)(v / wt[i]);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->cycle_end = 0;
 }
 // k_fg_prec_in fused with the V-cycle's first level-0 sweep from zero
 // (Y_SMOOTH0, same arithmetic): b = V[j] ./ wt and x = w inv b
 template <typename T>
 __global__ void k_fg_prec_smooth0(long long n, double* __restrict__ V, const double* __restrict__ wt,
-                                  const T* __restrict__ inv, T* __restrict__ b, T* __restrict__ x, FgState* st) {
+                                  const T* __restrict__ inv, T* __restrict__ b, T* __restrict__ x,
+                                  const FgState* st) {
   pdl_wait_release();
   const long long j = st->j;
   const bool sc = j > 0;   // normalise V[j] as k_fg_prec_in does
@@ -2539,7 +2543,6 @@ __global__ void k_fg_prec_smooth0(long long n, double* __restrict__ V, const dou
     b[i] = bi;
     x[i] = T(kOmega) * inv[i] * bi;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->cycle_end = 0;
 }
 // Z[j] = z (the preconditioner's output, widened exactly to fp64) and
 // V[j+1] = wt .* (A_s z), LPR lanes per row (the level-0 Y_W_AX product)
@@ -2568,154 +2571,275 @@ __global__ void __launch_bounds__(TB) k_fg_op(int n, const int* __restrict__ row
     }
   }
 }
-// Gram-Schmidt dots of pass `pass` against w = V[j+1]: pass 0 over V[0..j] and
-// w.w (k_multidot_g's self); pass 1 only when the reorth flag is set.
-__global__ void __launch_bounds__(TB, 4) k_fg_multidot(long long n, const double* __restrict__ V,
-                                                    double* __restrict__ partial, double* __restrict__ H, int ldh,
-                                                    double* __restrict__ y, FgState* st, int pass) {
-  pdl_wait_release();
-  if (pass == 1 && !st->reorth) return;
-  const int j = st->j, k = j + 1, self = pass == 0;
-  const int q0 = blockIdx.y * kMD;
-  if (q0 >= k + self) return;
-  const double* w = V + (long long)(j + 1) * n;
-  __shared__ double sm[kMD][TB / 32];
-  __shared__ int s_last;
-  double acc[kMD];
-#pragma unroll
-  for (int u = 0; u < kMD; ++u) acc[u] = 0.0;
-  multidot_acc(acc, n, V, n, q0, k, self, w);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int u = 0; u < kMD; ++u) {
-    double v = warp_sum(acc[u]);
-    if (lane == 0) sm[u][wid] = v;
+// Column j of the Hessenberg matrix, by one block of TB threads: h plus the second
+// pass's terms, h[j+1][j] = ||w||, then on thread 0 the Givens rotation
+// (k_givens) and the estimate |g[j+1]|; the counters, the inner loop's
+// condition and, at a cycle's end, y = R^-1 g column by column.  The column and
+// the rotations are staged in shared memory (sm: 5 * 128 doubles), so the serial
+// part waits on no global load.
+__device__ void fg_column(double* H, int ldh, double* cs, double* sn, double* g, double* y, FgState* st, double tol,
+                          int max_iters, int m, cudaGraphConditionalHandle inner, double* sm) {
+  double *hj = sm, *c_ = sm + 128, *s_ = c_ + 128, *gg = s_ + 128, *yy = gg + 128;
+  const int j = st->j;
+  double* Hj = H + (long long)j * ldh;
+  const bool second = st->reorth != 0;
+  for (int q = threadIdx.x; q <= j; q += TB) {
+    hj[q] = second ? __ldcg(Hj + q) + __ldcg(y + q) : __ldcg(Hj + q);
+    c_[q] = q < j ? cs[q] : 0.0;
+    s_[q] = q < j ? sn[q] : 0.0;
   }
+  __shared__ int s_end;
   __syncthreads();
-  if (threadIdx.x < kMD && q0 + (int)threadIdx.x < k + self) {
-    double t = 0.0;
-    for (int u = 0; u < TB / 32; ++u) t += sm[threadIdx.x][u];
-    partial[(q0 + threadIdx.x) * kDotBlocks + blockIdx.x] = t;
-    __threadfence();
-  }
-  __syncthreads();
-  // the last block of the launch to finish sums every dot's partials in block
-  // order (warp w takes dots w, w + 8, ...): into column j of H in pass 0
-  // (entry j + 1 is ||w||^2 until k_fg_column), into y in pass 1
   if (threadIdx.x == 0) {
-    const int active = kDotBlocks * ((k + self + kMD - 1) / kMD);
-    s_last = atomicAdd(&st->gs_count, 1) == active - 1;
+    double up = hj[0];
+    for (int i = 0; i < j; ++i) {
+      const double dn = hj[i + 1];
+      hj[i] = c_[i] * up + s_[i] * dn;
+      up = -s_[i] * up + c_[i] * dn;
+    }
+    const double a = up, b = sqrt(st->wn2);
+    const double d = hypot(a, b);
+    const double c = d > 0 ? a / d : 1.0, sv = d > 0 ? b / d : 0.0;
+    cs[j] = c;
+    sn[j] = sv;
+    hj[j] = d;
+    const double gj = g[j];
+    g[j + 1] = -sv * gj;
+    g[j] = c * gj;
+    const double est = fabs(sv * gj) / st->bnorm;
+    st->rel = est;
+    st->total += 1;
+    st->j = j + 1;
+    const bool nan = !(est == est);
+    if (nan) st->nan = 1;
+    const bool end = nan || est < tol || j + 1 >= m || st->total >= max_iters;
+    cudaGraphSetConditional(inner, end ? 0u : 1u);
+    s_end = end && !nan;
   }
   __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  double* out = pass == 0 ? H + (long long)j * ldh : y;
-  for (int q = wid; q < k + self; q += TB / 32) {
-    double t = 0.0;
-    for (int b = lane; b < kDotBlocks; b += 32) t += __ldcg(partial + (long long)q * kDotBlocks + b);
-    t = warp_sum(t);
-    if (lane == 0) out[q] = t;
+  for (int q = threadIdx.x; q <= j; q += TB) Hj[q] = hj[q];
+  if (!s_end) return;
+  const int k = j + 1;
+  for (int q = threadIdx.x; q < k; q += TB) gg[q] = g[q];
+  __syncthreads();
+  for (int i = k - 1; i >= 0; --i) {
+    const double* col = H + (long long)i * ldh;
+    if (threadIdx.x == 0) yy[i] = gg[i] / (i == j ? hj[i] : col[i]);
+    __syncthreads();
+    const double yi = yy[i];
+    for (int q = threadIdx.x; q < i; q += TB) gg[q] -= (i == j ? hj[q] : col[q]) * yi;
+    __syncthreads();
   }
-  if (threadIdx.x == 0) st->gs_count = 0;
+  for (int q = threadIdx.x; q < k; q += TB) y[q] = yy[q];
 }
-// w -= sum_q h_q V[q] (h = column j of H, or y in pass 1); the last block to
-// finish sums the blocks' partial squares (||w||^2, FgState::wn2) and, after
-// pass 0, sets the reorthogonalisation flag, which also opens the conditional
-// node of pass 1
-__global__ void __launch_bounds__(TB) k_fg_update(long long n, double* __restrict__ V, const double* __restrict__ H,
-                                                  int ldh, const double* __restrict__ y,
-                                                  double* __restrict__ partial, FgState* st, int pass,
-                                                  cudaGraphConditionalHandle reorth_if) {
-  pdl_wait_release();
-  if (pass == 1 && !st->reorth) return;
-  __shared__ double sh[128];
-  __shared__ double sm[TB / 32];
+
+// Classical Gram-Schmidt of w = V[j+1] against V[0..j], twice when the first pass
+// left less than 0.7 of the norm, in three launches that each read the basis once
+// (PASS 0: h = V^T w and ||w||^2; PASS 1: w -= V h and, from the same registers,
+// y = V^T w and ||w||^2; PASS 2: w -= V y, ||w||^2, then the Hessenberg column).
+// Warp v of a block holds vectors v, v + 8, .. (U of them) at 32 E elements in
+// registers (U E = 16 while n leaves every block a tile), the next tile's loads
+// in flight while the current one is worked on.  The update sums the warps'
+// parts of V h in shared memory; the dots stay in registers over the block's
+// tiles.  The last block to finish sums the blocks' partials in block order.
+//
+// Bound by HBM, (j + 2) n 8 bytes a launch: at n = 1e6 and 60 vectors passes 0
+// and 1 take 91 and 105 us (5.4 and 4.7 TB/s of 6.45 measured).  A thread per
+// element with eight vectors' loads in flight read the basis four times at
+// 3.6 TB/s; tiles in shared memory (cp.async, two buffers) took 57 / 83 us a
+// pass at 30 vectors, their update bound by shared-memory reads.
+constexpr int kGsBlocks = 296;                 // two an SM; fixed, so partials have a fixed order
+constexpr int kGsWarps = TB / 32;
+struct GsSmem {
+  double part[2][kGsWarps][512];               // the warps' parts of V h, by parity
+  double w[2][512];                            // the updated elements
+};
+template <int PASS, int U, int E>
+__device__ __forceinline__ void gs_tiles(long long n, const double* __restrict__ V, int k, double* __restrict__ w,
+                                         const double* __restrict__ h, double* __restrict__ partial, GsSmem& sm,
+                                         double& nrm) {
+  constexpr int TE = 32 * E;
+  constexpr int WU = (TE + TB - 1) / TB;       // elements of w a thread updates
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long tiles = (n + TE - 1) / TE;
+  double hq[U], acc[U], r[U][E], wv[PASS == 0 ? E : WU];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int q = warp + kGsWarps * u;
+    acc[u] = 0.0;
+    hq[u] = (PASS > 0 && q < k) ? h[q] : 0.0;
+  }
+  auto load = [&](long long t, double (&rr)[U][E], double (&ww)[PASS == 0 ? E : WU]) {
+    const long long i0 = t * TE;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = warp + kGsWarps * u;
+      if (q < k) {
+#pragma unroll
+        for (int x = 0; x < E; ++x) {
+          const long long i = i0 + lane + 32 * x;
+          rr[u][x] = i < n ? __ldcg(V + q * n + i) : 0.0;
+        }
+      } else {
+#pragma unroll
+        for (int x = 0; x < E; ++x) rr[u][x] = 0.0;
+      }
+    }
+    if (PASS == 0) {
+#pragma unroll
+      for (int x = 0; x < E; ++x) {
+        const long long i = i0 + lane + 32 * x;
+        ww[x] = i < n ? w[i] : 0.0;
+      }
+    } else {
+#pragma unroll
+      for (int x = 0; x < WU; ++x) {
+        const int e = threadIdx.x + TB * x;
+        ww[x] = (e < TE && i0 + e < n) ? w[i0 + e] : 0.0;
+      }
+    }
+  };
+  if (blockIdx.x < tiles) load(blockIdx.x, r, wv);
+  int par = 0;
+  for (long long t = blockIdx.x; t < tiles; t += gridDim.x, par ^= 1) {
+    double rn[U][E], wn[PASS == 0 ? E : WU];
+    const bool more = t + gridDim.x < tiles;
+    if (more) load(t + gridDim.x, rn, wn);
+    if (PASS == 0) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int x = 0; x < E; ++x) acc[u] += r[u][x] * wv[x];
+      if (warp == 0)
+#pragma unroll
+        for (int x = 0; x < E; ++x) nrm += wv[x] * wv[x];
+    } else {
+#pragma unroll
+      for (int x = 0; x < E; ++x) {
+        double p = hq[0] * r[0][x];
+#pragma unroll
+        for (int u = 1; u < U; ++u) p += hq[u] * r[u][x];
+        sm.part[par][warp][lane + 32 * x] = p;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int x = 0; x < WU; ++x) {
+        const int e = threadIdx.x + TB * x;
+        if (e < TE) {
+          double p = sm.part[par][0][e];
+#pragma unroll
+          for (int q = 1; q < kGsWarps; ++q) p += sm.part[par][q][e];
+          const double v = wv[x] - p;
+          const long long i = t * TE + e;
+          if (i < n) w[i] = v;
+          nrm += v * v;
+          if (PASS == 1) sm.w[par][e] = v;
+        }
+      }
+      if (PASS == 1) {
+        __syncthreads();
+#pragma unroll
+        for (int x = 0; x < E; ++x) {
+          const double v = sm.w[par][lane + 32 * x];
+#pragma unroll
+          for (int u = 0; u < U; ++u) acc[u] += r[u][x] * v;
+        }
+      }
+    }
+    if (more) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int x = 0; x < E; ++x) r[u][x] = rn[u][x];
+#pragma unroll
+      for (int x = 0; x < (PASS == 0 ? E : WU); ++x) wv[x] = wn[x];
+    }
+  }
+  if (PASS < 2) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = warp + kGsWarps * u;
+      if (q < k) {
+        const double v = warp_sum(acc[u]);
+        if (lane == 0) partial[(long long)q * kGsBlocks + blockIdx.x] = v;
+      }
+    }
+  }
+}
+template <int PASS, int U>
+__device__ __forceinline__ void gs_pick(long long n, const double* V, int k, double* w, const double* h,
+                                        double* partial, GsSmem& sm, double& nrm) {
+  // one element a lane where larger tiles would leave blocks without one
+  if (U < 16 && n < (long long)gridDim.x * (512 / U)) gs_tiles<PASS, U, 1>(n, V, k, w, h, partial, sm, nrm);
+  else gs_tiles<PASS, U, 16 / U>(n, V, k, w, h, partial, sm, nrm);
+}
+template <int PASS>
+__global__ void __launch_bounds__(TB, 2) k_fg_gs(long long n, double* V, double* partial, double* H, int ldh,
+                                                 double* y, FgState* st, double* cs, double* sn, double* g,
+                                                 double tol, int max_iters, int m,
+                                                 cudaGraphConditionalHandle inner) {
+  extern __shared__ __align__(16) unsigned char gs_smem[];
+  GsSmem& sm = *reinterpret_cast<GsSmem*>(gs_smem);
+  double* scratch = reinterpret_cast<double*>(gs_smem);
+  __shared__ double s_n[kGsWarps];
   __shared__ int s_last;
+  pdl_wait_release();
+  if (PASS == 2 && !st->reorth) {
+    if (blockIdx.x == 0) fg_column(H, ldh, cs, sn, g, y, st, tol, max_iters, m, inner, scratch);
+    return;
+  }
   const int j = st->j, k = j + 1;
-  const double* h = pass == 0 ? H + (long long)j * ldh : y;
-  for (int q = threadIdx.x; q < k; q += blockDim.x) sh[q] = h[q];
-  __syncthreads();
-  double* w = V + (long long)(j + 1) * n;
-  const double acc = update_rows(n, V, n, sh, k, w);
-  double t = warp_sum(acc);
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = t;
+  double* w = V + (long long)k * n;
+  const double* h = PASS == 1 ? H + (long long)j * ldh : y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double nrm = 0.0;
+  if (k <= 8) gs_pick<PASS, 1>(n, V, k, w, h, partial, sm, nrm);
+  else if (k <= 16) gs_pick<PASS, 2>(n, V, k, w, h, partial, sm, nrm);
+  else if (k <= 32) gs_pick<PASS, 4>(n, V, k, w, h, partial, sm, nrm);
+  else if (k <= 64) gs_pick<PASS, 8>(n, V, k, w, h, partial, sm, nrm);
+  else gs_pick<PASS, 16>(n, V, k, w, h, partial, sm, nrm);
+  nrm = warp_sum(nrm);
+  if (lane == 0) s_n[warp] = nrm;
+  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     double u = 0.0;
-    for (int q = 0; q < TB / 32; ++q) u += sm[q];
-    partial[blockIdx.x] = u;
+    for (int q = 0; q < kGsWarps; ++q) u += s_n[q];
+    partial[(long long)k * kGsBlocks + blockIdx.x] = u;
     __threadfence();
     s_last = atomicAdd(&st->gs_count, 1) == (int)gridDim.x - 1;
   }
   __syncthreads();
-  if (!s_last || threadIdx.x >= 32) return;
+  if (!s_last) return;
   __threadfence();
-  double nt = 0.0;
-  for (int b = threadIdx.x; b < kDotBlocks; b += 32) nt += __ldcg(partial + b);
-  nt = warp_sum(nt);
-  if (threadIdx.x == 0) {
-    st->gs_count = 0;
-    st->wn2 = nt;
-    if (pass == 0) {
-      st->reorth = nt < 0.49 * H[(long long)st->j * ldh + st->j + 1];
-      st->reorths += st->reorth;
-      cudaGraphSetConditional(reorth_if, st->reorth ? 1u : 0u);
+  for (int q = PASS < 2 ? warp : k; q <= k; q += kGsWarps) {
+    if (PASS == 2 && warp > 0) break;
+    double t = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(partial + (long long)q * kGsBlocks + b);
+    t = warp_sum(t);
+    if (lane == 0) {
+      if (PASS == 0) H[(long long)j * ldh + q] = t;            // entry j + 1: ||w||^2
+      else if (q < k) y[q] = t;
+      else {
+        st->wn2 = t;
+        if (PASS == 1) {
+          st->reorth = t < 0.49 * H[(long long)j * ldh + k];
+          st->reorths += st->reorth;
+        }
+      }
     }
   }
-}
-// Column j of the Hessenberg matrix in one block: the reorthogonalisation
-// terms and h[j+1][j], then on thread 0 the Givens rotation (k_givens), the
-// estimate |g[j+1]|, the counters, the continue/cycle-end decision and, at a
-// cycle's end, y = R^-1 g (k_backsolve over the j columns).
-__global__ void k_fg_column(double* H, int ldh, double* cs, double* sn, double* g, double* y, FgState* st,
-                            double tol, int max_iters, int m, cudaGraphConditionalHandle cond,
-                            cudaGraphConditionalHandle end_if) {
-  pdl_wait_release();
-  const int j = st->j;
-  double* hj = H + (long long)j * ldh;
-  if (st->reorth)
-    for (int q = threadIdx.x; q <= j; q += blockDim.x) hj[q] += y[q];
-  if (threadIdx.x == 0) hj[j + 1] = sqrt(st->wn2);
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  for (int i = 0; i < j; ++i) {
-    double t = cs[i] * hj[i] + sn[i] * hj[i + 1];
-    hj[i + 1] = -sn[i] * hj[i] + cs[i] * hj[i + 1];
-    hj[i] = t;
-  }
-  double a = hj[j], b = hj[j + 1];
-  double d = hypot(a, b);
-  double c = d > 0 ? a / d : 1.0, sv = d > 0 ? b / d : 0.0;
-  cs[j] = c; sn[j] = sv;
-  hj[j] = d; hj[j + 1] = 0.0;
-  g[j + 1] = -sv * g[j];
-  g[j] = c * g[j];
-  const double est = fabs(g[j + 1]) / st->bnorm;
-  st->rel = est;
-  st->total += 1;
-  st->j = j + 1;
-  const bool nan = !(est == est);
-  if (nan) st->nan = 1;
-  const bool conv = est < tol;
-  st->cycle_end = nan || conv || st->j >= m || st->total >= max_iters;
-  cudaGraphSetConditional(end_if, st->cycle_end ? 1u : 0u);
-  if (!st->cycle_end) {
-    cudaGraphSetConditional(cond, 1u);
-    return;
-  }
-  if (st->nan) return;
-  const int k = st->j;
-  for (int i = k - 1; i >= 0; --i) {
-    double s = g[i];
-    for (int jj = i + 1; jj < k; ++jj) s -= H[(long long)jj * ldh + i] * y[jj];
-    y[i] = s / H[(long long)i * ldh + i];
+  if (threadIdx.x == 0) st->gs_count = 0;
+  if (PASS == 2) {
+    __syncthreads();
+    fg_column(H, ldh, cs, sn, g, y, st, tol, max_iters, m, inner, scratch);
   }
 }
 // at a cycle's end x_s += Z y ...
 __global__ void k_fg_combine(long long n, const double* __restrict__ Z, const double* __restrict__ y,
                              double* __restrict__ x, const FgState* st) {
   pdl_wait_release();
-  if (!st->cycle_end || st->nan) return;
+  if (st->nan) return;
   __shared__ double sy[128];
   const int k = st->j;
   for (int q = threadIdx.x; q < k; q += blockDim.x) sy[q] = y[q];
@@ -2730,7 +2854,7 @@ __global__ void __launch_bounds__(TB) k_fg_resid(int n, const int* __restrict__ 
                                                  double* __restrict__ V, int rel, double* __restrict__ partial,
                                                  const FgState* st) {
   pdl_wait_release();
-  if (!st->cycle_end || st->nan) return;
+  if (st->nan) return;
   __shared__ double sm[TB / 32];
   const int g = threadIdx.x / LPR, lane = threadIdx.x % LPR;
   const int rows_per_block = TB / LPR;
@@ -2763,15 +2887,16 @@ __global__ void __launch_bounds__(TB) k_fg_resid(int n, const int* __restrict__ 
 __global__ void k_fg_restart(const double* partial, int nb, FgState* st, double* g, int m1, double tol,
                              int max_iters, cudaGraphConditionalHandle cond) {
   pdl_wait_release();
-  if (!st->cycle_end) return;
+  double r2 = 0.0;
+  for (int q = threadIdx.x; q < nb; q += 32) r2 += partial[q];
+  r2 = warp_sum(r2);
+  if (threadIdx.x != 0) return;
   if (st->nan) {
     st->done = 1;
     st->converged = 0;
     cudaGraphSetConditional(cond, 0u);
     return;
   }
-  double r2 = 0.0;
-  for (int q = 0; q < nb; ++q) r2 += partial[q];
   const double beta = sqrt(r2);
   st->beta = beta;
   st->true_rel = beta / st->bnorm;
@@ -2868,37 +2993,50 @@ void fg_resid(const Level& L0, const CT* col, const double* xs, const double* bs
              st);
 }
 
-// Appends an IF conditional node on `hc` to the graph that `s` is capturing,
-// captures emit(q) into the node's body on the handle's third stream, and
-// continues the capture of `s` after the node.
+// Appends a WHILE conditional node on `hc` to the graph that `s` is capturing,
+// captures emit() into the node's body on the stream `body` (created on first
+// use), and continues the capture of `s` after the node.
 template <typename F>
-void capture_if(cudaStream_t s, AMG& h, cudaGraphConditionalHandle hc, F emit) {
+void capture_while(cudaStream_t s, cudaStream_t& body, cudaGraphConditionalHandle hc, F emit) {
   cudaStreamCaptureStatus cst;
   cudaGraph_t g = nullptr;
   const cudaGraphNode_t* deps = nullptr;
   size_t ndeps = 0;
   IMPES_CUDA(cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, &deps, &ndeps));
-  IMPES_REQUIRE(cst == cudaStreamCaptureStatusActive, IMPES_ERR_STATE, "conditional block needs a capturing stream");
+  IMPES_REQUIRE(cst == cudaStreamCaptureStatusActive, IMPES_ERR_STATE, "a loop node needs a capturing stream");
   cudaGraphNodeParams cp = {};
   cp.type = cudaGraphNodeTypeConditional;
   cp.conditional.handle = hc;
-  cp.conditional.type = cudaGraphCondTypeIf;
+  cp.conditional.type = cudaGraphCondTypeWhile;
   cp.conditional.size = 1;
   cudaGraphNode_t node;
   IMPES_CUDA(cudaGraphAddNode(&node, g, deps, ndeps, &cp));
-  if (!h.if_stream) IMPES_CUDA(cudaStreamCreateWithFlags(&h.if_stream, cudaStreamNonBlocking));
-  IMPES_CUDA(cudaStreamBeginCaptureToGraph(h.if_stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                           cudaStreamCaptureModeThreadLocal));
+  if (!body) IMPES_CUDA(cudaStreamCreateWithFlags(&body, cudaStreamNonBlocking));
+  cudaGraph_t bg = cp.conditional.phGraph_out[0];
+  IMPES_CUDA(cudaStreamBeginCaptureToGraph(body, bg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   try {
-    emit(h.if_stream);
+    emit(bg);
   } catch (...) {
     cudaGraph_t dummy = nullptr;
-    cudaStreamEndCapture(h.if_stream, &dummy);
+    cudaStreamEndCapture(body, &dummy);
     throw;
   }
   cudaGraph_t out = nullptr;
-  IMPES_CUDA(cudaStreamEndCapture(h.if_stream, &out));
+  IMPES_CUDA(cudaStreamEndCapture(body, &out));
   IMPES_CUDA(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
+}
+
+void launch_gs(AMG& h, long long n, int ldh, const impes_krylov_params& kp, int m, cudaGraphConditionalHandle inner,
+               cudaStream_t s) {
+  const int grid = (int)std::min<long long>(kGsBlocks, (n + 31) / 32);
+  auto run = [&](auto* kern) {
+    raise_smem_limit((const void*)kern, sizeof(GsSmem));
+    launch_pdl(kern, grid, TB, sizeof(GsSmem), s, n, h.V.p, h.red.p, h.H.p, ldh, h.y.p, h.fgst.p, h.cs.p, h.sn.p,
+               h.g.p, kp.tol, kp.max_iters, m, inner);
+  };
+  run(k_fg_gs<0>);
+  run(k_fg_gs<1>);
+  run(k_fg_gs<2>);
 }
 }  // namespace
 
@@ -2949,102 +3087,52 @@ void amg_fgmres_capture(AMG& h, const double* b, double* x, const impes_krylov_p
                                    L0.col16.p, L0.col16_rel, L0.lpr_a[0]);
   launch_pdl(k_mul_inplace, gn, TB, 0, s, n, h.V.p, (const double*)wt);
   launch_pdl(k_fg_norm_partials, kDotBlocks, TB, 0, s, n, (const double*)h.V.p, part_r);
-  // the while node; the init kernel sets its condition (0: nothing to do)
+  // the cycles; the init kernel sets the outer condition (0: nothing to do)
   cudaStreamCaptureStatus cst;
   cudaGraph_t cap = nullptr;
-  const cudaGraphNode_t* deps = nullptr;
-  size_t ndeps = 0;
-  IMPES_CUDA(cudaStreamGetCaptureInfo(s, &cst, nullptr, &cap, &deps, &ndeps));
+  IMPES_CUDA(cudaStreamGetCaptureInfo(s, &cst, nullptr, &cap, nullptr, nullptr));
   IMPES_REQUIRE(cst == cudaStreamCaptureStatusActive, IMPES_ERR_STATE, "device FGMRES needs a capturing stream");
-  cudaGraphConditionalHandle cond;
-  IMPES_CUDA(cudaGraphConditionalHandleCreate(&cond, cap, 1, cudaGraphCondAssignDefault));
-  launch_pdl(k_fg_init, 1, 1, 0, s, st, (const double*)part_b, (const double*)part_r, (int)kDotBlocks, kp.tol,
-             kp.max_iters, m + 1, h.g.p, cond);
-  launch_pdl(k_fg_scale_v0, gn, TB, 0, s, n, h.V.p, (const FgState*)st, 0);
-  IMPES_CUDA(cudaStreamGetCaptureInfo(s, &cst, nullptr, &cap, &deps, &ndeps));
-  cudaGraphNodeParams cp = {};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = cond;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  cudaGraphNode_t wnode;
-  IMPES_CUDA(cudaGraphAddNode(&wnode, cap, deps, ndeps, &cp));
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  // the body, captured on a second stream into the node's graph
-  if (!h.body_stream) IMPES_CUDA(cudaStreamCreateWithFlags(&h.body_stream, cudaStreamNonBlocking));
-  cudaStream_t bsm = h.body_stream;
-  IMPES_CUDA(cudaStreamBeginCaptureToGraph(bsm, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  const unsigned long long body_start = thread_launches();
-  try {
-    const unsigned gb = grid_for(n, TB);
-    // z = M^-1 (V[j] / wt); Z[j] = z is written by the operator kernel
-    // the l1-Jacobi V-cycle's first level-0 sweep is fused with the input
-    // conversion (not for Chebyshev smoothing or a one-level hierarchy)
-    const bool fuse0 = h.prm.smoother != IMPES_SMOOTHER_CHEBYSHEV && !L0.coarsest;
-    if (kp.precision == 1) {
-      if (fuse0)
-        launch_pdl(k_fg_prec_smooth0<float>, gb, TB, 0, bsm, n, h.V.p, (const double*)wt,
-                   (const float*)L0.inv_relaxf.p, L0.bf.p, L0.xf.p, st);
-      else
-        launch_pdl(k_fg_prec_in<float>, gb, TB, 0, bsm, n, h.V.p, (const double*)wt, L0.bf.p, st);
-      const float* zf = vcycle<float>(h, 0, true, bsm, fuse0);
-      if (L0.col16.p)
-        fg_op(L0, (const unsigned short*)L0.col16.p, zf, h.Z.p, wt, h.V.p, L0.col16_rel, st, bsm);
-      else
-        fg_op(L0, (const int*)L0.col.p, zf, h.Z.p, wt, h.V.p, 0, st, bsm);
-    } else {
-      if (fuse0)
-        launch_pdl(k_fg_prec_smooth0<double>, gb, TB, 0, bsm, n, h.V.p, (const double*)wt,
-                   (const double*)L0.inv_relax.p, L0.b.p, L0.x.p, st);
-      else
-        launch_pdl(k_fg_prec_in<double>, gb, TB, 0, bsm, n, h.V.p, (const double*)wt, L0.b.p, st);
-      const double* zd = vcycle<double>(h, 0, true, bsm, fuse0);
-      if (L0.col16.p)
-        fg_op(L0, (const unsigned short*)L0.col16.p, zd, h.Z.p, wt, h.V.p, L0.col16_rel, st, bsm);
-      else
-        fg_op(L0, (const int*)L0.col.p, zd, h.Z.p, wt, h.V.p, 0, st, bsm);
-    }
-    // Gram-Schmidt: pass 0, then pass 1 inside an IF node that k_fg_update opens
-    // when the first pass lost too much of the vector's norm
-    const dim3 gd(kDotBlocks, (unsigned)((m + 2 + kMD - 1) / kMD));
-    cudaGraphConditionalHandle reorth_if, end_if;
-    IMPES_CUDA(cudaGraphConditionalHandleCreate(&reorth_if, body, 0, cudaGraphCondAssignDefault));
-    IMPES_CUDA(cudaGraphConditionalHandleCreate(&end_if, body, 0, cudaGraphCondAssignDefault));
-    auto gs_pass = [&](int pass, cudaStream_t q) {
-      launch_pdl(k_fg_multidot, gd, dim3(TB), 0, q, n, (const double*)h.V.p, h.red.p, h.H.p, ldh, h.y.p, st, pass);
-      launch_pdl(k_fg_update, kDotBlocks, TB, 0, q, n, h.V.p, (const double*)h.H.p, ldh, (const double*)h.y.p,
-                 h.red.p, st, pass, reorth_if);
-    };
-    gs_pass(0, bsm);
-    unsigned long long mark = thread_launches();
-    capture_if(bsm, h, reorth_if, [&](cudaStream_t q) { gs_pass(1, q); });
-    h.fg_reorth_kernels = (long long)(thread_launches() - mark);
-    // (V[j+1] is normalised by the next iteration's input kernel)
-    launch_pdl(k_fg_column, 1, 128, 0, bsm, h.H.p, ldh, h.cs.p, h.sn.p, h.g.p, h.y.p, st, kp.tol, kp.max_iters, m,
-               cond, end_if);
-    // a cycle's end (IF node opened by k_fg_column): x_s += Z y, the true
-    // residual, the restart/stop decision and the new V[0]
-    mark = thread_launches();
-    capture_if(bsm, h, end_if, [&](cudaStream_t q) {
-      launch_pdl(k_fg_combine, gb, TB, 0, q, n, (const double*)h.Z.p, (const double*)h.y.p, xs, (const FgState*)st);
-      if (L0.col16.p)
-        fg_resid<unsigned short>(L0, L0.col16.p, xs, bs, wt, h.V.p, L0.col16_rel, part_r, st, q);
-      else
-        fg_resid<int>(L0, L0.col.p, xs, bs, wt, h.V.p, 0, part_r, st, q);
-      launch_pdl(k_fg_restart, 1, 1, 0, q, (const double*)part_r, (int)kDotBlocks, st, h.g.p, m + 1, kp.tol,
-                 kp.max_iters, cond);
-      launch_pdl(k_fg_scale_v0, gb, TB, 0, q, n, h.V.p, (const FgState*)st, 1);
+  cudaGraphConditionalHandle outer;
+  IMPES_CUDA(cudaGraphConditionalHandleCreate(&outer, cap, 1, cudaGraphCondAssignDefault));
+  launch_pdl(k_fg_init, 1, 32, 0, s, st, (const double*)part_b, (const double*)part_r, (int)kDotBlocks, kp.tol,
+             kp.max_iters, m + 1, h.g.p, outer);
+  const unsigned long long mark = thread_launches();
+  capture_while(s, h.body_stream, outer, [&](cudaGraph_t body) {
+    cudaStream_t bs_ = h.body_stream;
+    cudaGraphConditionalHandle inner;
+    IMPES_CUDA(cudaGraphConditionalHandleCreate(&inner, body, 0, cudaGraphCondAssignDefault));
+    launch_pdl(k_fg_scale_v0, gn, TB, 0, bs_, n, h.V.p, (const FgState*)st, inner);
+    const unsigned long long mark_in = thread_launches();
+    capture_while(bs_, h.inner_stream, inner, [&](cudaGraph_t) {
+      cudaStream_t q = h.inner_stream;
+      // z = M^-1 (V[j] / wt); Z[j] = z is written by the operator kernel.  The
+      // l1-Jacobi V-cycle's first level-0 sweep is fused with the input
+      // conversion (not for Chebyshev smoothing or a one-level hierarchy)
+      const bool fuse0 = h.prm.smoother != IMPES_SMOOTHER_CHEBYSHEV && !L0.coarsest;
+      auto precondition = [&](auto* b0, auto* x0, const auto* inv0) {
+        using T = std::remove_pointer_t<decltype(b0)>;
+        if (fuse0) launch_pdl(k_fg_prec_smooth0<T>, gn, TB, 0, q, n, h.V.p, (const double*)wt, inv0, b0, x0, (const FgState*)st);
+        else launch_pdl(k_fg_prec_in<T>, gn, TB, 0, q, n, h.V.p, (const double*)wt, b0, (const FgState*)st);
+        const T* z = vcycle<T>(h, 0, true, q, fuse0);
+        if (L0.col16.p) fg_op(L0, (const unsigned short*)L0.col16.p, z, h.Z.p, wt, h.V.p, L0.col16_rel, st, q);
+        else fg_op(L0, (const int*)L0.col.p, z, h.Z.p, wt, h.V.p, 0, st, q);
+      };
+      if (kp.precision == 1) precondition(L0.bf.p, L0.xf.p, (const float*)L0.inv_relaxf.p);
+      else precondition(L0.b.p, L0.x.p, (const double*)L0.inv_relax.p);
+      // (V[j+1] is normalised by the next iteration's input kernel)
+      launch_gs(h, n, ldh, kp, m, inner, q);
     });
-    h.fg_end_kernels = (long long)(thread_launches() - mark);
-  } catch (...) {
-    cudaGraph_t dummy = nullptr;
-    cudaStreamEndCapture(bsm, &dummy);
-    throw;
-  }
-  cudaGraph_t body_out = nullptr;
-  IMPES_CUDA(cudaStreamEndCapture(bsm, &body_out));
-  h.fg_body_kernels = (long long)(thread_launches() - body_start) - h.fg_reorth_kernels - h.fg_end_kernels;
-  IMPES_CUDA(cudaStreamUpdateCaptureDependencies(s, &wnode, 1, cudaStreamSetCaptureDependencies));
+    h.fg_body_kernels = (long long)(thread_launches() - mark_in);
+    // a cycle's end: x_s += Z y, the true residual, the restart/stop decision
+    launch_pdl(k_fg_combine, gn, TB, 0, bs_, n, (const double*)h.Z.p, (const double*)h.y.p, xs, (const FgState*)st);
+    if (L0.col16.p)
+      fg_resid<unsigned short>(L0, L0.col16.p, xs, bs, wt, h.V.p, L0.col16_rel, part_r, st, bs_);
+    else
+      fg_resid<int>(L0, L0.col.p, xs, bs, wt, h.V.p, 0, part_r, st, bs_);
+    launch_pdl(k_fg_restart, 1, 32, 0, bs_, (const double*)part_r, (int)kDotBlocks, st, h.g.p, m + 1, kp.tol,
+               kp.max_iters, outer);
+  });
+  h.fg_end_kernels = (long long)(thread_launches() - mark) - h.fg_body_kernels;
   // epilogue: x = D^-1/2 x_s (zero for a zero right-hand side)
   launch_pdl(k_fg_final, gn, TB, 0, s, n, (const double*)h.dhalf_inv.p, (const double*)xs, x, (const FgState*)st);
 }
