@@ -95,9 +95,11 @@ struct Level {
 // Solver state of the device-driven FGMRES (amg_cycle.cu), read by the host
 // after the captured solve has run.
 struct FgState {
-  int j, total, restarts, converged, done, reorth, bzero, nan;
+  int j, total, restarts, converged, done, cycle_end, reorth, bzero, nan;
   int reorths;                          // second Gram-Schmidt passes taken
   int gs_count;                         // blocks of a Gram-Schmidt launch done (last block reduces)
+  int max_iters;                        // limits of the solve (k_fg_params)
+  double tol;
   double bnorm, beta, wn2, rel, true_rel;
 };
 
@@ -121,14 +123,14 @@ struct AMG {
   int krylov_m = 0;
   DBuf<double> V, Z, H, cs, sn, g, y, kw, kb, kx;
   bool krylov_mode = false;        // V-cycles issued by FGMRES
-  // CUDA graphs of a whole V-cycle from level 0, per [fp32][zero start][krylov][timed]
+  // CUDA graphs of a whole stand-alone V-cycle from level 0, per [fp32][zero start][timed]
   struct VGraph {
     cudaGraphExec_t exec = nullptr;
     void* out = nullptr;
     long long kernels = 0;
     std::vector<PhaseTimers::Rec> timers;
   };
-  VGraph vgraph[2][2][2][2];
+  VGraph vgraph[2][2][2];
   cudaStream_t cap_stream = nullptr;
   cudaStream_t body_stream = nullptr;   // captures a cycle of the device FGMRES
   cudaStream_t inner_stream = nullptr;  // captures an iteration inside it
@@ -147,6 +149,15 @@ struct AMG {
     long long kernels_fixed = 0, kernels_body = 0, kernels_end = 0;
   };
   std::vector<StepGraph> step_graphs;
+  // FGMRES solves captured on the handle's own vectors, per norm and precision
+  struct FgGraph {
+    cudaGraphExec_t exec = nullptr;
+    bool jac = false;
+    int precision = 0;
+    long long kernels_fixed = 0, kernels_body = 0, kernels_end = 0;
+  };
+  std::vector<FgGraph> fg_graphs;
+  bool fg_graph_failed = false;         // capture refused once: host-driven solves
   bool step_graph_failed = false;       // capture refused once: keep the host-driven path
   bool use_graphs = true;
   bool use_step_graph = true;           // whole IMPES steps as graphs (IMPES_NO_STEP_GRAPH=1: off)
@@ -165,7 +176,7 @@ struct AMG {
   int stail_level = -1;                 // first level of the shared-memory fp32 tail, -1: none
   size_t stail_smem = 0;                // its shared-memory bytes
   void drop_graphs() {
-    for (auto& a : vgraph) for (auto& b : a) for (auto& c : b) for (auto& g : c) {
+    for (auto& a : vgraph) for (auto& b : a) for (auto& g : b) {
       if (g.exec) cudaGraphExecDestroy(g.exec);
       g.exec = nullptr;
       for (auto& r : g.timers) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
@@ -174,6 +185,9 @@ struct AMG {
     for (auto& g : step_graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     step_graphs.clear();
+    for (auto& g : fg_graphs)
+      if (g.exec) cudaGraphExecDestroy(g.exec);
+    fg_graphs.clear();
   }
   ~AMG() {
     drop_graphs();

@@ -829,11 +829,9 @@ __global__ void k_mul_inplace(long long n, double* a, const double* b) {
 __global__ void k_zero(long long n, double* a) {
   pdl_wait_release(); GRID_LOOP(i, n) a[i] = 0.0; }
 
-// v - sum_{q<k} h[q] * V[q*ld + i] (or v + ..., sign = -1 / +1) with the q
-// terms added one after another as in the plain loop, but with the loads of up
+// v + sum_{q<k} h[q] * V[q*ld + i] with the q terms added one after another as in the plain loop, but with the loads of up
 // to eight vectors issued together so that each thread keeps several HBM
 // requests in flight.
-template <int SIGN>
 __device__ __forceinline__ double axpy_rows(double v, const double* __restrict__ h, int k,
                                             const double* __restrict__ V, long long ld, long long i) {
   int q = 0;
@@ -842,9 +840,9 @@ __device__ __forceinline__ double axpy_rows(double v, const double* __restrict__
 #pragma unroll
     for (int u = 0; u < 8; ++u) a[u] = V[(q + u) * ld + i];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v = SIGN > 0 ? v + h[q + u] * a[u] : v - h[q + u] * a[u];
+    for (int u = 0; u < 8; ++u) v = v + h[q + u] * a[u];
   }
-  for (; q < k; ++q) v = SIGN > 0 ? v + h[q] * V[q * ld + i] : v - h[q] * V[q * ld + i];
+  for (; q < k; ++q) v = v + h[q] * V[q * ld + i];
   return v;
 }
 
@@ -880,143 +878,13 @@ __global__ void __launch_bounds__(TB) k_multidot(long long n, const double* __re
     partial[threadIdx.x * kDotBlocks + blockIdx.x] = t;
   }
 }
-// Gram-Schmidt dot accumulation over this thread's elements (grid stride),
-// two elements per trip so that each thread has the loads of 2 x 8 vectors in
-// flight; every accumulator adds its elements in index order, as a one-element
-// loop would.
-__device__ __forceinline__ void multidot_acc(double* acc, long long n, const double* __restrict__ V,
-                                             long long ldv, int q0, int k, int self,
-                                             const double* __restrict__ w) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  for (; i + stride < n; i += 2 * stride) {
-    const double w0 = w[i], w1 = w[i + stride];
-    double a0[kMD], a1[kMD];
-#pragma unroll
-    for (int u = 0; u < kMD; ++u) {
-      const int q = q0 + u;
-      a0[u] = q < k ? V[q * ldv + i] : w0;
-      a1[u] = q < k ? V[q * ldv + i + stride] : w1;
-    }
-#pragma unroll
-    for (int u = 0; u < kMD; ++u) {
-      const int q = q0 + u;
-      if (q < k || (q == k && self)) {
-        acc[u] += a0[u] * w0;
-        acc[u] += a1[u] * w1;
-      }
-    }
-  }
-  for (; i < n; i += stride) {
-    const double wi = w[i];
-#pragma unroll
-    for (int u = 0; u < kMD; ++u) {
-      const int q = q0 + u;
-      if (q < k) acc[u] += V[q * ldv + i] * wi;
-      else if (q == k && self) acc[u] += wi * wi;
-    }
-  }
-}
-// w -= sum_q h[q] V[q] over this thread's elements, two per trip; returns the
-// partial sum of squares of the new w in index order.
-__device__ __forceinline__ double update_rows(long long n, const double* __restrict__ V, long long ldv,
-                                              const double* __restrict__ h, int k, double* __restrict__ w) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  double acc = 0.0;
-  for (; i + stride < n; i += 2 * stride) {
-    const double v0 = axpy_rows<-1>(w[i], h, k, V, ldv, i);
-    const double v1 = axpy_rows<-1>(w[i + stride], h, k, V, ldv, i + stride);
-    w[i] = v0;
-    w[i + stride] = v1;
-    acc += v0 * v0;
-    acc += v1 * v1;
-  }
-  for (; i < n; i += stride) {
-    const double v = axpy_rows<-1>(w[i], h, k, V, ldv, i);
-    w[i] = v;
-    acc += v * v;
-  }
-  return acc;
-}
-
-// Gram-Schmidt dots of FGMRES in one launch: block (x, g) sums, over its slice
-// of rows, V[q] . w for the 8 vectors q = 8g .. 8g+7 below k, and w . w as
-// vector q = k when self is set; partial[q * kDotBlocks + x].  With pred set
-// the launch does nothing unless *pred is non-zero (the optional second
-// Gram-Schmidt pass, decided on the device).
-__global__ void __launch_bounds__(TB, 4) k_multidot_g(long long n, const double* __restrict__ Vbase,
-                                                   long long ldv, int k, int self,
-                                                   const double* __restrict__ w,
-                                                   double* __restrict__ partial, const int* pred) {
+// out[0] = sum of partials, fixed order
+__global__ void k_dot_finalize(const double* partial, double* out) {
   pdl_wait_release();
-  if (pred && *pred == 0) return;
-  __shared__ double s[kMD][TB / 32];
-  const int q0 = blockIdx.y * kMD;
-  const int kk = k + (self ? 1 : 0);
-  double acc[kMD];
-#pragma unroll
-  for (int u = 0; u < kMD; ++u) acc[u] = 0.0;
-  multidot_acc(acc, n, Vbase, ldv, q0, k, self, w);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int u = 0; u < kMD; ++u) {
-    double v = warp_sum(acc[u]);
-    if (lane == 0) s[u][wid] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < kMD && q0 + (int)threadIdx.x < kk) {
-    double t = 0.0;
-    for (int u = 0; u < TB / 32; ++u) t += s[threadIdx.x][u];
-    partial[(q0 + threadIdx.x) * kDotBlocks + blockIdx.x] = t;
-  }
-}
-// Second Gram-Schmidt pass wanted when the first pass left less than 0.7 of the
-// vector's norm ("twice is enough", Giraud, Langou & Rozloznik 2005):
-// flag = ||w'||^2 < 0.49 ||w||^2.
-__global__ void k_reorth_flag(const double* nrm2_after, const double* nrm2_before, int* flag) {
-  pdl_wait_release();
-  *flag = (*nrm2_after < 0.49 * *nrm2_before) ? 1 : 0;
-}
-// out[q] (+)= sum of partials, fixed order
-__global__ void k_dot_finalize(int k, const double* partial, double* out, int accumulate,
-                               const int* pred = nullptr) {
-  pdl_wait_release();
-  if (pred && *pred == 0) return;
-  const int q = blockIdx.x;
   double t = 0.0;
-  for (int b = threadIdx.x; b < kDotBlocks; b += 32) t += partial[q * kDotBlocks + b];
+  for (int b = threadIdx.x; b < kDotBlocks; b += 32) t += partial[b];
   t = warp_sum(t);
-  if (threadIdx.x == 0) out[q] = accumulate ? out[q] + t : t;
-  (void)k;
-}
-// w -= sum_q h[q] V[q]; optionally partial norms of the result
-__global__ void __launch_bounds__(TB) k_update(long long n, const double* __restrict__ Vbase,
-                                               long long ldv, int k, const double* __restrict__ h,
-                                               double* __restrict__ w, double* __restrict__ partial,
-                                               const int* pred = nullptr) {
-  pdl_wait_release();
-  if (pred && *pred == 0) return;
-  __shared__ double sh[128];
-  __shared__ double s[TB / 32];
-  for (int q = threadIdx.x; q < k; q += blockDim.x) sh[q] = h[q];
-  __syncthreads();
-  const double acc = update_rows(n, Vbase, ldv, sh, k, w);
-  if (partial) {
-    double t = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double u = 0.0;
-      for (int q = 0; q < TB / 32; ++q) u += s[q];
-      partial[blockIdx.x] = u;
-    }
-  }
-}
-__global__ void k_scale_by_inv_sqrt(long long n, const double* in, double* out, const double* nrm2) {
-  pdl_wait_release();
-  const double inv = 1.0 / sqrt(*nrm2);
-  GRID_LOOP(i, n) out[i] = in[i] * inv;
+  if (threadIdx.x == 0) *out = t;
 }
 
 // --------------------------------------------------- coarsest dense solve
@@ -1061,7 +929,7 @@ void spmv(const Level& L, const double* x, double* y, cudaStream_t s) {
 double dot_host(AMG& h, const double* a, const double* b, int n, cudaStream_t s) {
   h.red.ensure((size_t)kMD * kDotBlocks);
   launch_pdl(k_multidot, kDotBlocks, TB, 0, s, n, a, 0, 1, b, h.red.p);
-  launch_pdl(k_dot_finalize, 1, 32, 0, s, 1, (const double*)h.red.p, h.scal.p, 0, (const int*)nullptr);
+  launch_pdl(k_dot_finalize, 1, 32, 0, s, (const double*)h.red.p, h.scal.p);
   IMPES_CHECK_LAUNCH();
   IMPES_CUDA(cudaMemcpyAsync(h.hbuf.p, h.scal.p, sizeof(double), cudaMemcpyDeviceToHost, s));
   IMPES_CUDA(cudaStreamSynchronize(s));
@@ -1774,7 +1642,7 @@ T* vcycle_top(AMG& h, bool zero_x, cudaStream_t s) {
   dense_ensure<T>(h, s);
   if (!h.use_graphs) return vcycle<T>(h, 0, zero_x, s);
   PhaseTimers& tm = timers();
-  AMG::VGraph& g = h.vgraph[sizeof(T) == 4][zero_x][h.krylov_mode][tm.on];
+  AMG::VGraph& g = h.vgraph[sizeof(T) == 4][zero_x][tm.on];
   if (!g.exec) {
     if (!h.cap_stream) IMPES_CUDA(cudaStreamCreateWithFlags(&h.cap_stream, cudaStreamNonBlocking));
     const unsigned long long before = thread_launches();
@@ -2262,65 +2130,10 @@ void amg_apply(AMG& h, const double* b, double* x, int cycles, double apply_tol,
 // ------------------------------------------------------------------ FGMRES
 namespace {
 
-__global__ void k_givens(int j, int ldh, double* H, double* cs, double* sn, double* g, double* est) {
-  pdl_wait_release();
-  double* hj = H + (long long)j * ldh;  // column j, rows 0..j+1
-  for (int i = 0; i < j; ++i) {
-    double t = cs[i] * hj[i] + sn[i] * hj[i + 1];
-    hj[i + 1] = -sn[i] * hj[i] + cs[i] * hj[i + 1];
-    hj[i] = t;
-  }
-  double a = hj[j], b = hj[j + 1];
-  double d = hypot(a, b);
-  double c = d > 0 ? a / d : 1.0, s = d > 0 ? b / d : 0.0;
-  cs[j] = c; sn[j] = s;
-  hj[j] = d; hj[j + 1] = 0.0;
-  g[j + 1] = -s * g[j];
-  g[j] = c * g[j];
-  *est = fabs(g[j + 1]);
-}
-__global__ void k_set_hcol(int j, int ldh, double* H, const double* nrm2) {
-  pdl_wait_release();
-  H[(long long)j * ldh + j + 1] = sqrt(*nrm2);
-}
-// y = R^{-1} g (upper triangular k x k, column-major with leading dim ldh)
-__global__ void k_backsolve(int k, int ldh, const double* H, const double* g, double* y) {
-  pdl_wait_release();
-  for (int i = k - 1; i >= 0; --i) {
-    double s = g[i];
-    for (int j = i + 1; j < k; ++j) s -= H[(long long)j * ldh + i] * y[j];
-    y[i] = s / H[(long long)i * ldh + i];
-  }
-}
-__global__ void k_combine(long long n, const double* __restrict__ Z, long long ldz, int k,
-                          const double* __restrict__ y, double* __restrict__ x) {
-  pdl_wait_release();
-  __shared__ double sy[128];
-  for (int q = threadIdx.x; q < k; q += blockDim.x) sy[q] = y[q];
-  __syncthreads();
-  GRID_LOOP(i, n) x[i] = axpy_rows<1>(x[i], sy, k, Z, ldz, i);
-}
-__global__ void k_hadd(int k, double* h, const double* y, const int* pred) {
-  pdl_wait_release();
-  if (pred && *pred == 0) return;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) h[i] += y[i];
-}
 __global__ void k_fill(long long n, double* a, double v) {
   pdl_wait_release(); GRID_LOOP(i, n) a[i] = v; }
-__global__ void k_init_g(double* g, int m1, const double* nrm2) {
-  pdl_wait_release();
-  for (int i = 0; i < m1; ++i) g[i] = 0.0;
-  g[0] = sqrt(*nrm2);
-}
-
 }  // namespace
 
-// Right-preconditioned flexible GMRES on the equilibrated system, with a row
-// weighting wt that selects the minimised norm: wt = 1 gives the reference's
-// equilibrated norm, wt = D^-1/2 (or 1/|a_ii| without equilibration) the Jacobi
-// norm ||D^-1 r||.  Operator K = diag(wt) A_s, preconditioner M(v) = V(v ./ wt).
-// Orthogonalisation is classical Gram-Schmidt with one re-orthogonalisation
-// pass; all reductions use a fixed block count (deterministic).
 namespace {
 struct KrylovModeGuard {
   AMG& h;
@@ -2329,153 +2142,37 @@ struct KrylovModeGuard {
 };
 }  // namespace
 
-void amg_fgmres(AMG& h, const double* b, double* x, const impes_krylov_params& kp,
-                impes_krylov_stats& st, cudaStream_t s) {
-  if (kp.precision == 0) amg_ensure_fp64(h, s);
-  KrylovModeGuard guard(h);
-  struct SolveTimer {
-    cudaStream_t s;
-    int id;
-    ~SolveTimer() { try { timers().end(id, s, 0.0); } catch (...) {} }
-  } solve_timer{s, timers().begin(IMPES_PH_SOLVE, s)};
-  Level& L0 = *h.levels[0];
-  const int n = L0.n;
-  const int m = std::max(1, std::min(kp.restart, 120));
-  if (h.krylov_m != m || h.V.n < (size_t)(m + 1) * n) {
-    h.V.alloc((size_t)(m + 1) * n);
-    h.Z.alloc((size_t)m * n);
-    h.H.alloc((size_t)(m + 2) * (m + 1));
-    h.cs.alloc(m + 1); h.sn.alloc(m + 1); h.g.alloc(m + 2); h.y.alloc(m + 1);
-    h.kw.alloc(n); h.kb.alloc(n); h.kx.alloc(n);
-    h.krylov_m = m;
-  }
-  h.red.ensure((size_t)(m + 2) * kDotBlocks + kDotBlocks);
-  const int ldh = m + 2;
-  const bool jac = kp.norm == IMPES_NORM_JACOBI;
-  double* wt = jac ? h.jac_w.p : h.kw.p;
-  if (!jac) { launch_pdl(k_fill, grid_for(n, TB), TB, 0, s, n, h.kw.p, 1.0); }
-  double* bs = h.kb.p;   // b_s = dhalf .* b
-  double* xs = h.kx.p;   // x_s
-  launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.dhalf_inv.p, b, bs);
-  if (kp.use_x0)
-    { launch_pdl(k_div_convert<double, double>, grid_for(n, TB), TB, 0, s, n, x, h.dhalf_inv.p, xs); }
-  else
-    { launch_pdl(k_zero, grid_for(n, TB), TB, 0, s, n, xs); }
-  IMPES_CHECK_LAUNCH();
-  double* r0 = h.V.p;
-  launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, wt, bs, r0);
-  const double bnorm = std::sqrt(dot_host(h, r0, r0, n, s));
-  st = impes_krylov_stats{0, 0, 0, 0.0, 0.0};
-  if (!(bnorm > 0.0)) {
-    if (!(bnorm == bnorm)) throw Error(IMPES_ERR_NAN, "non-finite right-hand side");
-    launch_pdl(k_zero, grid_for(n, TB), TB, 0, s, n, x);
-    st.converged = 1;
-    return;
-  }
-  double* dscal = h.scal.p;  // [0] squared norm, [1] residual estimate
-  int total = 0;
-  double est_rel = INFINITY;
-  const int prec = kp.precision;
-  if (prec == 1)
-    IMPES_REQUIRE(h.prm.mixed_precision, IMPES_ERR_STATE, "fp32 V-cycle needs mixed_precision=1");
-  while (true) {
-    // V[0] = wt .* (b_s - A_s x_s), beta = ||V[0]||
-    launch_csr<double, Y_B_MINUS_AX>(n, L0.avg_row, L0.rowptr.p, L0.col.p, L0.val.p, xs, bs,
-                                     nullptr, h.V.p, s);
-    launch_pdl(k_mul_inplace, grid_for(n, TB), TB, 0, s, n, h.V.p, wt);
-    launch_pdl(k_multidot, kDotBlocks, TB, 0, s, n, h.V.p, 0, 1, h.V.p, h.red.p);
-    launch_pdl(k_dot_finalize, 1, 32, 0, s, 1, (const double*)h.red.p, dscal, 0, (const int*)nullptr);
-    IMPES_CUDA(cudaMemcpyAsync(h.hbuf.p, dscal, sizeof(double), cudaMemcpyDeviceToHost, s));
-    IMPES_CUDA(cudaStreamSynchronize(s));
-    const double beta = std::sqrt(h.hbuf.p[0]);
-    if (!(beta == beta)) throw Error(IMPES_ERR_NAN, "NaN residual in FGMRES");
-    est_rel = beta / bnorm;
-    st.rel_res = est_rel;
-    if (est_rel < kp.tol || total >= kp.max_iters) break;
-    launch_pdl(k_init_g, 1, 1, 0, s, h.g.p, m + 1, dscal);
-    launch_pdl(k_scale_by_inv_sqrt, grid_for(n, TB), TB, 0, s, n, h.V.p, h.V.p, dscal);
-    int j = 0;
-    for (; j < m && total < kp.max_iters; ++j) {
-      double* vj = h.V.p + (size_t)j * n;
-      double* zj = h.Z.p + (size_t)j * n;
-      double* w = h.V.p + (size_t)(j + 1) * n;
-      // z_j = V(v_j ./ wt)
-      if (prec == 1) {
-        launch_pdl(k_div_convert<double, float>, grid_for(n, TB), TB, 0, s, n, vj, wt, L0.bf.p);
-        float* zf = vcycle_top<float>(h, true, s);
-        launch_pdl(k_convert<float, double>, grid_for(n, TB), TB, 0, s, n, zf, zj);
-      } else {
-        launch_pdl(k_div_convert<double, double>, grid_for(n, TB), TB, 0, s, n, vj, wt, L0.b.p);
-        double* zd = vcycle_top<double>(h, true, s);
-        IMPES_CUDA(cudaMemcpyAsync(zj, zd, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-      }
-      // w = wt .* (A_s z_j)
-      const int tsp = timers().begin(IMPES_PH_SPMV_L0, s);
-      launch_a<double, Y_W_AX>(L0, 0, zj, nullptr, wt, w, s);
-      timers().end(tsp, s, L0.dia_on[0] ? 8.0 * L0.dia_nd * (double)n + 24.0 * n
-                                        : spmv_bytes(8.0, 8.0, L0.nnz, n, n, L0.col16.p ? 2.0 : 4.0) + 8.0 * n);
-      // classical Gram-Schmidt; the second pass only when the first cancelled
-      // more than 0.3 of the norm (flag on the device).  H[j+1, j] holds
-      // ||w||^2 before the first pass until k_set_hcol overwrites it.
-      const int tor = timers().begin(IMPES_PH_ORTHO, s);
-      double* hcol = h.H.p + (size_t)j * ldh;
-      int* reorth = h.iflag.p + 4;
-      const dim3 g1(kDotBlocks, (unsigned)((j + 2 + kMD - 1) / kMD));
-      launch_pdl(k_multidot_g, g1, dim3(TB), 0, s, (long long)n, (const double*)h.V.p, (long long)n, j + 1, 1,
-                 (const double*)w, h.red.p, (const int*)nullptr);
-      launch_pdl(k_dot_finalize, j + 2, 32, 0, s, j + 2, (const double*)h.red.p, hcol, 0, (const int*)nullptr);
-      launch_pdl(k_update, kDotBlocks, TB, 0, s, n, h.V.p, n, j + 1, hcol, w, h.red.p, (const int*)nullptr);
-      launch_pdl(k_dot_finalize, 1, 32, 0, s, 1, (const double*)h.red.p, dscal, 0, (const int*)nullptr);
-      launch_pdl(k_reorth_flag, 1, 1, 0, s, (const double*)dscal, (const double*)(hcol + j + 1), reorth);
-      const dim3 g2(kDotBlocks, (unsigned)((j + 1 + kMD - 1) / kMD));
-      launch_pdl(k_multidot_g, g2, dim3(TB), 0, s, (long long)n, (const double*)h.V.p, (long long)n, j + 1, 0,
-                 (const double*)w, h.red.p, (const int*)reorth);
-      launch_pdl(k_dot_finalize, j + 1, 32, 0, s, j + 1, (const double*)h.red.p, h.y.p, 0, (const int*)reorth);
-      launch_pdl(k_update, kDotBlocks, TB, 0, s, n, h.V.p, n, j + 1, (const double*)h.y.p, w, h.red.p,
-                 (const int*)reorth);
-      launch_pdl(k_dot_finalize, 1, 32, 0, s, 1, (const double*)h.red.p, dscal, 0, (const int*)reorth);
-      launch_pdl(k_hadd, 1, 128, 0, s, j + 1, hcol, (const double*)h.y.p, (const int*)reorth);
-      launch_pdl(k_set_hcol, 1, 1, 0, s, j, ldh, h.H.p, dscal);
-      launch_pdl(k_scale_by_inv_sqrt, grid_for(n, TB), TB, 0, s, n, w, w, dscal);
-      timers().end(tor, s, 8.0 * n * (2.0 * (j + 1) + 3.0));
-      launch_pdl(k_givens, 1, 1, 0, s, j, ldh, h.H.p, h.cs.p, h.sn.p, h.g.p, dscal + 1);
-      IMPES_CHECK_LAUNCH();
-      ++total;
-      IMPES_CUDA(cudaMemcpyAsync(h.hbuf.p, dscal + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
-      IMPES_CUDA(cudaStreamSynchronize(s));
-      timers().harvest();
-      est_rel = h.hbuf.p[0] / bnorm;
-      if (!(est_rel == est_rel)) throw Error(IMPES_ERR_NAN, "NaN in FGMRES");
-      if (est_rel < kp.tol) { ++j; break; }
-    }
-    // x_s += Z y with y = R^-1 g; the loop head re-checks the true residual
-    launch_pdl(k_backsolve, 1, 1, 0, s, j, ldh, h.H.p, h.g.p, h.y.p);
-    launch_pdl(k_combine, grid_for(n, TB), TB, 0, s, n, h.Z.p, n, j, h.y.p, xs);
-    IMPES_CHECK_LAUNCH();
-    st.restarts++;
-  }
-  st.iterations = total;
-  st.converged = est_rel < kp.tol;
-  st.true_rel_res = est_rel;
-  launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.dhalf_inv.p, xs, x);
-  IMPES_CHECK_LAUNCH();
-}
-
 // ===================================================== device-driven FGMRES
-// The FGMRES above with its control on the device, for capture into a CUDA
-// graph: the iteration count, the Arnoldi index j, the convergence test and
-// the restart decision live in FgState, every kernel reads j from there, and a
-// two conditional WHILE nodes, one inside the other, hold the loops: a pass of
-// the inner one is one iteration (preconditioner application, operator product,
-// Gram-Schmidt with the optional second pass, Givens rotation) and its last
-// kernel ends it at the end of a cycle (converged, j == restart or the iteration
-// cap), after back-solving; a pass of the outer one is a cycle, which updates
-// x_s and recomputes the true residual, which decides whether to stop or to
-// restart.  The algorithm of amg_fgmres; no host synchronisation until the
-// caller reads the state after the graph.
+// Arnoldi index, counters, convergence test and restart decision live in FgState
+// on the device.  Captured into a CUDA graph, two conditional WHILE nodes, one
+// inside the other, hold the loops: a pass of the inner one is one iteration
+// (preconditioner application, operator product, Gram-Schmidt with the optional
+// second pass, Givens rotation) and its last kernel ends it at the end of a cycle
+// (converged, j == restart or the iteration cap), after back-solving; a pass of
+// the outer one is a cycle, which updates x_s and recomputes the true residual,
+// which decides whether to stop or to restart.  No host synchronisation until
+// the caller reads the state after the graph.  Without graphs (or with the phase
+// timers on) the host launches the same kernels and reads the state after each.
+//
+// IF nodes for the second pass and the cycle's end, evaluated every iteration,
+// cost more than the launches they saved: 5.67 ms against 3.92 ms for the 64x64
+// two-phase step of 51 iterations.
 namespace {
-__global__ void k_fg_init(FgState* st, const double* part_b, const double* part_r, int nb, double tol,
-                          int max_iters, int m1, double* g, cudaGraphConditionalHandle cond) {
+// A loop node's condition, set by the kernels that decide; without a node (the
+// host drives the loops) nothing is set.
+struct FgCond {
+  cudaGraphConditionalHandle handle;
+  int node;
+  __device__ void set(unsigned v) const { if (node) cudaGraphSetConditional(handle, v); }
+};
+// the solve's limits, kept by k_fg_init
+__global__ void k_fg_params(FgState* st, double tol, int max_iters) {
+  pdl_wait_release();
+  st->tol = tol;
+  st->max_iters = max_iters;
+}
+__global__ void k_fg_init(FgState* st, const double* part_b, const double* part_r, int nb, int m1, double* g,
+                          FgCond outer) {
   pdl_wait_release();
   double b2 = 0.0, r2 = 0.0;
   for (int q = threadIdx.x; q < nb; q += 32) { b2 += part_b[q]; r2 += part_r[q]; }
@@ -2485,22 +2182,24 @@ __global__ void k_fg_init(FgState* st, const double* part_b, const double* part_
   __syncwarp();
   if (threadIdx.x != 0) return;
   FgState t{};
+  t.tol = st->tol;
+  t.max_iters = st->max_iters;
   t.bnorm = sqrt(b2);
   t.beta = sqrt(r2);
   t.rel = t.bnorm > 0.0 ? t.beta / t.bnorm : 0.0;
   t.true_rel = t.rel;
   t.bzero = !(t.bnorm > 0.0);
   t.nan = !(t.beta == t.beta) || !(t.bnorm == t.bnorm);
-  t.converged = t.bzero || t.rel < tol;
-  t.done = t.bzero || t.nan || t.rel < tol || max_iters <= 0;
+  t.converged = t.bzero || t.rel < t.tol;
+  t.done = t.bzero || t.nan || t.rel < t.tol || t.max_iters <= 0;
   *st = t;
   g[0] = t.beta;
-  cudaGraphSetConditional(cond, t.done ? 0u : 1u);
+  outer.set(t.done ? 0u : 1u);
 }
 // a cycle's start: V[0] /= beta, and the inner loop runs
-__global__ void k_fg_scale_v0(long long n, double* V, const FgState* st, cudaGraphConditionalHandle inner) {
+__global__ void k_fg_scale_v0(long long n, double* V, const FgState* st, FgCond inner) {
   pdl_wait_release();
-  if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(inner, 1u);
+  if (blockIdx.x == 0 && threadIdx.x == 0) inner.set(1u);
   const double inv = 1.0 / st->beta;
   GRID_LOOP(i, n) V[i] *= inv;
 }
@@ -2577,8 +2276,8 @@ __global__ void __launch_bounds__(TB) k_fg_op(int n, const int* __restrict__ row
 // condition and, at a cycle's end, y = R^-1 g column by column.  The column and
 // the rotations are staged in shared memory (sm: 5 * 128 doubles), so the serial
 // part waits on no global load.
-__device__ void fg_column(double* H, int ldh, double* cs, double* sn, double* g, double* y, FgState* st, double tol,
-                          int max_iters, int m, cudaGraphConditionalHandle inner, double* sm) {
+__device__ void fg_column(double* H, int ldh, double* cs, double* sn, double* g, double* y, FgState* st, int m,
+                          FgCond inner, double* sm) {
   double *hj = sm, *c_ = sm + 128, *s_ = c_ + 128, *gg = s_ + 128, *yy = gg + 128;
   const int j = st->j;
   double* Hj = H + (long long)j * ldh;
@@ -2612,8 +2311,9 @@ __device__ void fg_column(double* H, int ldh, double* cs, double* sn, double* g,
     st->j = j + 1;
     const bool nan = !(est == est);
     if (nan) st->nan = 1;
-    const bool end = nan || est < tol || j + 1 >= m || st->total >= max_iters;
-    cudaGraphSetConditional(inner, end ? 0u : 1u);
+    const bool end = nan || est < st->tol || j + 1 >= m || st->total >= st->max_iters;
+    st->cycle_end = end;
+    inner.set(end ? 0u : 1u);
     s_end = end && !nan;
   }
   __syncthreads();
@@ -2776,8 +2476,7 @@ __device__ __forceinline__ void gs_pick(long long n, const double* V, int k, dou
 template <int PASS>
 __global__ void __launch_bounds__(TB, 2) k_fg_gs(long long n, double* V, double* partial, double* H, int ldh,
                                                  double* y, FgState* st, double* cs, double* sn, double* g,
-                                                 double tol, int max_iters, int m,
-                                                 cudaGraphConditionalHandle inner) {
+                                                 int m, FgCond inner) {
   extern __shared__ __align__(16) unsigned char gs_smem[];
   GsSmem& sm = *reinterpret_cast<GsSmem*>(gs_smem);
   double* scratch = reinterpret_cast<double*>(gs_smem);
@@ -2785,7 +2484,7 @@ __global__ void __launch_bounds__(TB, 2) k_fg_gs(long long n, double* V, double*
   __shared__ int s_last;
   pdl_wait_release();
   if (PASS == 2 && !st->reorth) {
-    if (blockIdx.x == 0) fg_column(H, ldh, cs, sn, g, y, st, tol, max_iters, m, inner, scratch);
+    if (blockIdx.x == 0) fg_column(H, ldh, cs, sn, g, y, st, m, inner, scratch);
     return;
   }
   const int j = st->j, k = j + 1;
@@ -2832,7 +2531,7 @@ __global__ void __launch_bounds__(TB, 2) k_fg_gs(long long n, double* V, double*
   if (threadIdx.x == 0) st->gs_count = 0;
   if (PASS == 2) {
     __syncthreads();
-    fg_column(H, ldh, cs, sn, g, y, st, tol, max_iters, m, inner, scratch);
+    fg_column(H, ldh, cs, sn, g, y, st, m, inner, scratch);
   }
 }
 // at a cycle's end x_s += Z y ...
@@ -2844,7 +2543,7 @@ __global__ void k_fg_combine(long long n, const double* __restrict__ Z, const do
   const int k = st->j;
   for (int q = threadIdx.x; q < k; q += blockDim.x) sy[q] = y[q];
   __syncthreads();
-  GRID_LOOP(i, n) x[i] = axpy_rows<1>(x[i], sy, k, Z, n, i);
+  GRID_LOOP(i, n) x[i] = axpy_rows(x[i], sy, k, Z, n, i);
 }
 // ... the true residual V[0] = wt .* (b_s - A_s x_s) and its norm partials ...
 template <typename CT, int LPR>
@@ -2884,8 +2583,8 @@ __global__ void __launch_bounds__(TB) k_fg_resid(int n, const int* __restrict__ 
 }
 // ... and the decision: stop (converged in the true residual, or the cap) or
 // restart with g = beta e_1.
-__global__ void k_fg_restart(const double* partial, int nb, FgState* st, double* g, int m1, double tol,
-                             int max_iters, cudaGraphConditionalHandle cond) {
+__global__ void k_fg_restart(const double* partial, int nb, FgState* st, double* g, int m1,
+                             FgCond outer) {
   pdl_wait_release();
   double r2 = 0.0;
   for (int q = threadIdx.x; q < nb; q += 32) r2 += partial[q];
@@ -2894,7 +2593,7 @@ __global__ void k_fg_restart(const double* partial, int nb, FgState* st, double*
   if (st->nan) {
     st->done = 1;
     st->converged = 0;
-    cudaGraphSetConditional(cond, 0u);
+    outer.set(0u);
     return;
   }
   const double beta = sqrt(r2);
@@ -2903,14 +2602,14 @@ __global__ void k_fg_restart(const double* partial, int nb, FgState* st, double*
   st->rel = st->true_rel;
   st->restarts += 1;
   if (!(beta == beta)) st->nan = 1;
-  st->converged = st->true_rel < tol;
-  st->done = st->nan || st->converged || st->total >= max_iters;
+  st->converged = st->true_rel < st->tol;
+  st->done = st->nan || st->converged || st->total >= st->max_iters;
   if (!st->done) {
     st->j = 0;
     for (int i = 0; i < m1; ++i) g[i] = 0.0;
     g[0] = beta;
   }
-  cudaGraphSetConditional(cond, st->done ? 0u : 1u);
+  outer.set(st->done ? 0u : 1u);
 }
 __global__ void k_fg_final(long long n, const double* dhalf, const double* xs, double* x, const FgState* st) {
   pdl_wait_release();
@@ -3026,13 +2725,12 @@ void capture_while(cudaStream_t s, cudaStream_t& body, cudaGraphConditionalHandl
   IMPES_CUDA(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
 }
 
-void launch_gs(AMG& h, long long n, int ldh, const impes_krylov_params& kp, int m, cudaGraphConditionalHandle inner,
-               cudaStream_t s) {
+void launch_gs(AMG& h, long long n, int ldh, int m, FgCond inner, cudaStream_t s) {
   const int grid = (int)std::min<long long>(kGsBlocks, (n + 31) / 32);
   auto run = [&](auto* kern) {
     raise_smem_limit((const void*)kern, sizeof(GsSmem));
     launch_pdl(kern, grid, TB, sizeof(GsSmem), s, n, h.V.p, h.red.p, h.H.p, ldh, h.y.p, h.fgst.p, h.cs.p, h.sn.p,
-               h.g.p, kp.tol, kp.max_iters, m, inner);
+               h.g.p, m, inner);
   };
   run(k_fg_gs<0>);
   run(k_fg_gs<1>);
@@ -3044,97 +2742,239 @@ void amg_fgmres_prepare(AMG& h, const impes_krylov_params& kp) {
   Level& L0 = *h.levels[0];
   const int n = L0.n;
   const int m = std::max(1, std::min(kp.restart, 120));
-  if (h.krylov_m != m || h.V.n < (size_t)(m + 1) * n) {
+  const size_t red = (size_t)(m + 2) * kDotBlocks + 2 * kDotBlocks;
+  if (h.krylov_m != m || h.V.n < (size_t)(m + 1) * n || h.red.n < red) {
+    h.drop_graphs();               // they hold the old buffers' addresses
     h.V.alloc((size_t)(m + 1) * n);
     h.Z.alloc((size_t)m * n);
     h.H.alloc((size_t)(m + 2) * (m + 1));
     h.cs.alloc(m + 1); h.sn.alloc(m + 1); h.g.alloc(m + 2); h.y.alloc(m + 1);
     h.kw.alloc(n); h.kb.alloc(n); h.kx.alloc(n);
+    h.red.ensure(red);
     h.krylov_m = m;
   }
-  h.red.ensure((size_t)(m + 2) * kDotBlocks + 2 * kDotBlocks);
   h.fgst.ensure(1);
   if (kp.precision == 1)
     IMPES_REQUIRE(h.prm.mixed_precision, IMPES_ERR_STATE, "fp32 V-cycle needs mixed_precision=1");
 }
 
+namespace {
+// before the loops: b_s and x_s from the caller's vectors, the limits
+void fg_prologue(AMG& h, const double* b, const double* x, const impes_krylov_params& kp, cudaStream_t s) {
+  const long long n = h.levels[0]->n;
+  const unsigned gn = grid_for(n, TB);
+  if (kp.norm != IMPES_NORM_JACOBI) launch_pdl(k_fill, gn, TB, 0, s, n, h.kw.p, 1.0);
+  launch_pdl(k_mul, gn, TB, 0, s, n, (const double*)h.dhalf_inv.p, b, h.kb.p);
+  if (kp.use_x0)
+    launch_pdl(k_div_convert<double, double>, gn, TB, 0, s, n, x, (const double*)h.dhalf_inv.p, h.kx.p);
+  else
+    launch_pdl(k_zero, gn, TB, 0, s, n, h.kx.p);
+  launch_pdl(k_fg_params, 1, 1, 0, s, h.fgst.p, kp.tol, kp.max_iters);
+}
+// after them: x = D^-1/2 x_s (zero for a zero right-hand side)
+void fg_epilogue(AMG& h, double* x, cudaStream_t s) {
+  const long long n = h.levels[0]->n;
+  launch_pdl(k_fg_final, grid_for(n, TB), TB, 0, s, n, (const double*)h.dhalf_inv.p, (const double*)h.kx.p, x,
+             (const FgState*)h.fgst.p);
+}
+// The solve between them, on the handle's own buffers only.
+struct Fgmres {
+  AMG& h;
+  Level& L0;
+  long long n;
+  int m, ldh, precision;
+  bool fuse0;
+  unsigned gn;
+  double *wt, *bs, *xs, *part_b, *part_r;
+  FgState* st;
+  Fgmres(AMG& a, bool jac, int prec) : h(a), L0(*a.levels[0]) {
+    n = L0.n;
+    m = h.krylov_m;
+    ldh = m + 2;
+    precision = prec;
+    // the l1-Jacobi V-cycle's first level-0 sweep is fused with the input
+    // conversion (not for Chebyshev smoothing or a one-level hierarchy)
+    fuse0 = h.prm.smoother != IMPES_SMOOTHER_CHEBYSHEV && !L0.coarsest;
+    gn = grid_for(n, TB);
+    wt = jac ? h.jac_w.p : h.kw.p;
+    bs = h.kb.p;
+    xs = h.kx.p;
+    part_b = h.red.p + (size_t)(m + 2) * kDotBlocks;
+    part_r = part_b + kDotBlocks;
+    st = h.fgst.p;
+  }
+  // ||wt b_s||, V[0] = wt (b_s - A x_s) and its norm
+  void start(FgCond outer, cudaStream_t s) const {
+    launch_pdl(k_mul, gn, TB, 0, s, n, (const double*)wt, (const double*)bs, h.V.p);
+    launch_pdl(k_fg_norm_partials, kDotBlocks, TB, 0, s, n, (const double*)h.V.p, part_b);
+    launch_csr<double, Y_B_MINUS_AX>((int)n, L0.avg_row, L0.rowptr.p, L0.col.p, L0.val.p, xs, bs, nullptr, h.V.p, s,
+                                     L0.col16.p, L0.col16_rel, L0.lpr_a[0]);
+    launch_pdl(k_mul_inplace, gn, TB, 0, s, n, h.V.p, (const double*)wt);
+    launch_pdl(k_fg_norm_partials, kDotBlocks, TB, 0, s, n, (const double*)h.V.p, part_r);
+    launch_pdl(k_fg_init, 1, 32, 0, s, st, (const double*)part_b, (const double*)part_r, (int)kDotBlocks, m + 1, h.g.p,
+               outer);
+  }
+  void begin_cycle(FgCond inner, cudaStream_t s) const {
+    launch_pdl(k_fg_scale_v0, gn, TB, 0, s, n, h.V.p, (const FgState*)st, inner);
+  }
+  // z = M^-1 (V[j] / wt); the operator kernel also stores Z[j] = z
+  template <typename T>
+  void precondition(T* b0, T* x0, const T* inv0, cudaStream_t s) const {
+    if (fuse0)
+      launch_pdl(k_fg_prec_smooth0<T>, gn, TB, 0, s, n, h.V.p, (const double*)wt, inv0, b0, x0, (const FgState*)st);
+    else
+      launch_pdl(k_fg_prec_in<T>, gn, TB, 0, s, n, h.V.p, (const double*)wt, b0, (const FgState*)st);
+    const T* z = vcycle<T>(h, 0, true, s, fuse0);
+    const int tsp = timers().begin(IMPES_PH_SPMV_L0, s);
+    if (L0.col16.p) fg_op(L0, (const unsigned short*)L0.col16.p, z, h.Z.p, wt, h.V.p, L0.col16_rel, st, s);
+    else fg_op(L0, (const int*)L0.col.p, z, h.Z.p, wt, h.V.p, 0, st, s);
+    timers().end(tsp, s, L0.dia_on[0] ? 8.0 * L0.dia_nd * (double)n + 24.0 * n
+                                      : spmv_bytes(8.0, 8.0, L0.nnz, n, n, L0.col16.p ? 2.0 : 4.0) + 8.0 * n);
+  }
+  // j: the iteration's index in its cycle when the host knows it (phase bytes)
+  void iterate(FgCond inner, cudaStream_t s, int j = 0) const {
+    if (precision == 1) precondition<float>(L0.bf.p, L0.xf.p, L0.inv_relaxf.p, s);
+    else precondition<double>(L0.b.p, L0.x.p, L0.inv_relax.p, s);
+    // (V[j+1] is normalised by the next iteration's input kernel)
+    const int tor = timers().begin(IMPES_PH_ORTHO, s);
+    launch_gs(h, n, ldh, m, inner, s);
+    timers().end(tor, s, 8.0 * n * (2.0 * (j + 1) + 3.0));
+  }
+  // x_s += Z y, the true residual, the restart/stop decision
+  void end_cycle(FgCond outer, cudaStream_t s) const {
+    launch_pdl(k_fg_combine, gn, TB, 0, s, n, (const double*)h.Z.p, (const double*)h.y.p, xs, (const FgState*)st);
+    if (L0.col16.p) fg_resid<unsigned short>(L0, L0.col16.p, xs, bs, wt, h.V.p, L0.col16_rel, part_r, st, s);
+    else fg_resid<int>(L0, L0.col.p, xs, bs, wt, h.V.p, 0, part_r, st, s);
+    launch_pdl(k_fg_restart, 1, 32, 0, s, (const double*)part_r, (int)kDotBlocks, st, h.g.p, m + 1, outer);
+  }
+  void capture(cudaStream_t s) const {
+    cudaStreamCaptureStatus cst;
+    cudaGraph_t cap = nullptr;
+    IMPES_CUDA(cudaStreamGetCaptureInfo(s, &cst, nullptr, &cap, nullptr, nullptr));
+    IMPES_REQUIRE(cst == cudaStreamCaptureStatusActive, IMPES_ERR_STATE, "device FGMRES needs a capturing stream");
+    FgCond outer{0, 1};
+    IMPES_CUDA(cudaGraphConditionalHandleCreate(&outer.handle, cap, 1, cudaGraphCondAssignDefault));
+    start(outer, s);
+    const unsigned long long mark = thread_launches();
+    capture_while(s, h.body_stream, outer.handle, [&](cudaGraph_t body) {
+      FgCond inner{0, 1};
+      IMPES_CUDA(cudaGraphConditionalHandleCreate(&inner.handle, body, 0, cudaGraphCondAssignDefault));
+      begin_cycle(inner, h.body_stream);
+      const unsigned long long mark_in = thread_launches();
+      capture_while(h.body_stream, h.inner_stream, inner.handle, [&](cudaGraph_t) { iterate(inner, h.inner_stream); });
+      h.fg_body_kernels = (long long)(thread_launches() - mark_in);
+      end_cycle(outer, h.body_stream);
+    });
+    h.fg_end_kernels = (long long)(thread_launches() - mark) - h.fg_body_kernels;
+  }
+};
+FgState* fg_read(AMG& h, cudaStream_t s) {
+  IMPES_CHECK_LAUNCH();
+  FgState* hs = reinterpret_cast<FgState*>(h.hbuf.p);
+  IMPES_CUDA(cudaMemcpyAsync(hs, h.fgst.p, sizeof(FgState), cudaMemcpyDeviceToHost, s));
+  IMPES_CUDA(cudaStreamSynchronize(s));
+  timers().harvest();
+  return hs;
+}
+
+// The captured solve of these settings, made on first use; null when this build
+// or driver refuses the capture.
+AMG::FgGraph* fg_graph(AMG& h, const impes_krylov_params& kp) {
+  const bool jac = kp.norm == IMPES_NORM_JACOBI;
+  for (auto& e : h.fg_graphs)
+    if (e.jac == jac && e.precision == kp.precision) return &e;
+  if (!h.cap_stream) IMPES_CUDA(cudaStreamCreateWithFlags(&h.cap_stream, cudaStreamNonBlocking));
+  AMG::FgGraph e;
+  e.jac = jac;
+  e.precision = kp.precision;
+  const unsigned long long before = thread_launches();
+  if (cudaStreamBeginCapture(h.cap_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  cudaGraph_t graph = nullptr;
+  bool ok = true;
+  try {
+    Fgmres(h, jac, kp.precision).capture(h.cap_stream);
+  } catch (const Error&) {
+    ok = false;
+  }
+  ok = cudaStreamEndCapture(h.cap_stream, &graph) == cudaSuccess && ok;
+  ok = ok && cudaGraphInstantiate(&e.exec, graph, 0) == cudaSuccess;
+  if (graph) cudaGraphDestroy(graph);
+  const long long all = (long long)(thread_launches() - before);
+  count_launches(-all);
+  if (!ok) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  e.kernels_body = h.fg_body_kernels;
+  e.kernels_end = h.fg_end_kernels;
+  e.kernels_fixed = all - e.kernels_body - e.kernels_end;
+  h.fg_graphs.push_back(e);
+  return &h.fg_graphs.back();
+}
+}  // namespace
+
 void amg_fgmres_capture(AMG& h, const double* b, double* x, const impes_krylov_params& kp, cudaStream_t s) {
   KrylovModeGuard guard(h);
   // part of the captured work: every replay follows an update of the values
   amg_dense_form(h, kp.precision == 1 ? 1 : 0, true, s);
-  Level& L0 = *h.levels[0];
-  const long long n = L0.n;
-  const int m = h.krylov_m;
-  const int ldh = m + 2;
-  const bool jac = kp.norm == IMPES_NORM_JACOBI;
-  double* wt = jac ? h.jac_w.p : h.kw.p;
-  double* bs = h.kb.p;
-  double* xs = h.kx.p;
-  double* part_b = h.red.p + (size_t)(m + 2) * kDotBlocks;
-  double* part_r = part_b + kDotBlocks;
-  FgState* st = h.fgst.p;
-  const unsigned gn = grid_for(n, TB);
-  // prologue: b_s, x_s, ||wt b_s||, V[0] = wt (b_s - A x_s) and its norm
-  if (!jac) launch_pdl(k_fill, gn, TB, 0, s, n, h.kw.p, 1.0);
-  launch_pdl(k_mul, gn, TB, 0, s, n, (const double*)h.dhalf_inv.p, b, bs);
-  if (kp.use_x0)
-    launch_pdl(k_div_convert<double, double>, gn, TB, 0, s, n, (const double*)x, (const double*)h.dhalf_inv.p, xs);
-  else
-    launch_pdl(k_zero, gn, TB, 0, s, n, xs);
-  launch_pdl(k_mul, gn, TB, 0, s, n, (const double*)wt, (const double*)bs, h.V.p);
-  launch_pdl(k_fg_norm_partials, kDotBlocks, TB, 0, s, n, (const double*)h.V.p, part_b);
-  launch_csr<double, Y_B_MINUS_AX>((int)n, L0.avg_row, L0.rowptr.p, L0.col.p, L0.val.p, xs, bs, nullptr, h.V.p, s,
-                                   L0.col16.p, L0.col16_rel, L0.lpr_a[0]);
-  launch_pdl(k_mul_inplace, gn, TB, 0, s, n, h.V.p, (const double*)wt);
-  launch_pdl(k_fg_norm_partials, kDotBlocks, TB, 0, s, n, (const double*)h.V.p, part_r);
-  // the cycles; the init kernel sets the outer condition (0: nothing to do)
-  cudaStreamCaptureStatus cst;
-  cudaGraph_t cap = nullptr;
-  IMPES_CUDA(cudaStreamGetCaptureInfo(s, &cst, nullptr, &cap, nullptr, nullptr));
-  IMPES_REQUIRE(cst == cudaStreamCaptureStatusActive, IMPES_ERR_STATE, "device FGMRES needs a capturing stream");
-  cudaGraphConditionalHandle outer;
-  IMPES_CUDA(cudaGraphConditionalHandleCreate(&outer, cap, 1, cudaGraphCondAssignDefault));
-  launch_pdl(k_fg_init, 1, 32, 0, s, st, (const double*)part_b, (const double*)part_r, (int)kDotBlocks, kp.tol,
-             kp.max_iters, m + 1, h.g.p, outer);
-  const unsigned long long mark = thread_launches();
-  capture_while(s, h.body_stream, outer, [&](cudaGraph_t body) {
-    cudaStream_t bs_ = h.body_stream;
-    cudaGraphConditionalHandle inner;
-    IMPES_CUDA(cudaGraphConditionalHandleCreate(&inner, body, 0, cudaGraphCondAssignDefault));
-    launch_pdl(k_fg_scale_v0, gn, TB, 0, bs_, n, h.V.p, (const FgState*)st, inner);
-    const unsigned long long mark_in = thread_launches();
-    capture_while(bs_, h.inner_stream, inner, [&](cudaGraph_t) {
-      cudaStream_t q = h.inner_stream;
-      // z = M^-1 (V[j] / wt); Z[j] = z is written by the operator kernel.  The
-      // l1-Jacobi V-cycle's first level-0 sweep is fused with the input
-      // conversion (not for Chebyshev smoothing or a one-level hierarchy)
-      const bool fuse0 = h.prm.smoother != IMPES_SMOOTHER_CHEBYSHEV && !L0.coarsest;
-      auto precondition = [&](auto* b0, auto* x0, const auto* inv0) {
-        using T = std::remove_pointer_t<decltype(b0)>;
-        if (fuse0) launch_pdl(k_fg_prec_smooth0<T>, gn, TB, 0, q, n, h.V.p, (const double*)wt, inv0, b0, x0, (const FgState*)st);
-        else launch_pdl(k_fg_prec_in<T>, gn, TB, 0, q, n, h.V.p, (const double*)wt, b0, (const FgState*)st);
-        const T* z = vcycle<T>(h, 0, true, q, fuse0);
-        if (L0.col16.p) fg_op(L0, (const unsigned short*)L0.col16.p, z, h.Z.p, wt, h.V.p, L0.col16_rel, st, q);
-        else fg_op(L0, (const int*)L0.col.p, z, h.Z.p, wt, h.V.p, 0, st, q);
-      };
-      if (kp.precision == 1) precondition(L0.bf.p, L0.xf.p, (const float*)L0.inv_relaxf.p);
-      else precondition(L0.b.p, L0.x.p, (const double*)L0.inv_relax.p);
-      // (V[j+1] is normalised by the next iteration's input kernel)
-      launch_gs(h, n, ldh, kp, m, inner, q);
-    });
-    h.fg_body_kernels = (long long)(thread_launches() - mark_in);
-    // a cycle's end: x_s += Z y, the true residual, the restart/stop decision
-    launch_pdl(k_fg_combine, gn, TB, 0, bs_, n, (const double*)h.Z.p, (const double*)h.y.p, xs, (const FgState*)st);
-    if (L0.col16.p)
-      fg_resid<unsigned short>(L0, L0.col16.p, xs, bs, wt, h.V.p, L0.col16_rel, part_r, st, bs_);
-    else
-      fg_resid<int>(L0, L0.col.p, xs, bs, wt, h.V.p, 0, part_r, st, bs_);
-    launch_pdl(k_fg_restart, 1, 32, 0, bs_, (const double*)part_r, (int)kDotBlocks, st, h.g.p, m + 1, kp.tol,
-               kp.max_iters, outer);
-  });
-  h.fg_end_kernels = (long long)(thread_launches() - mark) - h.fg_body_kernels;
-  // epilogue: x = D^-1/2 x_s (zero for a zero right-hand side)
-  launch_pdl(k_fg_final, gn, TB, 0, s, n, (const double*)h.dhalf_inv.p, (const double*)xs, x, (const FgState*)st);
+  fg_prologue(h, b, x, kp, s);
+  Fgmres(h, kp.norm == IMPES_NORM_JACOBI, kp.precision).capture(s);
+  fg_epilogue(h, x, s);
+}
+
+// Right-preconditioned flexible GMRES on the equilibrated system, with a row
+// weighting wt that selects the minimised norm: wt = 1 gives the reference's
+// equilibrated norm, wt = D^-1/2 (or 1/|a_ii| without equilibration) the Jacobi
+// norm ||D^-1 r||.  Operator K = diag(wt) A_s, preconditioner M(v) = V(v ./ wt).
+// One graph launch and one host synchronisation; the captured solve runs on the
+// handle's own vectors, so it serves any b and x (84 iterations at 330,000 rows:
+// 32.5 ms driven from the host).
+void amg_fgmres(AMG& h, const double* b, double* x, const impes_krylov_params& kp, impes_krylov_stats& st,
+                cudaStream_t s) {
+  if (kp.precision == 0) amg_ensure_fp64(h, s);
+  KrylovModeGuard guard(h);
+  struct SolveTimer {
+    cudaStream_t s;
+    int id;
+    ~SolveTimer() { try { timers().end(id, s, 0.0); } catch (...) {} }
+  } solve_timer{s, timers().begin(IMPES_PH_SOLVE, s)};
+  amg_fgmres_prepare(h, kp);
+  AMG::FgGraph* g = nullptr;
+  if (h.use_graphs && h.use_step_graph && !h.fg_graph_failed && !timers().on) {
+    g = fg_graph(h, kp);
+    h.fg_graph_failed = g == nullptr;
+  }
+  if (kp.precision == 1) dense_ensure<float>(h, s);
+  else dense_ensure<double>(h, s);
+  fg_prologue(h, b, x, kp, s);
+  FgState* hs = nullptr;
+  if (g) {
+    IMPES_CUDA(cudaGraphLaunch(g->exec, s));
+    fg_epilogue(h, x, s);
+    hs = fg_read(h, s);
+    count_launches(g->kernels_fixed + (long long)hs->total * g->kernels_body + (long long)hs->restarts * g->kernels_end);
+  } else {
+    const Fgmres f(h, kp.norm == IMPES_NORM_JACOBI, kp.precision);
+    const FgCond none{0, 0};
+    f.start(none, s);
+    for (hs = fg_read(h, s); !hs->done; hs = fg_read(h, s)) {
+      f.begin_cycle(none, s);
+      int j = 0;
+      do {
+        f.iterate(none, s, j++);
+        hs = fg_read(h, s);
+      } while (!hs->cycle_end);
+      f.end_cycle(none, s);
+    }
+    fg_epilogue(h, x, s);
+    IMPES_CHECK_LAUNCH();
+  }
+  if (!(hs->bnorm == hs->bnorm)) throw Error(IMPES_ERR_NAN, "non-finite right-hand side");
+  if (hs->nan) throw Error(IMPES_ERR_NAN, "NaN in FGMRES");
+  st = impes_krylov_stats{hs->total, hs->restarts, hs->converged ? 1 : 0, hs->rel, hs->true_rel};
 }
 
 }  // namespace impes
