@@ -344,45 +344,76 @@ __global__ void k_p_count(int n, const int* rowptr, const int* col, const unsign
 }
 __device__ __forceinline__ double nan_to_zero(double v) { return isfinite(v) ? v : 0.0; }
 
-__global__ void k_p_fill(int n, const int* rowptr, const int* col, const double* val,
-                         const unsigned char* strong, const signed char* cf, const int* f2c,
-                         const double* pdiag, const double* ssum, const double* wcsum,
-                         const double* wfsum, const int* scnt, const int* cptr, int* ccol,
-                         double* cval) {
-  GRID_LOOP(i, n) {
+// One warp per row: the terms of a row are found by ballot and written in the
+// order a walk over the row would meet them, and the weak sum adds its terms in
+// that order too.  (A thread per row walked the hundreds of entries of a coarse
+// level's rows, and each neighbour's, one dependent load after another: 1.48 ms
+// a level at 16,497 rows.)
+__global__ void __launch_bounds__(256) k_p_fill(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
+                                                const double* __restrict__ val,
+                                                const unsigned char* __restrict__ strong,
+                                                const signed char* __restrict__ cf, const int* __restrict__ f2c,
+                                                const double* __restrict__ pdiag, const double* __restrict__ ssum,
+                                                const double* __restrict__ wcsum, const double* __restrict__ wfsum,
+                                                const int* __restrict__ scnt, const int* __restrict__ cptr,
+                                                int* __restrict__ ccol, double* __restrict__ cval) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
     int o = cptr[i];
-    if (cf[i] == 0) { ccol[o] = f2c[i]; cval[o] = 1.0; continue; }
+    if (cf[i] == 0) {
+      if (lane == 0) { ccol[o] = f2c[i]; cval[o] = 1.0; }
+      continue;
+    }
     const int a = rowptr[i], b = rowptr[i + 1];
     const double di = pdiag[i];
     double fws = wfsum[i];
-    for (int e = a; e < b; ++e) {  // invalid F-F entries join the weak sum (:280-284)
-      int j = col[e];
-      if (j != i && strong[e] && cf[j] == 1 && !ff_valid(j, scnt, ssum)) fws += -val[e];
+    for (int e0 = a; e0 < b; e0 += 32) {  // invalid F-F entries join the weak sum (:280-284)
+      const int e = e0 + lane;
+      const int j = e < b ? col[e] : i;
+      const bool in = j != i && strong[e] && cf[j] == 1 && !ff_valid(j, scnt, ssum);
+      const double t = in ? -val[e] : 0.0;
+      for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1) fws += __shfl_sync(0xffffffffu, t, __ffs(m) - 1);
     }
     const double tw = wcsum[i] + fws;
     const double corr = ssum[i] > 1e-14 ? tw / ssum[i] : 0.0;
-    for (int e = a; e < b; ++e) {  // direct RS weights (:240-246, 292-296)
-      int j = col[e];
-      if (j != i && strong[e] && cf[j] == 0) {
-        double v = nan_to_zero(-val[e] / di) * (1.0 + corr);
-        ccol[o] = f2c[j];
-        cval[o] = v < 0.0 ? 0.0 : v;
-        ++o;
+    for (int e0 = a; e0 < b; e0 += 32) {  // direct RS weights (:240-246, 292-296)
+      const int e = e0 + lane;
+      const int j = e < b ? col[e] : i;
+      const bool in = j != i && strong[e] && cf[j] == 0;
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (in) {
+        const double v = nan_to_zero(-val[e] / di) * (1.0 + corr);
+        const int at = o + __popc(m & below);
+        ccol[at] = f2c[j];
+        cval[at] = v < 0.0 ? 0.0 : v;
       }
+      o += __popc(m);
     }
-    for (int e = a; e < b; ++e) {  // F-F distribution (:248-278)
-      int j = col[e];
-      if (j == i || !strong[e] || cf[j] != 1 || !ff_valid(j, scnt, ssum)) continue;
-      const double fac = nan_to_zero(-val[e] / di);
-      const double sj = ssum[j];
-      for (int f = rowptr[j]; f < rowptr[j + 1]; ++f) {
-        int c = col[f];
-        if (c != j && strong[f] && cf[c] == 0) {
-          double w = sj > 1e-14 ? -val[f] / sj : 0.0;
-          double v = fac * w;
-          ccol[o] = f2c[c];
-          cval[o] = v < 0.0 ? 0.0 : v;
-          ++o;
+    for (int e0 = a; e0 < b; e0 += 32) {  // F-F distribution (:248-278)
+      const int e = e0 + lane;
+      const int j = e < b ? col[e] : i;
+      const bool in = j != i && strong[e] && cf[j] == 1 && ff_valid(j, scnt, ssum);
+      const double fac_l = in ? nan_to_zero(-val[e] / di) : 0.0;
+      for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const int jj = __shfl_sync(0xffffffffu, j, src);
+        const double fac = __shfl_sync(0xffffffffu, fac_l, src);
+        const double sj = ssum[jj];
+        const int f1 = rowptr[jj + 1];
+        for (int f0 = rowptr[jj]; f0 < f1; f0 += 32) {
+          const int f = f0 + lane;
+          const int c = f < f1 ? col[f] : jj;
+          const bool fin = c != jj && strong[f] && cf[c] == 0;
+          const unsigned fm = __ballot_sync(0xffffffffu, fin);
+          if (fin) {
+            const double w = sj > 1e-14 ? -val[f] / sj : 0.0;
+            const double v = fac * w;
+            const int at = o + __popc(fm & below);
+            ccol[at] = f2c[c];
+            cval[at] = v < 0.0 ? 0.0 : v;
+          }
+          o += __popc(fm);
         }
       }
     }
@@ -640,9 +671,6 @@ __host__ __device__ __forceinline__ int hash_cap(int bound) {
 // Rows with more than kWideBound candidates keep their hash table in global
 // scratch (offset goff[r], table + list of cap ints each); others use shared memory.
 constexpr int kWideBound = 2048;
-__global__ void k_wide_size(int rows, const int* bound, long long* gsize) {
-  GRID_LOOP(r, rows) gsize[r] = bound[r] > kWideBound ? 2LL * hash_cap(bound[r]) : 0LL;
-}
 
 // One warp per output row.  Pass 1 (outcol == nullptr): count distinct columns.
 // Pass 2: write the sorted distinct columns at outptr[row].
@@ -693,60 +721,177 @@ __global__ void k_union_rows(int rows, const int* optr, const int* ocol, const i
 }
 
 // --------------------------------------------------- Galerkin product plans
-// Output position of every (outer entry, inner entry) product, enumerated row
-// by row in (outer, inner) order; kbase = exclusive scan of the row bounds.
-__global__ void k_plan_pos(int rows, const int* optr, const int* ocol, const int* iptr,
-                           const int* icol, const int* outptr, const int* outcol,
-                           const long long* kbase, int* ppos) {
-  GRID_LOOP(r, rows) {
-    long long k = kbase[r];
+// Every (outer entry e, inner entry f) product of row r belongs to one of row r's
+// outputs, so the row's terms fill exactly kbase[r] .. kbase[r+1] (kbase: scan of
+// the rows' product counts) and each row is planned by itself: count per output,
+// scan, fill.  Where the inner columns of an outer entry are distinct, its terms
+// go to distinct outputs; taking the outer entries one after another then leaves
+// every segment in enumeration order with no atomics and no sort.  A row of P
+// that k_p_insert gave an extra first entry may hold that column a second time:
+// with first_apart the first inner entry is taken before the others.  The outer
+// index is remapped by `omap` (R entry -> P entry) when given.
+//
+// (One thread per row found the places, counted, filled by atomics and sorted:
+// 82 ms of a hierarchy of 16,497 rows, against 3.4 ms.)
+//
+// k_plan_group: G lanes per row, an output found by binary search in the row's
+// columns; cur holds the outputs' counters, then cursors.
+template <int G>
+__global__ void __launch_bounds__(256) k_plan_group(int rows, const int* __restrict__ optr,
+                                                    const int* __restrict__ ocol, const int* __restrict__ iptr,
+                                                    const int* __restrict__ icol, const int* __restrict__ outptr,
+                                                    const int* __restrict__ outcol, const int* __restrict__ kbase,
+                                                    const int* __restrict__ omap, int first_apart,
+                                                    int* __restrict__ seg, int* cur, int* __restrict__ pe,
+                                                    int* __restrict__ pf) {
+  const int lane = threadIdx.x % G;
+  const unsigned mask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << ((threadIdx.x & 31) / G * G);
+  const long long groups = (long long)gridDim.x * blockDim.x / G;
+  for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G; r < rows; r += groups) {
     const int ob = outptr[r], L = outptr[r + 1] - ob;
-    for (int e = optr[r]; e < optr[r + 1]; ++e) {
-      const int j = ocol[e];
-      for (int f = iptr[j]; f < iptr[j + 1]; ++f, ++k) {
-        const int key = icol[f];
-        int lo = 0, hi = L - 1;
-        while (lo < hi) {
-          int mid = (lo + hi) >> 1;
-          if (outcol[ob + mid] < key) lo = mid + 1; else hi = mid;
-        }
-        ppos[k] = ob + lo;
+    const int e0 = optr[r], e1 = optr[r + 1];
+    auto find = [&](int key) {
+      int lo = 0, hi = L - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (outcol[ob + mid] < key) lo = mid + 1; else hi = mid;
       }
+      return ob + lo;
+    };
+    for (int x = lane; x < L; x += G) cur[ob + x] = 0;
+    __syncwarp(mask);
+    for (int e = e0; e < e1; ++e) {
+      const int j = ocol[e], f1 = iptr[j + 1];
+      int f0 = iptr[j];
+      if (first_apart && f0 < f1) {
+        if (lane == 0) cur[find(icol[f0])] += 1;
+        __syncwarp(mask);
+        ++f0;
+      }
+      for (int f = f0 + lane; f < f1; f += G) cur[find(icol[f])] += 1;
+      __syncwarp(mask);
     }
-  }
-}
-__global__ void k_plan_count(long long nprod, const int* ppos, int* cnt) {
-  GRID_LOOP(k, nprod) atomicAdd(&cnt[ppos[k]], 1);
-}
-// Scatter products into their output segments; outer index is remapped by
-// `omap` (R entry -> P entry) when given.
-__global__ void k_plan_fill(int rows, const int* optr, const int* ocol, const int* iptr,
-                            const long long* kbase, const int* ppos, const int* omap, int* fill,
-                            long long* key, int* pe, int* pf) {
-  GRID_LOOP(r, rows) {
-    long long k = kbase[r];
-    for (int e = optr[r]; e < optr[r + 1]; ++e) {
-      const int j = ocol[e];
-      const int eo = omap ? omap[e] : e;
-      for (int f = iptr[j]; f < iptr[j + 1]; ++f, ++k) {
-        const int slot = atomicAdd(&fill[ppos[k]], 1);
-        key[slot] = k;
+    int run = kbase[r];
+    for (int x0 = 0; x0 < L; x0 += G) {
+      const int x = x0 + lane;
+      const int v = x < L ? cur[ob + x] : 0;
+      int t = v;
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) {
+        const int up = __shfl_up_sync(mask, t, o, G);
+        if (lane >= o) t += up;
+      }
+      if (x < L) {
+        seg[ob + x] = run + t - v;
+        cur[ob + x] = run + t - v;
+      }
+      run += __shfl_sync(mask, t, G - 1, G);
+    }
+    __syncwarp(mask);
+    for (int e = e0; e < e1; ++e) {
+      const int j = ocol[e], f1 = iptr[j + 1], eo = omap ? omap[e] : e;
+      auto put = [&](int f) {
+        const int at = find(icol[f]);
+        const int slot = cur[at];
+        cur[at] = slot + 1;
         pe[slot] = eo;
         pf[slot] = f;
+      };
+      int f0 = iptr[j];
+      if (first_apart && f0 < f1) {
+        if (lane == 0) put(f0);
+        __syncwarp(mask);
+        ++f0;
       }
+      for (int f = f0 + lane; f < f1; f += G) put(f);
+      __syncwarp(mask);
     }
   }
 }
-// Order every segment by product index: the sums then run in enumeration order.
-__global__ void k_plan_sort(int nout, const int* seg, long long* key, int* pe, int* pf) {
-  GRID_LOOP(o, nout) {
-    const int a = seg[o], b = seg[o + 1];
-    for (int x = a + 1; x < b; ++x) {
-      long long kk = key[x];
-      int e = pe[x], f = pf[x], y = x - 1;
-      while (y >= a && key[y] > kk) { key[y + 1] = key[y]; pe[y + 1] = pe[y]; pf[y + 1] = pf[y]; --y; }
-      key[y + 1] = kk; pe[y + 1] = e; pf[y + 1] = f;
+// k_plan_wide: a block per row of at least kPlanWide products on average and at
+// most kPlanCols output columns, an output found in a column map in shared memory
+// (map[c]: the output of column c in the row; cnt: counters, then cursors).
+constexpr int kPlanWide = 1024, kPlanCols = 12288;
+__global__ void __launch_bounds__(256) k_plan_wide(int rows, int ncols, const int* __restrict__ optr,
+                                                   const int* __restrict__ ocol, const int* __restrict__ iptr,
+                                                   const int* __restrict__ icol, const int* __restrict__ outptr,
+                                                   const int* __restrict__ outcol, const int* __restrict__ kbase,
+                                                   const int* __restrict__ omap, int first_apart,
+                                                   int* __restrict__ seg, int* __restrict__ pe,
+                                                   int* __restrict__ pf) {
+  extern __shared__ int sh_plan[];
+  int* map = sh_plan;
+  int* cnt = map + ncols;
+  __shared__ int s_warp[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    const int ob = outptr[r], L = outptr[r + 1] - ob;
+    const int e0 = optr[r], e1 = optr[r + 1];
+    for (int x = threadIdx.x; x < L; x += 256) {
+      map[outcol[ob + x]] = x;
+      cnt[x] = 0;
     }
+    __syncthreads();
+    for (int e = e0 + warp; e < e1; e += 8) {
+      const int j = ocol[e], f1 = iptr[j + 1];
+      for (int f = iptr[j] + lane; f < f1; f += 32) atomicAdd(&cnt[map[icol[f]]], 1);
+    }
+    __syncthreads();
+    // exclusive scan of cnt, a contiguous piece per thread
+    const int per = (L + 255) / 256, x0 = min(L, (int)threadIdx.x * per), x1 = min(L, x0 + per);
+    int sum = 0;
+    for (int x = x0; x < x1; ++x) sum += cnt[x];
+    int t = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += up;
+    }
+    if (lane == 31) s_warp[warp] = t;
+    __syncthreads();
+    int run = kbase[r] + t - sum;
+    for (int q = 0; q < warp; ++q) run += s_warp[q];
+    for (int x = x0; x < x1; ++x) {
+      const int c = cnt[x];
+      seg[ob + x] = run;
+      cnt[x] = run;
+      run += c;
+    }
+    __syncthreads();
+    for (int e = e0; e < e1; ++e) {
+      const int j = ocol[e], f1 = iptr[j + 1], eo = omap ? omap[e] : e;
+      auto put = [&](int f) {
+        const int at = map[icol[f]];
+        const int slot = cnt[at];
+        cnt[at] = slot + 1;
+        pe[slot] = eo;
+        pf[slot] = f;
+      };
+      int f0 = iptr[j];
+      if (first_apart && f0 < f1) {
+        if (threadIdx.x == 0) put(f0);
+        __syncthreads();
+        ++f0;
+      }
+      for (int f = f0 + threadIdx.x; f < f1; f += 256) put(f);
+      __syncthreads();
+    }
+  }
+}
+// sum of the bounds, and of the wide rows' scratch sizes
+__global__ void k_bound_totals(int rows, const int* bound, unsigned long long* prod, unsigned long long* wide) {
+  unsigned long long a = 0, w = 0;
+  GRID_LOOP(r, rows) {
+    a += (unsigned long long)bound[r];
+    if (bound[r] > kWideBound) w += 2ull * hash_cap(bound[r]);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    w += __shfl_down_sync(0xffffffffu, w, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (prod && a) atomicAdd(prod, a);
+    if (wide && w) atomicAdd(wide, w);
   }
 }
 // out[o] = sum over the segment of a[pe] * b[pf]; one thread per output walks
@@ -1080,22 +1225,27 @@ void union_symbolic(AMG& h, int rows, const int* optr, const int* ocol, const in
   DBuf<int> bound(rows), ucnt(rows + 1);
   k_union_bound<<<grid_for(rows, TB), TB, 0, s>>>(rows, optr, ocol, iptr, bound.p); ::impes::count_launch();
   IMPES_CHECK_LAUNCH();
-  // global scratch for the wide rows
-  DBuf<long long> gsize(rows + 1), goff(rows + 1);
-  k_wide_size<<<grid_for(rows, TB), TB, 0, s>>>(rows, bound.p, gsize.p); ::impes::count_launch();
+  // shared-memory table size for the narrow rows, global scratch for the wide ones
+  struct Sizes { int maxc, pad; unsigned long long wide; } hz{};
+  DBuf<Sizes> sizes(1);
+  IMPES_CUDA(cudaMemsetAsync(sizes.p, 0, sizeof(Sizes), s));
+  k_max_narrow<<<grid_for(rows, TB), TB, 0, s>>>(rows, bound.p, kWideBound, &sizes.p->maxc); ::impes::count_launch();
+  k_bound_totals<<<grid_for(rows, TB), TB, 0, s>>>(rows, bound.p, nullptr, &sizes.p->wide); ::impes::count_launch();
   IMPES_CHECK_LAUNCH();
-  std::vector<long long> hs(rows);
-  IMPES_CUDA(cudaMemcpyAsync(hs.data(), gsize.p, sizeof(long long) * rows, cudaMemcpyDeviceToHost, s));
+  IMPES_CUDA(cudaMemcpyAsync(&hz, sizes.p, sizeof(Sizes), cudaMemcpyDeviceToHost, s));
   IMPES_CUDA(cudaStreamSynchronize(s));
-  std::vector<long long> ho(rows + 1, 0);
-  for (int r = 0; r < rows; ++r) ho[r + 1] = ho[r] + hs[r];
-  IMPES_CUDA(cudaMemcpyAsync(goff.p, ho.data(), sizeof(long long) * (rows + 1), cudaMemcpyHostToDevice, s));
-  DBuf<int> gscratch(std::max<long long>(ho[rows], 1));
-  // shared-memory table size for the narrow rows
-  IMPES_CUDA(cudaMemsetAsync(h.iflag.p, 0, sizeof(int), s));
-  k_max_narrow<<<grid_for(rows, TB), TB, 0, s>>>(rows, bound.p, kWideBound, h.iflag.p); ::impes::count_launch();
-  IMPES_CHECK_LAUNCH();
-  const int maxc = to_host_int(h, h.iflag.p, s);
+  const int maxc = hz.maxc;
+  DBuf<long long> goff(hz.wide ? rows + 1 : 1);
+  if (hz.wide) {
+    std::vector<int> hb(rows);
+    IMPES_CUDA(cudaMemcpyAsync(hb.data(), bound.p, sizeof(int) * rows, cudaMemcpyDeviceToHost, s));
+    IMPES_CUDA(cudaStreamSynchronize(s));
+    std::vector<long long> ho(rows + 1, 0);
+    for (int r = 0; r < rows; ++r) ho[r + 1] = ho[r] + (hb[r] > kWideBound ? 2LL * hash_cap(hb[r]) : 0LL);
+    IMPES_CUDA(cudaMemcpyAsync(goff.p, ho.data(), sizeof(long long) * (rows + 1), cudaMemcpyHostToDevice, s));
+    IMPES_CUDA(cudaStreamSynchronize(s));   // ho goes out of scope
+  }
+  DBuf<int> gscratch(std::max<unsigned long long>(hz.wide, 1));
   const int hsize = hash_cap(maxc);
   const size_t per_warp = sizeof(int) * (2 * (size_t)hsize + 1);
   const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (64u << 10) / per_warp));
@@ -1117,47 +1267,52 @@ void union_symbolic(AMG& h, int rows, const int* optr, const int* ocol, const in
   maxrow = to_host_int(h, h.iflag.p, s);
 }
 
-// Product plan of out = outer * inner on a known output pattern (see Level).
-// Returns false (no plan) when the product count does not fit the memory budget.
-bool build_plan(int rows, const int* optr, const int* ocol, const int* iptr, const int* icol,
-                const int* outptr, const int* outcol, int nout, const int* omap, DBuf<int>& seg,
+// Product plan of out = outer * inner (ncols columns) on a known output pattern
+// (see Level).  Returns false (no plan) when the product count does not fit the
+// memory budget.
+bool build_plan(int rows, int ncols, const int* optr, const int* ocol, const int* iptr, const int* icol,
+                const int* outptr, const int* outcol, int nout, int onnz, const int* omap, bool first_apart, DBuf<int>& seg,
                 DBuf<int>& pe, DBuf<int>& pf, long long& nterms, cudaStream_t s) {
   nterms = 0;
-  DBuf<int> bound(std::max(rows, 1));
+  DBuf<int> bound(std::max(rows, 1)), kbase(rows + 1);
+  DBuf<unsigned long long> total(1);
+  IMPES_CUDA(cudaMemsetAsync(total.p, 0, sizeof(unsigned long long), s));
   k_union_bound<<<grid_for(rows, TB), TB, 0, s>>>(rows, optr, ocol, iptr, bound.p); ::impes::count_launch();
+  k_bound_totals<<<grid_for(rows, TB), TB, 0, s>>>(rows, bound.p, total.p, nullptr); ::impes::count_launch();
   IMPES_CHECK_LAUNCH();
-  std::vector<int> hb(rows);
-  IMPES_CUDA(cudaMemcpyAsync(hb.data(), bound.p, sizeof(int) * rows, cudaMemcpyDeviceToHost, s));
+  unsigned long long ht = 0;
+  IMPES_CUDA(cudaMemcpyAsync(&ht, total.p, sizeof(ht), cudaMemcpyDeviceToHost, s));
   IMPES_CUDA(cudaStreamSynchronize(s));
-  std::vector<long long> hk(rows + 1, 0);
-  for (int r = 0; r < rows; ++r) hk[r + 1] = hk[r] + hb[r];
-  const long long nprod = hk[rows];
-  if (nprod >= (1LL << 31) - 1) return false;
+  if (ht >= (1ull << 31) - 1) return false;
+  const int nprod = (int)ht;
   size_t free_b = 0, total_b = 0;
   IMPES_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  const double keep = 8.0 * nprod + 4.0 * nout, temp = 16.0 * nprod;
-  if (keep + temp > 0.5 * (double)free_b) return false;
-  DBuf<long long> kbase(rows + 1);
-  IMPES_CUDA(cudaMemcpyAsync(kbase.p, hk.data(), sizeof(long long) * (rows + 1), cudaMemcpyHostToDevice, s));
-  DBuf<int> ppos(std::max<long long>(nprod, 1));
-  k_plan_pos<<<grid_for(rows, TB), TB, 0, s>>>(rows, optr, ocol, iptr, icol, outptr, outcol, kbase.p, ppos.p); ::impes::count_launch();
-  IMPES_CHECK_LAUNCH();
-  DBuf<int> cnt(nout + 1), fill(nout + 1);
-  IMPES_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (nout + 1), s));
-  k_plan_count<<<grid_for(nprod, TB), TB, 0, s>>>(nprod, ppos.p, cnt.p); ::impes::count_launch();
-  IMPES_CHECK_LAUNCH();
+  if (8.0 * nprod + 8.0 * nout > 0.5 * (double)free_b) return false;
+  exclusive_scan_i32_dev(bound.p, kbase.p, rows, s);
   seg.alloc(nout + 1);
-  exclusive_scan_i32(cnt.p, seg.p, nout, s);
-  IMPES_CUDA(cudaMemcpyAsync(fill.p, seg.p, sizeof(int) * nout, cudaMemcpyDeviceToDevice, s));
-  DBuf<long long> key(std::max<long long>(nprod, 1));
-  pe.alloc(std::max<long long>(nprod, 1));
-  pf.alloc(std::max<long long>(nprod, 1));
-  k_plan_fill<<<grid_for(rows, TB), TB, 0, s>>>(rows, optr, ocol, iptr, kbase.p, ppos.p, omap, fill.p,
-                                                key.p, pe.p, pf.p); ::impes::count_launch();
-  IMPES_CHECK_LAUNCH();
-  k_plan_sort<<<grid_for(nout, TB), TB, 0, s>>>(nout, seg.p, key.p, pe.p, pf.p); ::impes::count_launch();
-  IMPES_CHECK_LAUNCH();
-  IMPES_CUDA(cudaStreamSynchronize(s));
+  pe.alloc(std::max(nprod, 1));
+  pf.alloc(std::max(nprod, 1));
+  IMPES_CUDA(cudaMemcpyAsync(seg.p + nout, kbase.p + rows, sizeof(int), cudaMemcpyDeviceToDevice, s));
+  if (ncols <= kPlanCols && nprod / std::max(rows, 1) >= kPlanWide) {
+    const size_t smem = sizeof(int) * 2 * (size_t)ncols;
+    raise_smem_limit((const void*)k_plan_wide, smem);
+    k_plan_wide<<<(unsigned)std::min(rows, num_sms() * 32), 256, smem, s>>>(
+        rows, ncols, optr, ocol, iptr, icol, outptr, outcol, kbase.p, omap, first_apart ? 1 : 0, seg.p, pe.p, pf.p); ::impes::count_launch();
+    IMPES_CHECK_LAUNCH();
+    IMPES_CUDA(cudaStreamSynchronize(s));
+  } else {
+    DBuf<int> cur(std::max(nout, 1));
+    // four lanes a row while an outer entry meets fewer than eight inner ones
+    if (nprod / std::max(onnz, 1) < 8)
+      k_plan_group<4><<<grid_for((size_t)rows * 4, 256), 256, 0, s>>>(rows, optr, ocol, iptr, icol, outptr, outcol,
+                                                                     kbase.p, omap, first_apart ? 1 : 0, seg.p, cur.p, pe.p, pf.p);
+    else
+      k_plan_group<32><<<grid_for((size_t)rows * 32, 256), 256, 0, s>>>(rows, optr, ocol, iptr, icol, outptr, outcol,
+                                                                       kbase.p, omap, first_apart ? 1 : 0, seg.p, cur.p, pe.p, pf.p);
+    ::impes::count_launch();
+    IMPES_CHECK_LAUNCH();
+    IMPES_CUDA(cudaStreamSynchronize(s));
+  }
   nterms = nprod;
   return true;
 }
@@ -1593,7 +1748,7 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
     int ctot = exclusive_scan_i32(ccnt.p, cptr.p, nl, s);
     DBuf<int> ccol(std::max(ctot, 1));
     DBuf<double> cval(std::max(ctot, 1));
-    k_p_fill<<<grid_for(nl, TB), TB, 0, s>>>(nl, L.rowptr.p, L.col.p, L.val.p, strong.p, cf2.p,
+    k_p_fill<<<grid_for((size_t)nl * 32, 256), 256, 0, s>>>(nl, L.rowptr.p, L.col.p, L.val.p, strong.p, cf2.p,
                                              f2c.p, pdiag.p, ssum.p, wcsum.p, wfsum.p, scnt.p,
                                              cptr.p, ccol.p, cval.p); ::impes::count_launch();
     DBuf<int> mcnt(nl + 1);
@@ -1675,10 +1830,10 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
     IMPES_CUDA(cudaStreamSynchronize(s));
     Nc.nnz = h.hint.p[0];
     Nc.val.alloc(std::max(Nc.nnz, 1));
-    L.planned = build_plan(nl, L.rowptr.p, L.col.p, L.prow.p, L.pcol.p, L.aprow.p, L.apcol.p, apnnz,
-                           nullptr, L.ap_seg, L.ap_e, L.ap_f, L.ap_terms, s) &&
-                build_plan(nc, L.rrow.p, L.rcol.p, L.aprow.p, L.apcol.p, Nc.rowptr.p, Nc.col.p, Nc.nnz,
-                           L.rsrc.p, L.ac_seg, L.ac_r, L.ac_f, L.ac_terms, s);
+    L.planned = build_plan(nl, nc, L.rowptr.p, L.col.p, L.prow.p, L.pcol.p, L.aprow.p, L.apcol.p, apnnz, L.nnz,
+                           nullptr, nzero > 0, L.ap_seg, L.ap_e, L.ap_f, L.ap_terms, s) &&
+                build_plan(nc, nc, L.rrow.p, L.rcol.p, L.aprow.p, L.apcol.p, Nc.rowptr.p, Nc.col.p, Nc.nnz, L.pnnz,
+                           L.rsrc.p, false, L.ac_seg, L.ac_r, L.ac_f, L.ac_terms, s);
     if (!L.planned) {
       L.ap_seg.release(); L.ap_e.release(); L.ap_f.release();
       L.ac_seg.release(); L.ac_r.release(); L.ac_f.release();

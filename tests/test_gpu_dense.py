@@ -112,3 +112,32 @@ def test_coarse_operator_vcycle(dims, kw):
         assert np.linalg.norm(x32 - ref) <= 2e-2 * np.linalg.norm(ref)
         x, st = amg.fgmres(bt, tol=1e-10, precision="mixed", max_iters=400)
         assert st["converged"]
+
+
+# rows of a few products, long rows (a block each), and a hierarchy whose P rows repeat a column (a row whose weights all
+# vanished takes its first coarse neighbour a second time)
+@pytest.mark.parametrize("dims", [(20, 20, 1), (15, 13, 11), (26, 24, 14)])
+def test_galerkin_plan(dims):
+    import scipy.sparse as sp
+    from impes_b200.amg import ClassicalAMG
+
+    def d1(m, a):
+        return sp.diags([-a * np.ones(m - 1), 2 * a * np.ones(m), -a * np.ones(m - 1)], [-1, 0, 1])
+
+    ix, iy, iz = (sp.identity(d) for d in dims)
+    A = (sp.kron(sp.kron(d1(dims[0], 1.0), iy), iz) + sp.kron(sp.kron(ix, d1(dims[1], 1.0)), iz)
+         + sp.kron(sp.kron(ix, iy), d1(dims[2], 0.1)) + 1e-3 * sp.identity(int(np.prod(dims)))).tocsr()
+    amg = ClassicalAMG(A, coarsest_size=30, mixed_precision=True)
+    A2 = A.copy()
+    A2.data = A2.data * np.where(A2.data > 0, 1.0, np.linspace(0.8, 1.0, A2.nnz))
+    amg.update_matrix(A2)
+    levels = amg.levels
+    for a, b in zip(levels[:-1], levels[1:]):
+        L, P, C = (t.to_dense().cpu().numpy() for t in (a["A"], a["P"], b["A"]))
+        ref = P.T @ L @ P
+        # sums of at most a few thousand products in another order
+        assert np.abs(C - ref).max() <= 1e-12 * np.abs(ref).max()
+    if dims[2] == 14:
+        rows = [a["P"].crow_indices().cpu().numpy() for a in levels[:-1]]
+        cols = [a["P"].col_indices().cpu().numpy() for a in levels[:-1]]
+        assert any(len(set(c[p[i]:p[i + 1]])) < p[i + 1] - p[i] for p, c in zip(rows, cols) for i in range(len(p) - 1))
