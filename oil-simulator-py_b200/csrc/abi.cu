@@ -26,7 +26,7 @@ impes::AMG* impes_amg_handle_core(impes_amg* h) { return &h->a; }
 namespace impes {
 void pcg_solve(int n, const int* rowptr, const int* col, const double* val, const double* b,
                double* x, double tol, int max_iter, int& iters, bool& converged, double& rs_out,
-               cudaStream_t s);
+               DBuf<double>& work, cudaStream_t s);
 void adjoint_check_model(const Model& m);
 int adjoint_num_producers(const Model& m);
 void adjoint_rates(Model& m, AMG& a, double* p, double* sw, int steps, double dt,
@@ -435,6 +435,7 @@ int impes_model_create(impes_model** out, const impes_model_desc* d, const impes
     auto* h = new impes_model();
     Model& m = h->m;
     try {
+      Arena::Scope scope(m.arena);
       ModelParams& P = m.P;
       P.nx = d->nx; P.ny = d->ny; P.nz = d->nz; P.N = (int)N;
       P.dx = d->dx; P.dy = d->dy; P.dz = d->dz;
@@ -648,11 +649,11 @@ int impes_step(impes_model* h, impes_amg* amg, double* p, double* sw, double* sg
         bool conv = false;
         double rz = 0.0;
         pcg_solve(m.P.N, m.rowptr.p, m.col.p, m.csr_val.p, m.rhs.p, p, kp->tol, kp->max_iters, it,
-                  conv, rz, s);
+                  conv, rz, m.pcg_work, s);
         st.iterations = it;
         if (!conv) {
           pcg_solve(m.P.N, m.rowptr.p, m.col.p, m.csr_val.p, m.rhs.p, p, kp->tol * 10.0,
-                    kp->max_iters * 4, it, conv, rz, s);
+                    kp->max_iters * 4, it, conv, rz, m.pcg_work, s);
           st.iterations += it;
           st.restarts = 1;
         }
@@ -846,7 +847,8 @@ int impes_pcg_solve(int n, const int* rowptr, const int* col, const double* val,
     int it = 0;
     bool conv = false;
     double r = 0.0;
-    pcg_solve(n, rowptr, col, val, b, x, tol, max_iter, it, conv, r, S(stream));
+    DBuf<double> work;
+    pcg_solve(n, rowptr, col, val, b, x, tol, max_iter, it, conv, r, work, S(stream));
     if (iterations) *iterations = it;
     if (converged) *converged = conv ? 1 : 0;
     if (rz) *rz = r;

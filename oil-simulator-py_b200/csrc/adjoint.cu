@@ -32,6 +32,7 @@
 #include "model.cuh"
 #include <algorithm>
 #include <cmath>
+#include <optional>
 #include <vector>
 
 namespace impes {
@@ -509,6 +510,8 @@ void adjoint_gradient(Model& m, AMG& a, const double* p0, const double* sw0, con
   IMPES_REQUIRE(np >= 1, IMPES_ERR_ARG, "adjoint: the model has no producer");
   out = impes_adjoint_stats{};
   out.checkpoints = nseg;
+  Arena arena;                                   // this call's buffers, freed after them
+  std::optional<Arena::Scope> scope(std::in_place, arena);
   DBuf<int> prod(np);
   IMPES_CUDA(cudaMemcpyAsync(prod.p, pc.data(), sizeof(int) * np, cudaMemcpyHostToDevice, s));
   DBuf<double> rates((size_t)steps * np), tgt((size_t)steps * np), scratch_rates(np);
@@ -524,6 +527,7 @@ void adjoint_gradient(Model& m, AMG& a, const double* p0, const double* sw0, con
   DBuf<double> gp(N), gs(N), gp2(N), gs2(N), gam(N), mu(N), gpv(N), gtx(Fx), gty(Fy), gtz(Fz),
       dmu(np);
   DBuf<double> bal(12);
+  scope.reset();
   IMPES_CUDA(cudaMemcpyAsync(bal.p, m.balances.p, sizeof(double) * 12, cudaMemcpyDeviceToDevice, s));
   const size_t bN = sizeof(double) * N;
   auto d2d = [&](double* dst, const double* src) {

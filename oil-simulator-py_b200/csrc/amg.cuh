@@ -104,6 +104,7 @@ struct FgState {
 };
 
 struct AMG {
+  Arena arena;                     // memory of the levels (destroyed after them)
   impes_amg_params prm;
   std::vector<std::unique_ptr<Level>> levels;
   bool built = false;
@@ -122,6 +123,7 @@ struct AMG {
   // FGMRES workspace
   int krylov_m = 0;
   DBuf<double> V, Z, H, cs, sn, g, y, kw, kb, kx;
+  DBuf<double> solve_work;         // right-hand side and residuals of the stand-alone V-cycle solves
   bool krylov_mode = false;        // V-cycles issued by FGMRES
   // CUDA graphs of a whole stand-alone V-cycle from level 0, per [fp32][zero start][timed]
   struct VGraph {

@@ -2031,7 +2031,10 @@ void amg_autotune(AMG& h, cudaStream_t s) {
       IMPES_CUDA(cudaMemsetAsync(L->rf.p, 0, n * sizeof(float), s));
     }
     tune_cache_load();
-    DBuf<char> flush(kFlushBytes);
+    // (a level's sweep reads at most its values, columns and vectors)
+    double most = 0.0;
+    for (auto& L : h.levels) most = std::max(most, 12.0 * L->nnz + 40.0 * L->n);
+    DBuf<char> flush(most > kColdBytes ? kFlushBytes : 0);
     g_flush = flush.p;
     tune_levels<double>(h, s, e0, e1);
     if (h.prm.mixed_precision) tune_levels<float>(h, s, e0, e1);
@@ -2073,13 +2076,14 @@ void amg_solve_vcycles(AMG& h, const double* b, double* x, double tol, int max_c
   amg_ensure_fp64(h, s);
   Level& L0 = *h.levels[0];
   const int n = L0.n;
-  DBuf<double> bs(n), r(n), wb(n);
-  launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.dhalf_inv.p, b, bs.p);
+  h.solve_work.ensure(3 * (size_t)n);
+  double *bs = h.solve_work.p, *r = bs + n, *wb = r + n;
+  launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.dhalf_inv.p, b, bs);
   IMPES_CHECK_LAUNCH();
   const bool jac = norm == IMPES_NORM_JACOBI;
-  if (jac) { launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.jac_w.p, bs.p, wb.p); }
-  const double bn = std::sqrt(jac ? dot_host(h, wb.p, wb.p, n, s) : dot_host(h, bs.p, bs.p, n, s));
-  IMPES_CUDA(cudaMemcpyAsync(L0.b.p, bs.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+  if (jac) { launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.jac_w.p, bs, wb); }
+  const double bn = std::sqrt(jac ? dot_host(h, wb, wb, n, s) : dot_host(h, bs, bs, n, s));
+  IMPES_CUDA(cudaMemcpyAsync(L0.b.p, bs, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
   double rr = INFINITY;
   int c = 0;
   double* xs = nullptr;
@@ -2088,10 +2092,10 @@ void amg_solve_vcycles(AMG& h, const double* b, double* x, double tol, int max_c
     if (xs != L0.x.p)
       IMPES_CUDA(cudaMemcpyAsync(L0.x.p, xs, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     xs = L0.x.p;
-    launch_csr<double, Y_B_MINUS_AX>(n, L0.avg_row, L0.rowptr.p, L0.col.p, L0.val.p, xs, bs.p,
-                                     nullptr, r.p, s);
-    if (jac) { launch_pdl(k_mul_inplace, grid_for(n, TB), TB, 0, s, n, r.p, h.jac_w.p); }
-    rr = std::sqrt(dot_host(h, r.p, r.p, n, s)) / (bn + 1e-30);
+    launch_csr<double, Y_B_MINUS_AX>(n, L0.avg_row, L0.rowptr.p, L0.col.p, L0.val.p, xs, bs,
+                                     nullptr, r, s);
+    if (jac) { launch_pdl(k_mul_inplace, grid_for(n, TB), TB, 0, s, n, r, h.jac_w.p); }
+    rr = std::sqrt(dot_host(h, r, r, n, s)) / (bn + 1e-30);
     if (!(rr == rr)) throw Error(IMPES_ERR_NAN, "NaN residual in V-cycle solve");
     if (rr < tol) break;
   }
@@ -2108,19 +2112,20 @@ void amg_apply(AMG& h, const double* b, double* x, int cycles, double apply_tol,
   amg_ensure_fp64(h, s);
   Level& L0 = *h.levels[0];
   const int n = L0.n;
-  DBuf<double> bs(n), r(n);
-  launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.dhalf_inv.p, b, bs.p);
-  IMPES_CUDA(cudaMemcpyAsync(L0.b.p, bs.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  const double bn = std::sqrt(dot_host(h, bs.p, bs.p, n, s));
+  h.solve_work.ensure(3 * (size_t)n);
+  double *bs = h.solve_work.p, *r = bs + n;
+  launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.dhalf_inv.p, b, bs);
+  IMPES_CUDA(cudaMemcpyAsync(L0.b.p, bs, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+  const double bn = std::sqrt(dot_host(h, bs, bs, n, s));
   int c = 0;
   while (c < apply_max_cycles) {
     double* xs = vcycle_top<double>(h, c == 0, s);
     if (xs != L0.x.p)
       IMPES_CUDA(cudaMemcpyAsync(L0.x.p, xs, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     ++c;
-    launch_csr<double, Y_B_MINUS_AX>(n, L0.avg_row, L0.rowptr.p, L0.col.p, L0.val.p, L0.x.p, bs.p,
-                                     nullptr, r.p, s);
-    double rel = std::sqrt(dot_host(h, r.p, r.p, n, s)) / (bn + 1e-30);
+    launch_csr<double, Y_B_MINUS_AX>(n, L0.avg_row, L0.rowptr.p, L0.col.p, L0.val.p, L0.x.p, bs,
+                                     nullptr, r, s);
+    double rel = std::sqrt(dot_host(h, r, r, n, s)) / (bn + 1e-30);
     if (c >= cycles && rel < apply_tol) break;
   }
   launch_pdl(k_mul, grid_for(n, TB), TB, 0, s, n, h.dhalf_inv.p, L0.x.p, x);

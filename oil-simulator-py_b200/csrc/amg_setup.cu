@@ -1667,6 +1667,9 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
                cudaStream_t s) {
   IMPES_REQUIRE(n > 0 && nnz > 0, IMPES_ERR_ARG, "empty matrix");
   h.drop_graphs();
+  // the old levels' memory is used again at once: nothing may still read it
+  if (!h.levels.empty()) IMPES_CUDA(cudaDeviceSynchronize());
+  Arena::Scope scope(h.arena);
   {
     const char* ev = getenv("IMPES_NO_GRAPHS");
     h.use_graphs = !(ev && ev[0] == '1');
@@ -1957,6 +1960,8 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
   }
   h.tail_level = amg_tail_level(h);
   amg_dense_setup(h);
+  IMPES_CUDA(cudaStreamSynchronize(s));
+  h.arena.trim();
   h.built = true;
 }
 

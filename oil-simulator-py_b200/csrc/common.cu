@@ -1,7 +1,9 @@
 // Shared host utilities: thread-local error text and a device exclusive scan.
 #include "common.cuh"
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
+#include <iterator>
 #include <map>
 #include <mutex>
 
@@ -34,6 +36,76 @@ void raise_smem_limit(const void* kernel, size_t bytes) {
     c = bytes;
   }
 }
+namespace {
+thread_local Arena* t_arena = nullptr;
+}
+Arena* Arena::current() { return t_arena; }
+Arena::Scope::Scope(Arena& a) : before(t_arena) { t_arena = &a; }
+Arena::Scope::~Scope() { t_arena = before; }
+
+Arena::~Arena() {
+  for (Chunk& c : chunks_) cudaFree(c.base);
+}
+
+void* Arena::take(size_t bytes) {
+  const size_t need = (bytes + kAlign - 1) / kAlign * kAlign;
+  Chunk* best = nullptr;
+  std::map<size_t, size_t>::iterator at;
+  for (Chunk& c : chunks_)             // the smallest free piece that holds it
+    for (auto it = c.free.begin(); it != c.free.end(); ++it)
+      if (it->second >= need && (!best || it->second < at->second)) {
+        best = &c;
+        at = it;
+      }
+  if (!best) {
+    const size_t size = std::max(need, next_);
+    void* base = nullptr;
+    if (cudaMalloc(&base, size) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    next_ = std::min<size_t>(next_ * 2, 64u << 20);
+    chunks_.push_back(Chunk{static_cast<char*>(base), size, {}});
+    best = &chunks_.back();
+    at = best->free.emplace(0, size).first;
+  }
+  const size_t off = at->first, len = at->second;
+  best->free.erase(at);
+  if (len > need) best->free.emplace(off + need, len - need);
+  return best->base + off;
+}
+
+void Arena::give(void* p, size_t bytes) {
+  const size_t len = (bytes + kAlign - 1) / kAlign * kAlign;
+  for (Chunk& c : chunks_) {
+    if (p < c.base || p >= c.base + c.size) continue;
+    auto it = c.free.emplace(static_cast<size_t>(static_cast<char*>(p) - c.base), len).first;
+    auto next = std::next(it);
+    if (next != c.free.end() && it->first + it->second == next->first) {
+      it->second += next->second;
+      c.free.erase(next);
+    }
+    if (it != c.free.begin()) {
+      auto prev = std::prev(it);
+      if (prev->first + prev->second == it->first) {
+        prev->second += it->second;
+        c.free.erase(it);
+      }
+    }
+    return;
+  }
+}
+
+void Arena::trim() {
+  for (size_t q = chunks_.size(); q-- > 0;) {
+    Chunk& c = chunks_[q];
+    if (c.free.size() == 1 && c.free.begin()->second == c.size) {
+      cudaFree(c.base);
+      chunks_.erase(chunks_.begin() + q);
+    }
+  }
+}
+
 const char* last_error_cstr() { return g_last_error.c_str(); }
 
 bool pdl_enabled() {

@@ -37,6 +37,7 @@ struct WellDev {
 };
 
 struct Model {
+  Arena arena;                         // its memory (destroyed after the buffers)
   ModelParams P;
   int nnz = 0;
   std::vector<WellDev> wells_host;
@@ -65,6 +66,7 @@ struct Model {
   double dt_prev2 = 0.0;
   bool have_prev2 = false;
   DBuf<int> rowptr, col;               // static pattern
+  DBuf<double> pcg_work;               // vectors of the Jacobi-PCG solver
   int red_blocks = 0;
 };
 

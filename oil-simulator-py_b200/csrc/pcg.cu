@@ -171,15 +171,16 @@ __global__ void __launch_bounds__(2 * TBP) k_pcg(int n, const int* __restrict__ 
 }  // namespace
 
 // Solves A x = b (x written); returns the iterations taken and whether the
-// stopping test fired.  rs_out: the last r.z.
+// stopping test fired.  rs_out: the last r.z.  work: the solve's vectors, grown to
+// what this size needs.
 void pcg_solve(int n, const int* rowptr, const int* col, const double* val, const double* b,
                double* x, double tol, int max_iter, int& iters, bool& converged, double& rs_out,
-               cudaStream_t s) {
+               DBuf<double>& work, cudaStream_t s) {
   IMPES_REQUIRE(n > 0 && max_iter >= 0, IMPES_ERR_ARG, "pcg: bad size or iteration limit");
   const bool one = n <= kBlocks * TBP;
   const size_t nv = (size_t)n;
   // z, two directions, and unless they stay in registers d, r and Ap
-  DBuf<double> work(nv * (one ? 3 : 6) + 2 * kBlocks + (sizeof(PcgOut) + 7) / 8);
+  work.ensure(nv * (one ? 3 : 6) + 2 * kBlocks + (sizeof(PcgOut) + 7) / 8);
   double* part = work.p;
   PcgOut* out = reinterpret_cast<PcgOut*>(part + 2 * kBlocks);
   double* z = part + 2 * kBlocks + (sizeof(PcgOut) + 7) / 8;
