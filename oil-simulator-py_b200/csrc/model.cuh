@@ -44,6 +44,7 @@ struct Model {
   std::vector<int> wc_cells_host;      // sorted distinct well cells
   DBuf<double> tx, ty, tz, pv;         // transmissibilities, pore volume
   DBuf<double> pvt;                    // rows x 9, row-major
+  DBuf<double> pvt_tab;                // by column, with the slopes (as the kernels stage it)
   DBuf<WellDev> wells;
   DBuf<int> wc_cells, wc_ptr, wc_wells;// well-cell -> wells (original order)
   // per-step scratch

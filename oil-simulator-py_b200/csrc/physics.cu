@@ -36,6 +36,8 @@ __device__ __forceinline__ double tpow(double x, double e) {
   if (e == -0.5) return 1.0 / sqrt(x);
   if (e == -1.0) return 1.0 / x;
   if (e == -2.0) return 1.0 / (x * x);
+  if (x == 1.0) return 1.0;            // the end points of a saturation range, as pow gives them
+  if (x == 0.0 && e > 0.0) return 0.0;
   return pow(x, e);
 }
 // torch.clamp semantics (NaN passes through; lo > hi yields hi).
@@ -58,46 +60,67 @@ struct PvtSmem {
   const double* slope;  // 8 * (rows - 1)
 };
 
-__device__ void pvt_stage(const double* __restrict__ g, int rows, double* s_col, double* s_slope) {
-  for (int t = threadIdx.x; t < rows * kPvtCols; t += blockDim.x) {
-    int r = t / kPvtCols, c = t % kPvtCols;
-    s_col[c * rows + r] = g[t];
-  }
-  __syncthreads();
+// The table as the kernels stage it: columns [9][rows], then slopes [8][rows - 1]
+// of the columns after the pressure.
+__global__ void k_pvt_table(int rows, const double* __restrict__ g, double* __restrict__ tab) {
+  for (int t = threadIdx.x; t < rows * kPvtCols; t += blockDim.x) tab[(t % kPvtCols) * rows + t / kPvtCols] = g[t];
   for (int t = threadIdx.x; t < (kPvtCols - 1) * (rows - 1); t += blockDim.x) {
-    int c = 1 + t / (rows - 1), r = t % (rows - 1);
-    const double* xp = s_col;
-    const double* fp = s_col + c * rows;
-    s_slope[(c - 1) * (rows - 1) + r] = (fp[r + 1] - fp[r]) / (xp[r + 1] - xp[r]);
+    const int c = 1 + t / (rows - 1), r = t % (rows - 1);
+    tab[kPvtCols * rows + t] = (g[(r + 1) * kPvtCols + c] - g[r * kPvtCols + c]) /
+                               (g[(r + 1) * kPvtCols] - g[r * kPvtCols]);
   }
+}
+__device__ void pvt_stage(const double* __restrict__ tab, int rows, double* s_col, double* s_slope) {
+  for (int t = threadIdx.x; t < kPvtCols * rows; t += blockDim.x) s_col[t] = tab[t];
+  for (int t = threadIdx.x; t < (kPvtCols - 1) * (rows - 1); t += blockDim.x) s_slope[t] = tab[kPvtCols * rows + t];
   __syncthreads();
 }
 
-// numpy.interp(x, xp, fp) with flat extrapolation (pvt.py:48-50).
-__device__ double pvt_interp(const PvtSmem& t, int c, double x) {
+// numpy.interp(x, xp, fp) with flat extrapolation (pvt.py:48-50), in two parts:
+// where x lies in the table (searched once for all columns read there) and the
+// value of a column.
+struct PvtAt {
+  double x;
+  int lo;       // interval, or the row whose value is taken
+  int kind;     // 0: interpolate, 1: row lo, 2: x is NaN
+};
+__device__ PvtAt pvt_find(const PvtSmem& t, double x) {
   const int n = t.rows;
   const double* xp = t.col;
-  const double* fp = t.col + c * n;
-  if (isnan(x)) return x;
-  if (x < xp[0]) return fp[0];
-  if (x >= xp[n - 1]) return fp[n - 1];
+  if (isnan(x)) return {x, 0, 2};
+  if (x < xp[0]) return {x, 0, 1};
+  if (x >= xp[n - 1]) return {x, n - 1, 1};
   int lo = 0, hi = n - 1;
   while (hi - lo > 1) {
     int mid = (lo + hi) >> 1;
     if (xp[mid] <= x) lo = mid; else hi = mid;
   }
-  if (xp[lo] == x) return fp[lo];
-  double sl = t.slope[(c - 1) * (n - 1) + lo];
-  double r = sl * (x - xp[lo]) + fp[lo];
+  return {x, lo, xp[lo] == x ? 1 : 0};
+}
+// pvt_find for an x near one found before: its interval is tried first
+__device__ PvtAt pvt_find_near(const PvtSmem& t, double x, const PvtAt& near) {
+  const int lo = near.lo;
+  if (near.kind != 2 && lo < t.rows - 1 && t.col[lo] < x && x < t.col[lo + 1]) return {x, lo, 0};
+  return pvt_find(t, x);
+}
+__device__ __forceinline__ double pvt_val(const PvtSmem& t, int c, const PvtAt& a) {
+  const int n = t.rows, lo = a.lo;
+  const double* xp = t.col;
+  const double* fp = t.col + c * n;
+  if (a.kind == 2) return a.x;
+  if (a.kind == 1) return fp[lo];
+  const double sl = t.slope[(c - 1) * (n - 1) + lo];
+  double r = sl * (a.x - xp[lo]) + fp[lo];
   if (isnan(r)) {
-    r = sl * (x - xp[lo + 1]) + fp[lo + 1];
+    r = sl * (a.x - xp[lo + 1]) + fp[lo + 1];
     if (isnan(r) && fp[lo] == fp[lo + 1]) r = fp[lo];
   }
   return r;
 }
 // Fluid._eval_pvt(p, key): interpolation at p / 1e6 MPa (fluid.py:186-187).
-__device__ __forceinline__ double pvt_at(const PvtSmem& t, int c, double p_pa) {
-  return pvt_interp(t, c, p_pa / 1e6);
+__device__ __forceinline__ PvtAt pvt_at(const ModelParams& P, const PvtSmem& t, double p_pa) {
+  if (P.pvt_rows == 0) return {0.0, 0, 1};
+  return pvt_find(t, p_pa / 1e6);
 }
 
 struct KR { double kro, krw, krg; };
@@ -126,12 +149,12 @@ __device__ KR relperms(const ModelParams& P, double sw, double sg) {
 }
 
 struct Visc { double o, w, g; };
-__device__ __forceinline__ Visc viscosities(const ModelParams& P, const PvtSmem& t, double p) {
+__device__ __forceinline__ Visc viscosities(const ModelParams& P, const PvtSmem& t, const PvtAt& at) {
   Visc v;
   if (P.pvt_rows > 0) {
-    v.o = pvt_at(t, C_MUO, p) * 1e-3;
-    v.w = pvt_at(t, C_MUW, p) * 1e-3;
-    v.g = pvt_at(t, C_MUG, p) * 1e-3;
+    v.o = pvt_val(t, C_MUO, at) * 1e-3;
+    v.w = pvt_val(t, C_MUW, at) * 1e-3;
+    v.g = pvt_val(t, C_MUG, at) * 1e-3;
   } else {
     v.o = P.mu_o; v.w = P.mu_w; v.g = P.mu_g;
   }
@@ -140,11 +163,11 @@ __device__ __forceinline__ Visc viscosities(const ModelParams& P, const PvtSmem&
 
 struct Rho { double w, o, g; };
 // Fluid.rho_w / rho_o / rho_g at pressure p (fluid.py:129-158, 330-375).
-__device__ Rho densities(const ModelParams& P, const PvtSmem& t, double p) {
+__device__ __forceinline__ Rho densities(const ModelParams& P, const PvtSmem& t, double p, const PvtAt& at) {
   Rho r;
   if (P.pvt_rows > 0) {
-    double bw = pvt_at(t, C_BW, p), bo = pvt_at(t, C_BO, p), rs = pvt_at(t, C_RS, p);
-    double bg = pvt_at(t, C_BG, p), rv = pvt_at(t, C_RV, p);
+    double bw = pvt_val(t, C_BW, at), bo = pvt_val(t, C_BO, at), rs = pvt_val(t, C_RS, at);
+    double bg = pvt_val(t, C_BG, at), rv = pvt_val(t, C_RV, at);
     r.w = P.rho_w_ref / (bw + 1e-12);
     r.o = (P.rho_o_ref + rs * P.rho_g_ref) / (bo + 1e-12);
     r.g = (P.rho_g_ref + rv * P.rho_o_ref) / (bg + 1e-12);
@@ -162,12 +185,13 @@ __device__ double total_compressibility(const ModelParams& P, const PvtSmem& t, 
   if (P.pvt_rows == 0) return P.cf;
   const double P_mpa = p / 1e6;
   const double Pp = P_mpa + 0.1, Pm = P_mpa - 0.1;
-  const double x0 = P_mpa * 1e6, xp = Pp * 1e6, xm = Pm * 1e6;
+  const PvtAt a0 = pvt_find(t, P_mpa * 1e6 / 1e6);
+  const PvtAt ap = pvt_find_near(t, Pp * 1e6 / 1e6, a0), am = pvt_find_near(t, Pm * 1e6 / 1e6, a0);
   double c[3];
   const int cols[3] = {C_BW, C_BO, C_BG};
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
-    double B = pvt_at(t, cols[q], x0), Bp = pvt_at(t, cols[q], xp), Bm = pvt_at(t, cols[q], xm);
+    double B = pvt_val(t, cols[q], a0), Bp = pvt_val(t, cols[q], ap), Bm = pvt_val(t, cols[q], am);
     double dB = (Bp - Bm) / (2 * 0.1);
     c[q] = -(dB / (B + 1e-12)) / 1e6;
   }
@@ -340,13 +364,14 @@ __global__ void __launch_bounds__(256, 4) k_assemble(
     long long c = ((long long)i * P.ny + j) * P.nz + k;
     double pc_ = p[c], swc = sw[c], sgc = sg[c];
     KR kr = relperms(P, swc, sgc);
-    Visc mu = viscosities(P, T, pc_);
+    const PvtAt at = pvt_at(P, T, pc_);
+    Visc mu = viscosities(P, T, at);
     s_p[t] = pc_;
     s_mw[t] = kr.krw / mu.w;
     s_mo[t] = kr.kro / mu.o;
     s_mg[t] = kr.krg / mu.g;
     if (grav) {
-      Rho r = densities(P, T, pc_);
+      Rho r = densities(P, T, pc_, at);
       s_rw[t] = r.w; s_ro[t] = r.o; s_rg[t] = r.g;
     }
     s_pc[t] = capillary(P, swc);
@@ -476,7 +501,7 @@ __global__ void __launch_bounds__(256, 4) k_assemble(
 __device__ void well_cell_phase(const ModelParams& P, const PvtSmem& T, double p, double sw,
                                 double sg, double& mt, double& fw, double& fg, double& fo) {
   KR kr = relperms(P, sw, sg);
-  Visc mu = viscosities(P, T, p);
+  Visc mu = viscosities(P, T, pvt_at(P, T, p));
   double mw = kr.krw / mu.w, mo = kr.kro / mu.o, mg = kr.krg / mu.g;
   mt = mw + mo + mg;
   fw = mw / (mt + 1e-10);
@@ -519,8 +544,9 @@ __global__ void k_well_sources(ModelParams P, const double* __restrict__ pvt_g,
       well_cell_phase(P, T, p, sw_c, sg_c, mt, fw_, fg_, fo_);
       double Bo = 0, Bw = 0, Bg = 0, Rs = 0, Rv = 0;
       if (pvt) {
-        Bo = pvt_at(T, C_BO, p); Bw = pvt_at(T, C_BW, p); Bg = pvt_at(T, C_BG, p);
-        Rs = pvt_at(T, C_RS, p); Rv = pvt_at(T, C_RV, p);
+        const PvtAt at = pvt_at(P, T, p);
+        Bo = pvt_val(T, C_BO, at); Bw = pvt_val(T, C_BW, at); Bg = pvt_val(T, C_BG, at);
+        Rs = pvt_val(T, C_RS, at); Rv = pvt_val(T, C_RV, at);
       }
       if (W.control_bhp == 0) {
         const double q_base = (W.value * P.rate_scale) / 86400.0;
@@ -647,22 +673,29 @@ __global__ void k_well_sources(ModelParams P, const double* __restrict__ pvt_g,
     for (int k = 0; k < 4; ++k) s_b[w][k] = db[k];
   }
   __syncthreads();
-  // phase 2: the sums in the reference's well order (one thread)
-  if (threadIdx.x != 0) return;
-  for (int t = 0; t < 3 * P.nwc; ++t) wq[t] = 0.0;
-  for (int w = 0; w < P.nwells; ++w) {
-    const int slot = s_slot[w], mask = s_mask[w];
-    if (slot < 0) continue;
-    if (mask & 1) wq[slot] += s_q[w][0];
-    if (mask & 2) wq[P.nwc + slot] += s_q[w][1];
-    if (mask & 4) wq[2 * P.nwc + slot] += s_q[w][2];
-    // balance additions in the order the serial loop made them: gas in then
-    // oil in (gas injectors), oil out then gas out (producers)
-    if (mask & 32) bal[6 + 3] += s_b[w][2];
-    if (mask & 8) bal[6 + 0] += s_b[w][0];
-    if (mask & 16) bal[6 + 1] += s_b[w][1];
-    if (mask & 64) bal[6 + 4] += s_b[w][3];
+  // phase 2: the sums in the reference's well order (one thread), kept on chip
+  __shared__ double s_wq[3 * kMaxWells];
+  for (int t = threadIdx.x; t < 3 * P.nwc; t += blockDim.x) s_wq[t] = 0.0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double b0 = bal[6 + 0], b1 = bal[6 + 1], b3 = bal[6 + 3], b4 = bal[6 + 4];
+    for (int w = 0; w < P.nwells; ++w) {
+      const int slot = s_slot[w], mask = s_mask[w];
+      if (slot < 0) continue;
+      if (mask & 1) s_wq[slot] += s_q[w][0];
+      if (mask & 2) s_wq[P.nwc + slot] += s_q[w][1];
+      if (mask & 4) s_wq[2 * P.nwc + slot] += s_q[w][2];
+      // balance additions in the order the serial loop made them: gas in then
+      // oil in (gas injectors), oil out then gas out (producers)
+      if (mask & 32) b3 += s_b[w][2];
+      if (mask & 8) b0 += s_b[w][0];
+      if (mask & 16) b1 += s_b[w][1];
+      if (mask & 64) b4 += s_b[w][3];
+    }
+    bal[6 + 0] = b0; bal[6 + 1] = b1; bal[6 + 3] = b3; bal[6 + 4] = b4;
   }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 3 * P.nwc; t += blockDim.x) wq[t] = s_wq[t];
 }
 
 // K4a: fluxes, divergence, dS and the substep ratio (simulation.py:968-1042, 1351-1379).
@@ -706,12 +739,13 @@ __global__ void __launch_bounds__(256, 4) k_saturation_flux(
     long long c = ((long long)i * P.ny + j) * P.nz + k;
     double pc_ = p[c], swc = sw[c], sgc = sg[c];
     KR kr = relperms(P, swc, sgc);
-    Visc mu = viscosities(P, T, pc_);
+    const PvtAt at = pvt_at(P, T, pc_);
+    Visc mu = viscosities(P, T, at);
     s_p[t] = pc_;
     s_mw[t] = kr.krw / mu.w;
     s_mg[t] = kr.krg / mu.g;
     if (grav) {
-      Rho r = densities(P, T, pc_);
+      Rho r = densities(P, T, pc_, at);
       s_rw[t] = r.w; s_rg[t] = r.g;
     }
     s_pcg[t] = capillary_og(P, sgc);
@@ -822,15 +856,22 @@ __global__ void __launch_bounds__(256, 4) k_saturation_flux(
   }
 }
 
-// Per-substep component balance of PVT runs (simulation.py:1396-1505): one
-// thread replays the substeps at the well cells.
+// Per-substep component balance of PVT runs (simulation.py:1396-1505): a thread
+// per (substep, well) replays the substeps at the well's cell, then four threads
+// add the terms in the reference's order.
+constexpr int kContribSmem = 3584;     // doubles of the terms kept in shared memory
+__host__ __device__ inline bool contrib_on_chip(const ModelParams& P) {
+  return 4ll * P.max_substeps * P.nwells <= kContribSmem;
+}
 __global__ void k_well_substeps(ModelParams P, const double* __restrict__ pvt_g,
                                 const WellDev* __restrict__ wells, const double* __restrict__ p_new,
                                 const double* __restrict__ sw, const double* __restrict__ sg,
                                 const double* __restrict__ dsw, const double* __restrict__ dsg,
-                                const int* __restrict__ nsub, double dt, double* __restrict__ contrib,
-                                double* bal, const int* pred) {
+                                const int* __restrict__ nsub, double dt, double* contrib, double* bal,
+                                const int* pred) {
   if (pred && *pred == 0) return;
+  extern __shared__ double s_contrib[];    // contrib on chip when it fits (kContribSmem)
+  if (contrib_on_chip(P)) contrib = s_contrib;
   // contrib[(s * nwells + w) * 4 + q]: the addend of bal[6 + {0, 1, 3, 4}[q]] for
   // substep s and well w (never negative), -1 where the reference adds nothing
   __shared__ double s_col[kPvtCols * kMaxPvtRows];
@@ -856,9 +897,10 @@ __global__ void k_well_substeps(ModelParams P, const double* __restrict__ pvt_g,
         sgc = tclamp(sgc, P.sg_cr, 1.0 - so_r - swc);
       }
       const double p = p_new[c];
-      const double Bo = pvt_at(T, C_BO, p), Bw = pvt_at(T, C_BW, p), Bg = pvt_at(T, C_BG, p);
-      const double Rs = pvt_at(T, C_RS, p), Rv = pvt_at(T, C_RV, p);
-      const double mu_w = pvt_at(T, C_MUW, p), mu_o = pvt_at(T, C_MUO, p), mu_g = pvt_at(T, C_MUG, p);
+      const PvtAt at = pvt_at(P, T, p);
+      const double Bo = pvt_val(T, C_BO, at), Bw = pvt_val(T, C_BW, at), Bg = pvt_val(T, C_BG, at);
+      const double Rs = pvt_val(T, C_RS, at), Rv = pvt_val(T, C_RV, at);
+      const double mu_w = pvt_val(T, C_MUW, at), mu_o = pvt_val(T, C_MUO, at), mu_g = pvt_val(T, C_MUG, at);
       KR kr = relperms(P, swc, sgc);
       double mw = kr.krw / (mu_w + 1e-12), mo = kr.kro / (mu_o + 1e-12), mg = kr.krg / (mu_g + 1e-12);
       double mt = mw + mo + mg;
@@ -915,9 +957,13 @@ __global__ void k_well_substeps(ModelParams P, const double* __restrict__ pvt_g,
     const int q = threadIdx.x;
     const int slot = q == 0 ? 0 : q == 1 ? 1 : q == 2 ? 3 : 4;
     double acc = bal[6 + slot];
-    for (int it = 0; it < items; ++it) {
-      const double v = contrib[(size_t)it * 4 + q];
-      if (!(v < 0.0)) acc += v;   // NaN propagates as before
+    for (int i0 = 0; i0 < items; i0 += 8) {      // eight loads ahead of their additions
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = i0 + u < items ? contrib[(size_t)(i0 + u) * 4 + q] : -1.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (!(v[u] < 0.0)) acc += v[u];   // NaN propagates as before
     }
     bal[6 + slot] = acc;
   }
@@ -947,19 +993,23 @@ __global__ void __launch_bounds__(kSatBlock) k_saturation_substeps(
     const double dws = dsw[c] / N, dgs = dsg[c] / N;
     double swc = sw0, sgc = sg0;
     for (int s = 0; s < N; ++s) {
+      const double w_ = swc, g_ = sgc;
       swc = swc + dws;
       sgc = sgc + dgs;
       swc = tclamp(swc, P.sw_cr, 1.0 - so_r - sgc);
       sgc = tclamp(sgc, P.sg_cr, 1.0 - so_r - swc);
+      if (swc == w_ && sgc == g_) break;   // a substep that changes nothing: nor do the others
     }
     sw[c] = swc;
     sg[c] = sgc;
     so[c] = 1.0 - swc - sgc;
     const double dwe = swc - sw0, dge = sgc - sg0;
-    Rho r = densities(P, T, p_new[c]);
-    const double mw = dwe * pv[c] * r.w;
-    const double mg = dge * pv[c] * r.g;
-    const double mo = (-(dwe + dge)) * pv[c] * r.o;
+    const double p = p_new[c], pvc = pv[c];
+    if (dwe == 0.0 && dge == 0.0 && isfinite(p) && isfinite(pvc)) continue;   // no mass moves
+    Rho r = densities(P, T, p, pvt_at(P, T, p));
+    const double mw = dwe * pvc * r.w;
+    const double mg = dge * pvc * r.g;
+    const double mo = (-(dwe + dge)) * pvc * r.o;
     acc[0] += tclamp_min(mw, 0.0); acc[1] += -tclamp_max(mw, 0.0);
     acc[2] += tclamp_min(mo, 0.0); acc[3] += -tclamp_max(mo, 0.0);
     acc[4] += tclamp_min(mg, 0.0); acc[5] += -tclamp_max(mg, 0.0);
@@ -1001,6 +1051,12 @@ size_t brick_smem(const Brick& b, int fields, int pvt_rows) {
 
 }  // namespace
 
+// blocks of the substep kernel: up to eight an SM, each with several cells a
+// thread, so that staging the PVT table and the block sums are paid once for them
+inline unsigned sat_grid(long long n) {
+  return (unsigned)std::max<long long>(1, std::min<long long>((n + kSatBlock - 1) / kSatBlock, (long long)num_sms() * 8));
+}
+
 // ---------------------------------------------------------------- host API
 void model_build_static(Model& m, const double* kx, const double* ky, const double* kz,
                         const double* poro, cudaStream_t s) {
@@ -1019,13 +1075,18 @@ void model_build_static(Model& m, const double* kx, const double* ky, const doub
   IMPES_CHECK_LAUNCH();
   Brick b = make_brick(P);
   int blocks = b.nbi * b.nbj * b.nbk;
-  m.red_blocks = std::max(blocks, (int)grid_for(P.N, kSatBlock));
+  m.red_blocks = std::max(blocks, (int)sat_grid(P.N));
   m.red.alloc((size_t)6 * m.red_blocks + 16);
   m.counter.alloc(2);
   IMPES_CUDA(cudaMemsetAsync(m.counter.p, 0, 2 * sizeof(unsigned), s));
   m.nsub.alloc(1);
   m.dsw.alloc(P.N);
   m.dsg.alloc(P.N);
+  if (P.pvt_rows > 0) {
+    m.pvt_tab.alloc((size_t)(2 * kPvtCols - 1) * P.pvt_rows);
+    k_pvt_table<<<1, 256, 0, s>>>(P.pvt_rows, m.pvt.p, m.pvt_tab.p); ::impes::count_launch();
+    IMPES_CHECK_LAUNCH();
+  }
   m.wq.alloc(std::max(1, 3 * P.nwc));
   m.wsub.alloc(std::max<size_t>(1, (size_t)4 * std::max(P.max_substeps, 1) * std::max(P.nwells, 1)));
 }
@@ -1043,7 +1104,7 @@ void model_assemble(Model& m, const double* p, const double* sw, const double* s
   const double F = 0.5 * (double)(m.nnz - m.P.N);
   const int tid = timers().begin(IMPES_PH_ASSEMBLE, s);
   k_assemble<<<blocks, 256, brick_smem(b, kK1Fields, m.P.pvt_rows), s>>>(
-      m.P, b, m.pvt.p, p, sw, sg, m.tx.p, m.ty.p, m.tz.p, m.pv.p, m.wells.p, m.wc_cells.p,
+      m.P, b, m.pvt_tab.p, p, sw, sg, m.tx.p, m.ty.p, m.tz.p, m.pv.p, m.wells.p, m.wc_cells.p,
       m.wc_ptr.p, m.wc_wells.p, m.well_mode.p, dt, csr_val, rhs); ::impes::count_launch();
   IMPES_CHECK_LAUNCH();
   timers().end(tid, s, 8.0 * (6.0 * m.P.N + 3.0 * F));   // reads p, Sw, Sg, PV, T; writes A, b
@@ -1054,7 +1115,7 @@ void model_saturation(Model& m, const double* p_new, double* sw, double* sg, dou
   const ModelParams& P = m.P;
   const int tid = timers().begin(IMPES_PH_SATURATION, s);
   if (P.nwells > 0) {
-    k_well_sources<<<1, kMaxWells, 0, s>>>(P, m.pvt.p, m.wells.p, m.wc_cells.p, p_new, sw, sg, m.pv.p,
+    k_well_sources<<<1, kMaxWells, 0, s>>>(P, m.pvt_tab.p, m.wells.p, m.wc_cells.p, p_new, sw, sg, m.pv.p,
                                      dt, m.wq.p, m.balances.p, m.well_q.p, m.well_rates.p, pred); ::impes::count_launch();
     IMPES_CHECK_LAUNCH();
   }
@@ -1062,16 +1123,17 @@ void model_saturation(Model& m, const double* p_new, double* sw, double* sg, dou
   int blocks = b.nbi * b.nbj * b.nbk;
   ensure_smem(k_saturation_flux, brick_smem(b, kK4Fields, P.pvt_rows), g_smem_k4);
   k_saturation_flux<<<blocks, 256, brick_smem(b, kK4Fields, P.pvt_rows), s>>>(
-      P, b, m.pvt.p, p_new, sw, sg, m.tx.p, m.ty.p, m.tz.p, m.pv.p, m.wc_cells.p, m.wq.p, dt,
+      P, b, m.pvt_tab.p, p_new, sw, sg, m.tx.p, m.ty.p, m.tz.p, m.pv.p, m.wc_cells.p, m.wq.p, dt,
       m.dsw.p, m.dsg.p, m.red.p, m.counter.p, m.nsub.p, pred); ::impes::count_launch();
   IMPES_CHECK_LAUNCH();
   if (P.pvt_rows > 0 && P.nwells > 0) {
-    k_well_substeps<<<1, 256, 0, s>>>(P, m.pvt.p, m.wells.p, p_new, sw, sg, m.dsw.p, m.dsg.p,
+    const size_t smem = contrib_on_chip(P) ? sizeof(double) * 4 * P.max_substeps * P.nwells : 0;
+    k_well_substeps<<<1, 512, smem, s>>>(P, m.pvt_tab.p, m.wells.p, p_new, sw, sg, m.dsw.p, m.dsg.p,
                                       m.nsub.p, dt, m.wsub.p, m.balances.p, pred); ::impes::count_launch();
     IMPES_CHECK_LAUNCH();
   }
-  unsigned g = grid_for(P.N, kSatBlock);
-  k_saturation_substeps<<<g, kSatBlock, 0, s>>>(P, m.pvt.p, p_new, sw, sg, so, m.dsw.p, m.dsg.p,
+  const unsigned g = sat_grid(P.N);
+  k_saturation_substeps<<<g, kSatBlock, 0, s>>>(P, m.pvt_tab.p, p_new, sw, sg, so, m.dsw.p, m.dsg.p,
                                                 m.pv.p, m.nsub.p, m.red.p, m.counter.p + 1,
                                                 m.balances.p, pred); ::impes::count_launch();
   IMPES_CHECK_LAUNCH();
