@@ -47,6 +47,10 @@ struct Model {
   DBuf<double> pvt_tab;                // by column, with the slopes (as the kernels stage it)
   DBuf<WellDev> wells;
   DBuf<int> wc_cells, wc_ptr, wc_wells;// well-cell -> wells (original order)
+  // per-cell properties of the assembly (total mobility, gravity sum, oil
+  // mobility, capillary pressure, accumulation) and of the saturation update
+  // (water and gas mobility and density, oil-gas capillary pressure)
+  DBuf<double> props;
   // per-step scratch
   DBuf<double> dsw, dsg;               // saturation increments
   DBuf<double> wq;                     // 3 x nwc well sources (q_w, q_g, q_o)
@@ -81,19 +85,14 @@ void model_assemble(Model& m, const double* p, const double* sw, const double* s
 void model_saturation(Model& m, const double* p_new, double* sw, double* sg, double* so,
                       double dt, cudaStream_t s, const int* pred = nullptr);
 
-// Closed-form CSR row pointer of the 7-point pattern (no scan needed).
-__host__ __device__ inline long long pattern_rowptr(long long c, int nx, int ny, int nz) {
-  long long plane = (long long)ny * nz;
-  long long i = c / plane, rem = c % plane, j = rem / nz, k = rem % nz;
-  long long cnt = c;                                           // diagonals
-  long long xm = c - plane; cnt += xm > 0 ? xm : 0;            // rows with i >= 1
-  long long xp_lim = (long long)(nx - 1) * plane; cnt += c < xp_lim ? c : xp_lim;  // i <= nx-2
-  long long jk = j * nz + k;
-  long long ym = jk - nz; cnt += i * (long long)(ny - 1) * nz + (ym > 0 ? ym : 0);
-  long long yp_lim = (long long)(ny - 1) * nz; cnt += i * (long long)(ny - 1) * nz + (jk < yp_lim ? jk : yp_lim);
-  long long col_ = i * ny + j;                                 // columns before
-  cnt += col_ * (nz - 1) + (k - 1 > 0 ? k - 1 : 0);            // k >= 1
-  cnt += col_ * (nz - 1) + (k < nz - 1 ? k : nz - 1);          // k <= nz-2
+// Closed-form CSR row pointer of the 7-point pattern (no scan needed) of cell
+// c = (i ny + j) nz + k: the entries of the rows before it, direction by direction.
+__host__ __device__ inline int pattern_row(int c, int i, int j, int k, int nx, int ny, int nz) {
+  const int plane = ny * nz, jk = j * nz + k, faces_y = i * (ny - 1) * nz, col = i * ny + j;
+  int cnt = c;                                                        // diagonals
+  cnt += (i > 0 ? c - plane : 0) + (i < nx - 1 ? c : (nx - 1) * plane);            // x-, x+
+  cnt += 2 * faces_y + (j > 0 ? jk - nz : 0) + (j < ny - 1 ? jk : (ny - 1) * nz);  // y-, y+
+  cnt += 2 * col * (nz - 1) + (k > 0 ? k - 1 : 0) + k;                             // z-, z+ (k <= nz - 1)
   return cnt;
 }
 

@@ -11,10 +11,9 @@
 // assembled system matches the reference's float64 evaluation to the last bit
 // wherever the reference's arithmetic is elementwise.
 //
-// K1 and K4a stage a 3-D brick of cells plus a one-cell face halo in shared
-// memory: per-cell phase properties (mobilities, densities, capillary pressure,
-// pressure) are evaluated once per brick cell, then every interior cell reads its
-// six neighbours from shared memory.
+// The assembly (K1) and the fluxes (K4a) run in two kernels each: the first
+// evaluates every cell's phase properties once (a few hundred FP64 instructions),
+// the second reads a cell's and its six neighbours' through L1 and L2.
 #include "model.cuh"
 #include <algorithm>
 #include <math.h>
@@ -180,12 +179,12 @@ __device__ __forceinline__ Rho densities(const ModelParams& P, const PvtSmem& t,
 }
 
 // calc_total_compressibility (fluid.py:190-222).
-__device__ double total_compressibility(const ModelParams& P, const PvtSmem& t, double p, double sw,
-                                        double sg) {
+__device__ __forceinline__ double total_compressibility(const ModelParams& P, const PvtSmem& t, double p, double sw,
+                                                        double sg, const PvtAt& at) {
   if (P.pvt_rows == 0) return P.cf;
   const double P_mpa = p / 1e6;
   const double Pp = P_mpa + 0.1, Pm = P_mpa - 0.1;
-  const PvtAt a0 = pvt_find(t, P_mpa * 1e6 / 1e6);
+  const PvtAt a0 = pvt_find_near(t, P_mpa * 1e6 / 1e6, at);
   const PvtAt ap = pvt_find_near(t, Pp * 1e6 / 1e6, a0), am = pvt_find_near(t, Pm * 1e6 / 1e6, a0);
   double c[3];
   const int cols[3] = {C_BW, C_BO, C_BG};
@@ -209,51 +208,6 @@ __device__ __forceinline__ double capillary_og(const ModelParams& P, double sg) 
   const double denom = (1 - P.sw_cr) - P.so_r;
   double sgn = tclamp(sg / (denom + 1e-12), 0.0, 1.0);
   return P.pc_og_scale * tpow(1.0 - sgn + 1e-6, -P.pc_og_exponent);
-}
-
-// Brick geometry shared by K1 and K4a.
-struct Brick {
-  int TI, TJ, TK;      // interior extents
-  int hi, hj, hk;      // halo widths (0 or 1)
-  int HI, HJ, HK;      // halo box extents
-  int nbi, nbj, nbk;   // bricks per dimension
-};
-
-// Interior extents <= 8 (z), <= 8 or 16 (y), and at most 256 cells per brick;
-// each dimension is split evenly so no brick is mostly empty.
-Brick make_brick(const ModelParams& P) {
-  Brick b;
-  b.nbk = (P.nz + 7) / 8;
-  b.TK = (P.nz + b.nbk - 1) / b.nbk;
-  int tj = std::min(P.ny, P.nz == 1 ? 16 : 8);
-  b.nbj = (P.ny + tj - 1) / tj;
-  b.TJ = (P.ny + b.nbj - 1) / b.nbj;
-  int ti = std::max(1, std::min(P.nx, 256 / (b.TK * b.TJ)));
-  b.nbi = (P.nx + ti - 1) / ti;
-  b.TI = (P.nx + b.nbi - 1) / b.nbi;
-  b.hi = P.nx > 1; b.hj = P.ny > 1; b.hk = P.nz > 1;
-  b.HI = b.TI + 2 * b.hi; b.HJ = b.TJ + 2 * b.hj; b.HK = b.TK + 2 * b.hk;
-  return b;
-}
-
-// Raise a kernel's dynamic shared-memory limit when a launch needs more.
-template <typename K>
-void ensure_smem(K kernel, size_t bytes, size_t& current) {
-  static std::mutex mu;   // several host threads may step different models
-  std::lock_guard<std::mutex> lock(mu);
-  if (bytes > current) {
-    raise_smem_limit((const void*)kernel, bytes);
-    current = bytes;
-  }
-}
-size_t g_smem_k1 = 48 << 10, g_smem_k4 = 48 << 10;
-
-__device__ __forceinline__ void brick_origin(const Brick& b, int& i0, int& j0, int& k0) {
-  int bid = blockIdx.x;
-  int bk = bid % b.nbk; bid /= b.nbk;
-  int bj = bid % b.nbj; bid /= b.nbj;
-  int bi = bid;
-  i0 = bi * b.TI; j0 = bj * b.TJ; k0 = bk * b.TK;
 }
 
 // Binary search of `cell` in the sorted distinct well-cell list.
@@ -297,19 +251,14 @@ __global__ void k_transmissibility(ModelParams P, const double* __restrict__ kx,
   }
 }
 
-__global__ void k_pattern(ModelParams P, int* rowptr, int* col) {
-  const long long N = P.N;
-  const long long plane = (long long)P.ny * P.nz;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c <= N;
+__global__ void k_pattern(ModelParams P, int nnz, int* rowptr, int* col) {
+  const int plane = P.ny * P.nz;
+  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c <= P.N;
        c += (long long)gridDim.x * blockDim.x) {
-    long long rp = pattern_rowptr(c, P.nx, P.ny, P.nz);
-    rowptr[c] = (int)rp;
-    if (c == N) continue;
-    int k = c % P.nz;
-    long long r = c / P.nz;
-    int j = r % P.ny;
-    int i = r / P.ny;
-    int e = (int)rp;
+    if (c == P.N) { rowptr[c] = nnz; continue; }
+    const int i = (int)c / plane, r = (int)c - i * plane, j = r / P.nz, k = r - j * P.nz;
+    int e = pattern_row((int)c, i, j, k, P.nx, P.ny, P.nz);
+    rowptr[c] = e;
     if (i > 0) col[e++] = (int)(c - plane);
     if (j > 0) col[e++] = (int)(c - P.nz);
     if (k > 0) col[e++] = (int)(c - 1);
@@ -320,178 +269,188 @@ __global__ void k_pattern(ModelParams P, int* rowptr, int* col) {
   }
 }
 
-// ------------------------------------------------------------ K1 assembly
-// Shared layout per halo cell: p, mw, mo, mg, rw, ro, rg, pc (8 doubles).
-constexpr int kK1Fields = 8;
+// The kernels over cells take them in runs of kCells consecutive ones, a thread
+// each; wells are looked up only in a run that holds a well's cell.
+constexpr int kCells = 256;
+__device__ __forceinline__ bool run_has_well(const int* wc, int nwc, int c0) {
+  int lo = 0, hi = nwc;                 // first well cell at or after c0
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (wc[mid] < c0) lo = mid + 1; else hi = mid;
+  }
+  return lo < nwc && wc[lo] < c0 + kCells;
+}
 
-__global__ void __launch_bounds__(256, 4) k_assemble(
-    ModelParams P, Brick B, const double* __restrict__ pvt_g, const double* __restrict__ p,
-    const double* __restrict__ sw, const double* __restrict__ sg, const double* __restrict__ tx,
-    const double* __restrict__ ty, const double* __restrict__ tz, const double* __restrict__ pv,
+// ------------------------------------------------------------ K1 assembly
+// K1a: per cell (simulation.py:870-882) the total mobility mt, the gravity sum
+// gs = sum of mobility x density, the oil mobility mo, the capillary pressure pc
+// (the last three where the right-hand side reads them) and the accumulation
+// coefficient acc = PV ct / dt (simulation.py:1569-1576).
+// Bound by FP64 and integer instructions, about 900 a cell.  Evaluated in bricks
+// with a one-cell halo in shared memory, every cell's properties were computed
+// 2.0 times and indexed with runtime divisions: 5,800 instructions a cell,
+// 268 us at 1e6 cells for the whole assembly.
+__global__ void __launch_bounds__(kCells) k_cell_props(
+    ModelParams P, const double* __restrict__ pvt_g, const double* __restrict__ p, const double* __restrict__ sw,
+    const double* __restrict__ sg, const double* __restrict__ pv, double dt, double* __restrict__ mt,
+    double* __restrict__ gs, double* __restrict__ mo, double* __restrict__ pc, double* __restrict__ acc) {
+  __shared__ double s_col[kPvtCols * kMaxPvtRows];
+  __shared__ double s_slope[(kPvtCols - 1) * kMaxPvtRows];
+  PvtSmem T{P.pvt_rows, s_col, s_slope};
+  if (P.pvt_rows > 0) pvt_stage(pvt_g, P.pvt_rows, s_col, s_slope);
+  const bool grav = (P.dz > 0) && (P.nz > 1);
+  for (int c = blockIdx.x * kCells + threadIdx.x; c < P.N; c += gridDim.x * kCells) {
+    const double p_ = p[c], swc = sw[c], sgc = sg[c];
+    const KR kr = relperms(P, swc, sgc);
+    const PvtAt at = pvt_at(P, T, p_);
+    const Visc mu = viscosities(P, T, at);
+    const double w = kr.krw / mu.w, o = kr.kro / mu.o, g = kr.krg / mu.g;
+    mt[c] = w + o + g;
+    if (grav) {
+      const Rho r = densities(P, T, p_, at);
+      gs[c] = w * r.w + o * r.o + g * r.g;
+    }
+    if (P.pc_scale > 0) {
+      mo[c] = o;
+      pc[c] = capillary(P, swc);
+    }
+    const double ct = total_compressibility(P, T, p_, swc, sgc, at);
+    acc[c] = pv[c] * ct / dt;
+  }
+}
+
+// K1b: one matrix row and right-hand side entry per cell, from its and its
+// neighbours' properties.  A run's matrix values are one contiguous piece of the
+// CSR array: rows are put together in shared memory and stored from there.
+// Bound by the loads' latency and the 10 doubles a row writes and reads.
+__global__ void __launch_bounds__(kCells) k_assemble(
+    ModelParams P, const double* __restrict__ p, const double* __restrict__ mt, const double* __restrict__ gs,
+    const double* __restrict__ mo, const double* __restrict__ pc, const double* __restrict__ acc,
+    const double* __restrict__ tx, const double* __restrict__ ty, const double* __restrict__ tz,
     const WellDev* __restrict__ wells, const int* __restrict__ wc_cells,
     const int* __restrict__ wc_ptr, const int* __restrict__ wc_wells, int* __restrict__ well_mode,
-    double dt, double* __restrict__ val, double* __restrict__ rhs) {
-  extern __shared__ double smem[];
-  double* s_pvt_col = smem;
-  const int pvt_r = P.pvt_rows > 0 ? P.pvt_rows : 1;     // tables sized by the actual rows
-  double* s_pvt_slope = s_pvt_col + kPvtCols * pvt_r;
-  double* s_cells = s_pvt_slope + (kPvtCols - 1) * pvt_r;
-  const int H = B.HI * B.HJ * B.HK;
-  double* s_p = s_cells;
-  double* s_mw = s_p + H;
-  double* s_mo = s_mw + H;
-  double* s_mg = s_mo + H;
-  double* s_rw = s_mg + H;
-  double* s_ro = s_rw + H;
-  double* s_rg = s_ro + H;
-  double* s_pc = s_rg + H;
-
-  PvtSmem T{P.pvt_rows, s_pvt_col, s_pvt_slope};
-  if (P.pvt_rows > 0) pvt_stage(pvt_g, P.pvt_rows, s_pvt_col, s_pvt_slope);
-
-  int i0, j0, k0;
-  brick_origin(B, i0, j0, k0);
+    double* __restrict__ val, double* __restrict__ rhs) {
+  __shared__ double s_val[7 * kCells];
+  __shared__ int s_e0, s_e1;
   const bool grav = (P.dz > 0) && (P.nz > 1);
-  const long long plane = (long long)P.ny * P.nz;
+  const int plane = P.ny * P.nz;
+  for (int c0 = blockIdx.x * kCells; c0 < P.N; c0 += gridDim.x * kCells) {
+    const int c = c0 + threadIdx.x;
+    const bool has_well = P.nwc > 0 && run_has_well(wc_cells, P.nwc, c0);
+    const int last = min(c0 + kCells, P.N) - 1;
+    int e = 0, entries = 0;
+    double row[7];
+    if (c <= last) {
+      const int i = c / plane, r = c - i * plane, j = r / P.nz, k = r - j * P.nz;
+      const bool hxm = i > 0, hxp = i < P.nx - 1, hym = j > 0, hyp = j < P.ny - 1;
+      const bool hzm = k > 0, hzp = k < P.nz - 1;
+      // the face arrays (one cell less along their own direction)
+      const int iy = c - i * P.nz, iz = c - (i * P.ny + j);
+      const bool have[6] = {hxp, hxm, hyp, hym, hzp, hzm};
+      const int nb[6] = {c + plane, c - plane, c + P.nz, c - P.nz, c + 1, c - 1};
+      const double t_[6] = {hxp ? tx[c] : 0.0, hxm ? tx[c - plane] : 0.0, hyp ? ty[iy] : 0.0,
+                            hym ? ty[iy - P.nz] : 0.0, hzp ? tz[iz] : 0.0, hzm ? tz[iz - 1] : 0.0};
+      const double p0 = p[c], mt0 = mt[c];
+      double pn[6], mn[6];
+#pragma unroll
+      for (int d = 0; d < 6; ++d) {
+        pn[d] = have[d] ? p[nb[d]] : 0.0;
+        mn[d] = have[d] ? mt[nb[d]] : 0.0;
+      }
+      // total-mobility transmissibility of a face, upwind by the pressure of its
+      // lower cell against its upper one (simulation.py:885-895); up[d]: the
+      // upwind side is this cell
+      bool up[6];
+      double tf[6];
+#pragma unroll
+      for (int d = 0; d < 6; ++d) {
+        const bool plus = d % 2 == 0;            // this cell is the lower one
+        const double dp = plus ? p0 - pn[d] : pn[d] - p0;
+        up[d] = plus ? dp > 0 : !(dp > 0);
+        tf[d] = have[d] ? t_[d] * (up[d] ? mt0 : mn[d]) : 0.0;
+      }
 
-  // phase 1: per-cell properties on the brick + face halo (simulation.py:870-882)
-  for (int t = threadIdx.x; t < H; t += blockDim.x) {
-    int lk = t % B.HK, lj = (t / B.HK) % B.HJ, li = t / (B.HK * B.HJ);
-    int i = i0 + li - B.hi, j = j0 + lj - B.hj, k = k0 + lk - B.hk;
-    int out = (li < B.hi || li >= B.hi + B.TI) + (lj < B.hj || lj >= B.hj + B.TJ) +
-              (lk < B.hk || lk >= B.hk + B.TK);
-    if (out > 1 || i < 0 || j < 0 || k < 0 || i >= P.nx || j >= P.ny || k >= P.nz) continue;
-    long long c = ((long long)i * P.ny + j) * P.nz + k;
-    double pc_ = p[c], swc = sw[c], sgc = sg[c];
-    KR kr = relperms(P, swc, sgc);
-    const PvtAt at = pvt_at(P, T, pc_);
-    Visc mu = viscosities(P, T, at);
-    s_p[t] = pc_;
-    s_mw[t] = kr.krw / mu.w;
-    s_mo[t] = kr.kro / mu.o;
-    s_mg[t] = kr.krg / mu.g;
-    if (grav) {
-      Rho r = densities(P, T, pc_, at);
-      s_rw[t] = r.w; s_ro[t] = r.o; s_rg[t] = r.g;
-    }
-    s_pc[t] = capillary(P, swc);
-  }
-  __syncthreads();
-
-  // phase 2: one matrix row and RHS entry per interior cell
-  const int TI = B.TI, TJ = B.TJ, TK = B.TK;
-  for (int t = threadIdx.x; t < TI * TJ * TK; t += blockDim.x) {
-    int tk = t % TK, tj = (t / TK) % TJ, ti = t / (TK * TJ);
-    int i = i0 + ti, j = j0 + tj, k = k0 + tk;
-    if (i >= P.nx || j >= P.ny || k >= P.nz) continue;
-    long long c = ((long long)i * P.ny + j) * P.nz + k;
-    int li = ti + B.hi, lj = tj + B.hj, lk = tk + B.hk;
-    auto sidx = [&](int a, int b_, int d) { return (a * B.HJ + b_) * B.HK + d; };
-    int s0 = sidx(li, lj, lk);
-    auto mt_at = [&](int s) { return s_mw[s] + s_mo[s] + s_mg[s]; };
-    // total-mobility transmissibility of the face (a lower, b upper), upwind by
-    // dp_prev = p_a - p_b > 0 (simulation.py:885-895)
-    auto face_t = [&](double T_, int sa, int sb) {
-      double dp = s_p[sa] - s_p[sb];
-      return T_ * (dp > 0 ? mt_at(sa) : mt_at(sb));
-    };
-    double txm = 0, typ_ = 0, tym = 0, tzp = 0, tzm = 0, txp = 0;
-    const bool hxm = i > 0, hxp = i < P.nx - 1, hym = j > 0, hyp = j < P.ny - 1;
-    const bool hzm = k > 0, hzp = k < P.nz - 1;
-    int sxm = hxm ? sidx(li - 1, lj, lk) : 0, sxp = hxp ? sidx(li + 1, lj, lk) : 0;
-    int sym_ = hym ? sidx(li, lj - 1, lk) : 0, syp = hyp ? sidx(li, lj + 1, lk) : 0;
-    int szm = hzm ? sidx(li, lj, lk - 1) : 0, szp = hzp ? sidx(li, lj, lk + 1) : 0;
-    const long long iy = ((long long)i * (P.ny - 1) + j) * P.nz + k;
-    const long long iz = ((long long)i * P.ny + j) * (P.nz - 1) + k;
-    if (hxm) txm = face_t(tx[c - plane], sxm, s0);
-    if (hxp) txp = face_t(tx[c], s0, sxp);
-    if (hym) tym = face_t(ty[iy - P.nz], sym_, s0);
-    if (hyp) typ_ = face_t(ty[iy], s0, syp);
-    if (hzm) tzm = face_t(tz[iz - 1], szm, s0);
-    if (hzp) tzp = face_t(tz[iz], s0, szp);
-
-    // wells at this cell (simulation.py:1622-1660), in configuration order
-    double well_diag = 0.0, q_well = 0.0;
-    if (P.nwc > 0) {
-      int slot = well_slot(wc_cells, P.nwc, (int)c);
-      if (slot >= 0) {
-        double mt = mt_at(s0);
-        for (int q = wc_ptr[slot]; q < wc_ptr[slot + 1]; ++q) {
-          int w = wc_wells[q];
-          const WellDev W = wells[w];
-          if (W.control_bhp == 0) {
-            double rate_si = (W.value * P.rate_scale) / 86400.0 * (W.is_injector ? 1 : -1);
-            if (!W.is_injector && W.has_bhp_min) {
-              double denom = W.well_index * mt + 1e-12;
-              double p_req = s_p[s0] - rate_si / denom;
-              double p_min = W.bhp_min * 1e6;
-              if (p_req < p_min) {
-                well_mode[w] = 1;
-                well_diag += W.well_index * mt;
-                q_well += W.well_index * mt * p_min;
-                continue;
+      // wells at this cell (simulation.py:1622-1660), in configuration order
+      double well_diag = 0.0, q_well = 0.0;
+      if (has_well) {
+        const int slot = well_slot(wc_cells, P.nwc, c);
+        if (slot >= 0) {
+          for (int q = wc_ptr[slot]; q < wc_ptr[slot + 1]; ++q) {
+            int w = wc_wells[q];
+            const WellDev W = wells[w];
+            if (W.control_bhp == 0) {
+              double rate_si = (W.value * P.rate_scale) / 86400.0 * (W.is_injector ? 1 : -1);
+              if (!W.is_injector && W.has_bhp_min) {
+                double denom = W.well_index * mt0 + 1e-12;
+                double p_req = p0 - rate_si / denom;
+                double p_min = W.bhp_min * 1e6;
+                if (p_req < p_min) {
+                  well_mode[w] = 1;
+                  well_diag += W.well_index * mt0;
+                  q_well += W.well_index * mt0 * p_min;
+                  continue;
+                }
               }
+              well_mode[w] = 0;
+              q_well += rate_si;
+            } else {
+              well_diag += W.well_index * mt0;
+              q_well += W.well_index * mt0 * (W.value * 1e6);
             }
-            well_mode[w] = 0;
-            q_well += rate_si;
-          } else {
-            well_diag += W.well_index * mt;
-            q_well += W.well_index * mt * (W.value * 1e6);
           }
         }
       }
-    }
 
-    // accumulation (simulation.py:1569-1576, 1586-1591)
-    const double ct = total_compressibility(P, T, s_p[s0], sw[c], sg[c]);
-    const double acc = pv[c] * ct / dt;
-    // diagonal in the reference's scatter_add order: x+, x-, y+, y-, z+, z-
-    double diag = 0.0;
-    if (hxp) diag += txp;
-    if (hxm) diag += txm;
-    if (hyp) diag += typ_;
-    if (hym) diag += tym;
-    if (hzp) diag += tzp;
-    if (hzm) diag += tzm;
-    diag += acc;
-    diag += well_diag;
+      // diagonal in the reference's scatter_add order: x+, x-, y+, y-, z+, z-
+      const double acc0 = acc[c];
+      double diag = 0.0;
+#pragma unroll
+      for (int d = 0; d < 6; ++d)
+        if (have[d]) diag += tf[d];
+      diag += acc0;
+      diag += well_diag;
 
-    // row in CSR order: x-, y-, z-, diag, z+, y+, x+
-    long long e = pattern_rowptr(c, P.nx, P.ny, P.nz);
-    if (hxm) val[e++] = -txm;
-    if (hym) val[e++] = -tym;
-    if (hzm) val[e++] = -tzm;
-    val[e++] = diag;
-    if (hzp) val[e++] = -tzp;
-    if (hyp) val[e++] = -typ_;
-    if (hxp) val[e++] = -txp;
+      // row in CSR order: x-, y-, z-, diag, z+, y+, x+
+      e = pattern_row(c, i, j, k, P.nx, P.ny, P.nz);
+      row[0] = -tf[1]; row[1] = -tf[3]; row[2] = -tf[5]; row[3] = diag;
+      row[4] = -tf[4]; row[5] = -tf[2]; row[6] = -tf[0];
+      entries = (hxm ? 1 : 0) | (hym ? 2 : 0) | (hzm ? 4 : 0) | 8 | (hzp ? 16 : 0) | (hyp ? 32 : 0) | (hxp ? 64 : 0);
 
-    // right-hand side (simulation.py:1582-1620)
-    const double comp = acc * s_p[s0];
-    double qg = 0.0;
-    if (grav) {
-      auto gflow = [&](double T_, int sa, int sb) {
-        int su = (s_p[sa] - s_p[sb] > 0) ? sa : sb;
-        return T_ * P.gravity * P.dz *
-               (s_mw[su] * s_rw[su] + s_mo[su] * s_ro[su] + s_mg[su] * s_rg[su]);
-      };
-      if (hzp) qg -= gflow(tz[iz], s0, szp);
-      if (hzm) qg += gflow(tz[iz - 1], szm, s0);
+      // right-hand side (simulation.py:1582-1620)
+      const double comp = acc0 * p0;
+      double qg = 0.0;
+      if (grav) {
+        const double gs0 = gs[c];
+        if (hzp) qg -= t_[4] * P.gravity * P.dz * (up[4] ? gs0 : gs[c + 1]);
+        if (hzm) qg += t_[5] * P.gravity * P.dz * (up[5] ? gs0 : gs[c - 1]);
+      }
+      double qpc = 0.0;
+      if (P.pc_scale > 0) {
+        const double mo0 = mo[c], pc0 = pc[c];
+        // the reference's order: x-, x+, y-, y+, z-, z+
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+          const int d = q ^ 1;
+          if (!have[d]) continue;
+          const double m = up[d] ? mo0 : mo[nb[d]];
+          if (d % 2) qpc += t_[d] * m * (pc0 - pc[nb[d]]);
+          else qpc -= t_[d] * m * (pc[nb[d]] - pc0);
+        }
+      }
+      rhs[c] = comp + q_well + qg + qpc;
+      if (c == c0) s_e0 = e;
+      if (c == last) s_e1 = e + __popc(entries);
     }
-    double qpc = 0.0;
-    if (P.pc_scale > 0) {
-      auto pflow = [&](double T_, int sa, int sb) {
-        double mo = (s_p[sa] - s_p[sb] > 0) ? s_mo[sa] : s_mo[sb];
-        return T_ * mo * (s_pc[sb] - s_pc[sa]);
-      };
-      if (hxm) qpc += pflow(tx[c - plane], sxm, s0);
-      if (hxp) qpc -= pflow(tx[c], s0, sxp);
-      if (hym) qpc += pflow(ty[iy - P.nz], sym_, s0);
-      if (hyp) qpc -= pflow(ty[iy], s0, syp);
-      if (hzm) qpc += pflow(tz[iz - 1], szm, s0);
-      if (hzp) qpc -= pflow(tz[iz], s0, szp);
+    __syncthreads();
+    if (entries) {
+      int at = e - s_e0;
+#pragma unroll
+      for (int d = 0; d < 7; ++d)
+        if (entries >> d & 1) s_val[at++] = row[d];
     }
-    rhs[c] = comp + q_well + qg + qpc;
+    __syncthreads();
+    for (int x = threadIdx.x; x < s_e1 - s_e0; x += kCells) val[s_e0 + x] = s_val[x];
+    __syncthreads();
   }
 }
 
@@ -699,99 +658,99 @@ __global__ void k_well_sources(ModelParams P, const double* __restrict__ pvt_g,
 }
 
 // K4a: fluxes, divergence, dS and the substep ratio (simulation.py:968-1042, 1351-1379).
-constexpr int kK4Fields = 6;  // p, mw, mg, rw, rg, pcog
+// K4a': water and gas mobilities and densities and the oil-gas capillary pressure
+// of every cell, at the new pressure.
+__global__ void __launch_bounds__(kCells) k_flux_props(
+    ModelParams P, const double* __restrict__ pvt_g, const double* __restrict__ p, const double* __restrict__ sw,
+    const double* __restrict__ sg, double* __restrict__ mw, double* __restrict__ mg, double* __restrict__ rw,
+    double* __restrict__ rg, double* __restrict__ pcg, const int* pred) {
+  if (pred && *pred == 0) return;
+  __shared__ double s_col[kPvtCols * kMaxPvtRows];
+  __shared__ double s_slope[(kPvtCols - 1) * kMaxPvtRows];
+  PvtSmem T{P.pvt_rows, s_col, s_slope};
+  if (P.pvt_rows > 0) pvt_stage(pvt_g, P.pvt_rows, s_col, s_slope);
+  const bool grav = (P.dz > 0) && (P.nz > 1);
+  for (int c = blockIdx.x * kCells + threadIdx.x; c < P.N; c += gridDim.x * kCells) {
+    const double p_ = p[c], swc = sw[c], sgc = sg[c];
+    const KR kr = relperms(P, swc, sgc);
+    const PvtAt at = pvt_at(P, T, p_);
+    const Visc mu = viscosities(P, T, at);
+    mw[c] = kr.krw / mu.w;
+    mg[c] = kr.krg / mu.g;
+    if (grav) {
+      const Rho r = densities(P, T, p_, at);
+      rw[c] = r.w;
+      rg[c] = r.g;
+    }
+    if (P.pc_og_scale > 0) pcg[c] = capillary_og(P, sgc);
+  }
+}
 
-__global__ void __launch_bounds__(256, 4) k_saturation_flux(
-    ModelParams P, Brick B, const double* __restrict__ pvt_g, const double* __restrict__ p,
+__global__ void __launch_bounds__(kCells) k_saturation_flux(
+    ModelParams P, const double* __restrict__ p, const double* __restrict__ mw, const double* __restrict__ mg,
+    const double* __restrict__ rw, const double* __restrict__ rg, const double* __restrict__ pcg,
     const double* __restrict__ sw, const double* __restrict__ sg, const double* __restrict__ tx,
     const double* __restrict__ ty, const double* __restrict__ tz, const double* __restrict__ pv,
     const int* __restrict__ wc_cells, const double* __restrict__ wq, double dt,
     double* __restrict__ dsw_out, double* __restrict__ dsg_out, double* __restrict__ red,
     unsigned* __restrict__ counter, int* __restrict__ nsub_out, const int* pred) {
   if (pred && *pred == 0) return;
-  extern __shared__ double smem[];
-  double* s_pvt_col = smem;
-  const int pvt_r = P.pvt_rows > 0 ? P.pvt_rows : 1;     // tables sized by the actual rows
-  double* s_pvt_slope = s_pvt_col + kPvtCols * pvt_r;
-  double* s_cells = s_pvt_slope + (kPvtCols - 1) * pvt_r;
-  const int H = B.HI * B.HJ * B.HK;
-  double* s_p = s_cells;
-  double* s_mw = s_p + H;
-  double* s_mg = s_mw + H;
-  double* s_rw = s_mg + H;
-  double* s_rg = s_rw + H;
-  double* s_pcg = s_rg + H;
   __shared__ double s_red[3 * 8];
   __shared__ bool s_last;
-
-  PvtSmem T{P.pvt_rows, s_pvt_col, s_pvt_slope};
-  if (P.pvt_rows > 0) pvt_stage(pvt_g, P.pvt_rows, s_pvt_col, s_pvt_slope);
-  int i0, j0, k0;
-  brick_origin(B, i0, j0, k0);
   const bool grav = (P.dz > 0) && (P.nz > 1);
-  const long long plane = (long long)P.ny * P.nz;
-  for (int t = threadIdx.x; t < H; t += blockDim.x) {
-    int lk = t % B.HK, lj = (t / B.HK) % B.HJ, li = t / (B.HK * B.HJ);
-    int i = i0 + li - B.hi, j = j0 + lj - B.hj, k = k0 + lk - B.hk;
-    int out = (li < B.hi || li >= B.hi + B.TI) + (lj < B.hj || lj >= B.hj + B.TJ) +
-              (lk < B.hk || lk >= B.hk + B.TK);
-    if (out > 1 || i < 0 || j < 0 || k < 0 || i >= P.nx || j >= P.ny || k >= P.nz) continue;
-    long long c = ((long long)i * P.ny + j) * P.nz + k;
-    double pc_ = p[c], swc = sw[c], sgc = sg[c];
-    KR kr = relperms(P, swc, sgc);
-    const PvtAt at = pvt_at(P, T, pc_);
-    Visc mu = viscosities(P, T, at);
-    s_p[t] = pc_;
-    s_mw[t] = kr.krw / mu.w;
-    s_mg[t] = kr.krg / mu.g;
-    if (grav) {
-      Rho r = densities(P, T, pc_, at);
-      s_rw[t] = r.w; s_rg[t] = r.g;
-    }
-    s_pcg[t] = capillary_og(P, sgc);
-  }
-  __syncthreads();
-
+  const bool pcog = P.pc_og_scale > 0;
+  const int plane = P.ny * P.nz;
   double rmax = 0.0, rnan = 0.0, rinf = 0.0;
-  const int TI = B.TI, TJ = B.TJ, TK = B.TK;
-  for (int t = threadIdx.x; t < TI * TJ * TK; t += blockDim.x) {
-    int tk = t % TK, tj = (t / TK) % TJ, ti = t / (TK * TJ);
-    int i = i0 + ti, j = j0 + tj, k = k0 + tk;
-    if (i >= P.nx || j >= P.ny || k >= P.nz) continue;
-    long long c = ((long long)i * P.ny + j) * P.nz + k;
-    int li = ti + B.hi, lj = tj + B.hj, lk = tk + B.hk;
-    auto sidx = [&](int a, int b_, int d) { return (a * B.HJ + b_) * B.HK + d; };
-    int s0 = sidx(li, lj, lk);
-    const long long iy = ((long long)i * (P.ny - 1) + j) * P.nz + k;
-    const long long iz = ((long long)i * P.ny + j) * (P.nz - 1) + k;
-    const bool pcog = P.pc_og_scale > 0;
-    // water / gas flux through face (sa lower, sb upper) in direction d (0 x, 1 y, 2 z)
-    auto flux = [&](double T_, int sa, int sb, bool zdir, double& fw, double& fg) {
-      double dp = s_p[sa] - s_p[sb];
-      bool up = dp > 0;
-      double mw = up ? s_mw[sa] : s_mw[sb];
-      double mg = up ? s_mg[sa] : s_mg[sb];
+  for (int c0 = blockIdx.x * kCells; c0 < P.N; c0 += gridDim.x * kCells) {
+    const bool has_well = P.nwc > 0 && run_has_well(wc_cells, P.nwc, c0);
+    const int c = c0 + threadIdx.x;
+    if (c >= P.N) continue;
+    const int i = c / plane, r = c - i * plane, j = r / P.nz, k = r - j * P.nz;
+    const int iy = c - i * P.nz, iz = c - (i * P.ny + j);
+    // the reference's order of a cell's faces: x+, x-, y+, y-, z+, z-
+    const bool have[6] = {i < P.nx - 1, i > 0, j < P.ny - 1, j > 0, k < P.nz - 1, k > 0};
+    const int nb[6] = {c + plane, c - plane, c + P.nz, c - P.nz, c + 1, c - 1};
+    const double t_[6] = {have[0] ? tx[c] : 0.0, have[1] ? tx[c - plane] : 0.0, have[2] ? ty[iy] : 0.0,
+                          have[3] ? ty[iy - P.nz] : 0.0, have[4] ? tz[iz] : 0.0, have[5] ? tz[iz - 1] : 0.0};
+    const double p0 = p[c], mw0 = mw[c], mg0 = mg[c];
+    double pn[6], wn[6], gn[6];
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+      pn[d] = have[d] ? p[nb[d]] : 0.0;
+      wn[d] = have[d] ? mw[nb[d]] : 0.0;
+      gn[d] = have[d] ? mg[nb[d]] : 0.0;
+    }
+    const double rw0 = grav ? rw[c] : 0.0, rg0 = grav ? rg[c] : 0.0, pcg0 = pcog ? pcg[c] : 0.0;
+    double dw = 0.0, dg = 0.0;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+      if (!have[d]) continue;
+      const bool plus = d % 2 == 0;              // this cell is the face's lower one
+      const double dp = plus ? p0 - pn[d] : pn[d] - p0;
+      const bool up = plus ? dp > 0 : !(dp > 0); // the upwind side is this cell
+      const double m_w = up ? mw0 : wn[d], m_g = up ? mg0 : gn[d];
       double pw = dp, pg = dp;
-      if (zdir && grav) {
-        double rwa = 0.5 * (s_rw[sa] + s_rw[sb]);
-        double rga = 0.5 * (s_rg[sa] + s_rg[sb]);
+      if (d >= 4 && grav) {
+        const double rwn = rw[nb[d]], rgn = rg[nb[d]];
+        const double rwa = 0.5 * (plus ? rw0 + rwn : rwn + rw0);
+        const double rga = 0.5 * (plus ? rg0 + rgn : rgn + rg0);
         pw = dp + P.gravity * rwa * P.dz;
         pg = dp + P.gravity * rga * P.dz;
       }
-      fw = T_ * mw * pw;
-      if (pcog) fg = T_ * mg * (pg - (s_pcg[sb] - s_pcg[sa]));
-      else fg = T_ * mg * pg;
-    };
-    double dw = 0.0, dg = 0.0, fw, fg;
-    if (i < P.nx - 1) { flux(tx[c], s0, sidx(li + 1, lj, lk), false, fw, fg); dw += fw; dg += fg; }
-    if (i > 0) { flux(tx[c - plane], sidx(li - 1, lj, lk), s0, false, fw, fg); dw -= fw; dg -= fg; }
-    if (j < P.ny - 1) { flux(ty[iy], s0, sidx(li, lj + 1, lk), false, fw, fg); dw += fw; dg += fg; }
-    if (j > 0) { flux(ty[iy - P.nz], sidx(li, lj - 1, lk), s0, false, fw, fg); dw -= fw; dg -= fg; }
-    if (k < P.nz - 1) { flux(tz[iz], s0, sidx(li, lj, lk + 1), true, fw, fg); dw += fw; dg += fg; }
-    if (k > 0) { flux(tz[iz - 1], sidx(li, lj, lk - 1), s0, true, fw, fg); dw -= fw; dg -= fg; }
+      const double fw = t_[d] * m_w * pw;
+      double fg;
+      if (pcog) {
+        const double pcn = pcg[nb[d]];
+        fg = t_[d] * m_g * (pg - (plus ? pcn - pcg0 : pcg0 - pcn));
+      } else {
+        fg = t_[d] * m_g * pg;
+      }
+      if (plus) { dw += fw; dg += fg; }
+      else { dw -= fw; dg -= fg; }
+    }
     double qwc = 0.0, qgc = 0.0;
-    if (P.nwc > 0) {
-      int slot = well_slot(wc_cells, P.nwc, (int)c);
+    if (has_well) {
+      const int slot = well_slot(wc_cells, P.nwc, c);
       if (slot >= 0) { qwc = wq[slot]; qgc = wq[P.nwc + slot]; }
     }
     const double f = dt / pv[c];
@@ -804,10 +763,10 @@ __global__ void __launch_bounds__(256, 4) k_saturation_flux(
     const double sw_dn = tclamp_min(swc - P.sw_cr, 0.0);
     const double sg_up = tclamp_min(1.0 - P.so_r - swc - sgc, 0.0);
     const double sg_dn = tclamp_min(sgc - P.sg_cr, 0.0);
-    double rw = dSw > 0 ? dSw / tclamp_min(sw_up, eps) : (-dSw) / tclamp_min(sw_dn, eps);
-    double rg = dSg > 0 ? dSg / tclamp_min(sg_up, eps) : (-dSg) / tclamp_min(sg_dn, eps);
+    double rw_ = dSw > 0 ? dSw / tclamp_min(sw_up, eps) : (-dSw) / tclamp_min(sw_dn, eps);
+    double rg_ = dSg > 0 ? dSg / tclamp_min(sg_up, eps) : (-dSg) / tclamp_min(sg_dn, eps);
     double rl = tmaximum(fabs(dSw) / P.max_dS, fabs(dSg) / P.max_dS);
-    double rat = tmaximum(tmaximum(rw, rg), rl);
+    double rat = tmaximum(tmaximum(rw_, rg_), rl);
     if (isnan(rat)) rnan = 1.0;
     else if (isinf(rat)) rinf = 1.0;
     else rmax = fmax(rmax, rat);
@@ -1043,12 +1002,6 @@ __global__ void __launch_bounds__(kSatBlock) k_saturation_substeps(
   }
 }
 
-size_t brick_smem(const Brick& b, int fields, int pvt_rows) {
-  const size_t r = pvt_rows > 0 ? (size_t)pvt_rows : 1;
-  return sizeof(double) * ((size_t)kPvtCols * r + (size_t)(kPvtCols - 1) * r +
-                           (size_t)fields * b.HI * b.HJ * b.HK);
-}
-
 }  // namespace
 
 // blocks of the substep kernel: up to eight an SM, each with several cells a
@@ -1068,14 +1021,15 @@ void model_build_static(Model& m, const double* kx, const double* ky, const doub
   k_transmissibility<<<grid_for(P.N, 256), 256, 0, s>>>(P, kx, ky, kz, poro, m.tx.p, m.ty.p,
                                                         m.tz.p, m.pv.p); ::impes::count_launch();
   IMPES_CHECK_LAUNCH();
-  m.nnz = (int)pattern_rowptr(P.N, P.nx, P.ny, P.nz);
+  const long long faces = (long long)(P.nx - 1) * P.ny * P.nz + (long long)P.nx * (P.ny - 1) * P.nz +
+                          (long long)P.nx * P.ny * (P.nz - 1);
+  m.nnz = (int)(P.N + 2 * faces);
   m.rowptr.alloc(P.N + 1);
   m.col.alloc(m.nnz);
-  k_pattern<<<grid_for(P.N + 1, 256), 256, 0, s>>>(P, m.rowptr.p, m.col.p); ::impes::count_launch();
+  k_pattern<<<grid_for(P.N + 1, 256), 256, 0, s>>>(P, m.nnz, m.rowptr.p, m.col.p); ::impes::count_launch();
   IMPES_CHECK_LAUNCH();
-  Brick b = make_brick(P);
-  int blocks = b.nbi * b.nbj * b.nbk;
-  m.red_blocks = std::max(blocks, (int)sat_grid(P.N));
+  m.red_blocks = (int)sat_grid(P.N);
+  m.props.alloc((size_t)5 * P.N);
   m.red.alloc((size_t)6 * m.red_blocks + 16);
   m.counter.alloc(2);
   IMPES_CUDA(cudaMemsetAsync(m.counter.p, 0, 2 * sizeof(unsigned), s));
@@ -1098,14 +1052,15 @@ void model_pattern(Model& m, int* rowptr, int* col, cudaStream_t s) {
 
 void model_assemble(Model& m, const double* p, const double* sw, const double* sg, double dt,
                     double* csr_val, double* rhs, cudaStream_t s) {
-  Brick b = make_brick(m.P);
-  int blocks = b.nbi * b.nbj * b.nbk;
-  ensure_smem(k_assemble, brick_smem(b, kK1Fields, m.P.pvt_rows), g_smem_k1);
   const double F = 0.5 * (double)(m.nnz - m.P.N);
   const int tid = timers().begin(IMPES_PH_ASSEMBLE, s);
-  k_assemble<<<blocks, 256, brick_smem(b, kK1Fields, m.P.pvt_rows), s>>>(
-      m.P, b, m.pvt_tab.p, p, sw, sg, m.tx.p, m.ty.p, m.tz.p, m.pv.p, m.wells.p, m.wc_cells.p,
-      m.wc_ptr.p, m.wc_wells.p, m.well_mode.p, dt, csr_val, rhs); ::impes::count_launch();
+  const size_t n = m.P.N;
+  double *mt = m.props.p, *gs = mt + n, *mo = gs + n, *pc = mo + n, *acc = pc + n;
+  const unsigned g = sat_grid(m.P.N);
+  k_cell_props<<<g, kCells, 0, s>>>(m.P, m.pvt_tab.p, p, sw, sg, m.pv.p, dt, mt, gs, mo, pc, acc);
+  k_assemble<<<g, kCells, 0, s>>>(m.P, p, mt, gs, mo, pc, acc, m.tx.p, m.ty.p, m.tz.p, m.wells.p, m.wc_cells.p,
+                                  m.wc_ptr.p, m.wc_wells.p, m.well_mode.p, csr_val, rhs);
+  ::impes::count_launches(2);
   IMPES_CHECK_LAUNCH();
   timers().end(tid, s, 8.0 * (6.0 * m.P.N + 3.0 * F));   // reads p, Sw, Sg, PV, T; writes A, b
 }
@@ -1119,12 +1074,14 @@ void model_saturation(Model& m, const double* p_new, double* sw, double* sg, dou
                                      dt, m.wq.p, m.balances.p, m.well_q.p, m.well_rates.p, pred); ::impes::count_launch();
     IMPES_CHECK_LAUNCH();
   }
-  Brick b = make_brick(P);
-  int blocks = b.nbi * b.nbj * b.nbk;
-  ensure_smem(k_saturation_flux, brick_smem(b, kK4Fields, P.pvt_rows), g_smem_k4);
-  k_saturation_flux<<<blocks, 256, brick_smem(b, kK4Fields, P.pvt_rows), s>>>(
-      P, b, m.pvt_tab.p, p_new, sw, sg, m.tx.p, m.ty.p, m.tz.p, m.pv.p, m.wc_cells.p, m.wq.p, dt,
-      m.dsw.p, m.dsg.p, m.red.p, m.counter.p, m.nsub.p, pred); ::impes::count_launch();
+  const unsigned g = sat_grid(P.N);
+  const size_t n = P.N;
+  double *mw = m.props.p, *mg = mw + n, *rw = mg + n, *rg = rw + n, *pcg = rg + n;
+  k_flux_props<<<g, kCells, 0, s>>>(P, m.pvt_tab.p, p_new, sw, sg, mw, mg, rw, rg, pcg, pred);
+  k_saturation_flux<<<g, kCells, 0, s>>>(P, p_new, mw, mg, rw, rg, pcg, sw, sg, m.tx.p, m.ty.p, m.tz.p, m.pv.p,
+                                         m.wc_cells.p, m.wq.p, dt, m.dsw.p, m.dsg.p, m.red.p, m.counter.p,
+                                         m.nsub.p, pred);
+  ::impes::count_launches(2);
   IMPES_CHECK_LAUNCH();
   if (P.pvt_rows > 0 && P.nwells > 0) {
     const size_t smem = contrib_on_chip(P) ? sizeof(double) * 4 * P.max_substeps * P.nwells : 0;
@@ -1132,7 +1089,6 @@ void model_saturation(Model& m, const double* p_new, double* sw, double* sg, dou
                                       m.nsub.p, dt, m.wsub.p, m.balances.p, pred); ::impes::count_launch();
     IMPES_CHECK_LAUNCH();
   }
-  const unsigned g = sat_grid(P.N);
   k_saturation_substeps<<<g, kSatBlock, 0, s>>>(P, m.pvt_tab.p, p_new, sw, sg, so, m.dsw.p, m.dsg.p,
                                                 m.pv.p, m.nsub.p, m.red.p, m.counter.p + 1,
                                                 m.balances.p, pred); ::impes::count_launch();
