@@ -53,7 +53,8 @@ struct Model {
   DBuf<double> props;
   // per-step scratch
   DBuf<double> dsw, dsg;               // saturation increments
-  DBuf<double> wq;                     // 3 x nwc well sources (q_w, q_g, q_o)
+  DBuf<double> wterms;                 // per well: its sources and balance terms (physics.cu, WellTerms)
+  DBuf<double> wstate;                 // nwc x (Sw, Sg, dSw, dSg) before the substeps
   DBuf<double> wsub;                   // per (substep, well) component-balance addends
   DBuf<double> red;                    // block partials for reductions
   DBuf<unsigned> counter;              // last-block counters

@@ -179,10 +179,10 @@ __device__ __forceinline__ Rho densities(const ModelParams& P, const PvtSmem& t,
 }
 
 // calc_total_compressibility (fluid.py:190-222).
-__device__ __forceinline__ double total_compressibility(const ModelParams& P, const PvtSmem& t, double p, double sw,
-                                                        double sg, const PvtAt& at) {
+__device__ __forceinline__ double total_compressibility(const ModelParams& P, const PvtSmem& t, double sw, double sg,
+                                                        const PvtAt& at) {
   if (P.pvt_rows == 0) return P.cf;
-  const double P_mpa = p / 1e6;
+  const double P_mpa = at.x;            // p / 1e6
   const double Pp = P_mpa + 0.1, Pm = P_mpa - 0.1;
   const PvtAt a0 = pvt_find_near(t, P_mpa * 1e6 / 1e6, at);
   const PvtAt ap = pvt_find_near(t, Pp * 1e6 / 1e6, a0), am = pvt_find_near(t, Pm * 1e6 / 1e6, a0);
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kCells) k_cell_props(
       mo[c] = o;
       pc[c] = capillary(P, swc);
     }
-    const double ct = total_compressibility(P, T, p_, swc, sgc, at);
+    const double ct = total_compressibility(P, T, swc, sgc, at);
     acc[c] = pv[c] * ct / dt;
   }
 }
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kCells) k_cell_props(
 // neighbours' properties.  A run's matrix values are one contiguous piece of the
 // CSR array: rows are put together in shared memory and stored from there.
 // Bound by the loads' latency and the 10 doubles a row writes and reads.
-__global__ void __launch_bounds__(kCells) k_assemble(
+__global__ void __launch_bounds__(kCells, 3) k_assemble(
     ModelParams P, const double* __restrict__ p, const double* __restrict__ mt, const double* __restrict__ gs,
     const double* __restrict__ mo, const double* __restrict__ pc, const double* __restrict__ acc,
     const double* __restrict__ tx, const double* __restrict__ ty, const double* __restrict__ tz,
@@ -468,36 +468,35 @@ __device__ void well_cell_phase(const ModelParams& P, const PvtSmem& T, double p
   fo = mo / (mt + 1e-10);
 }
 
-__global__ void k_well_sources(ModelParams P, const double* __restrict__ pvt_g,
-                               const WellDev* __restrict__ wells, const int* __restrict__ wc_cells,
-                               const double* __restrict__ p_new, const double* __restrict__ sw,
-                               const double* __restrict__ sg, const double* __restrict__ pv,
-                               double dt, double* wq /*3*nwc*/, double* bal /*12*/,
-                               double* well_q, double* well_rates, const int* pred) {
-  if (pred && *pred == 0) return;
-  __shared__ double s_col[kPvtCols * kMaxPvtRows];
-  __shared__ double s_slope[(kPvtCols - 1) * kMaxPvtRows];
-  // per well: its additions to the (water, gas, oil) sources of its cell and to
-  // the component balance (oil in, oil out, gas in, gas out), which phase 2 adds
-  // up in well order; bit k of s_mask marks addition k as made
-  __shared__ double s_q[kMaxWells][3];
-  __shared__ double s_b[kMaxWells][4];
-  __shared__ int s_mask[kMaxWells];
-  __shared__ int s_slot[kMaxWells];
-  PvtSmem T{P.pvt_rows, s_col, s_slope};
-  if (P.pvt_rows > 0) pvt_stage(pvt_g, P.pvt_rows, s_col, s_slope);
+// What a well adds: to the (water, gas, oil) sources of its cell and to the
+// component balance (oil in, oil out, gas in, gas out); bit k of mask marks
+// addition k as made.
+struct WellTerms {
+  double q[3], b[4];
+  int mask, pad;
+};
+struct WellArgs {
+  const WellDev* wells;
+  const int *wc_cells, *wc_ptr, *wc_wells;
+  WellTerms* terms;    // per well
+  double* state;       // per well cell: Sw, Sg and their increments before the substeps
+  double* bal;         // 12 balances
+  double* well_q;
+  double* well_rates;
+};
+// A well's terms, by one thread (they depend only on its cell's state).
+__device__ __noinline__ void well_source(const ModelParams& P, const PvtSmem& T, const WellArgs& A, int w,
+                                         const double* __restrict__ p_new, const double* __restrict__ sw,
+                                         const double* __restrict__ sg, const double* __restrict__ pv, double dt) {
+  double *well_q = A.well_q, *well_rates = A.well_rates;
   const bool pvt = P.pvt_rows > 0;
   const double so_r = P.so_r, sw_min = P.sw_cr, sg_min = P.sg_cr;
-  // phase 1: every well on its own thread (a well's numbers depend only on its
-  // cell's state)
-  for (int w = threadIdx.x; w < P.nwells; w += blockDim.x) {
-    const WellDev W = wells[w];
+  {
+    const WellDev W = A.wells[w];
     const int c = W.cell;
     int mask = 0;
     double dq[3] = {0.0, 0.0, 0.0}, db[4] = {0.0, 0.0, 0.0, 0.0};
-    s_slot[w] = -1;
     if (c >= 0) {  // a well outside the grid contributes nothing (simulation.py:1053-1054)
-      s_slot[w] = well_slot(wc_cells, P.nwc, c);
       const double p = p_new[c], sw_c = sw[c], sg_c = sg[c], pv_c = pv[c];
       double mt, fw_, fg_, fo_;
       well_cell_phase(P, T, p, sw_c, sg_c, mt, fw_, fg_, fo_);
@@ -627,48 +626,29 @@ __global__ void k_well_sources(ModelParams P, const double* __restrict__ pvt_g,
         }
       }
     }
-    s_mask[w] = mask;
-    for (int k = 0; k < 3; ++k) s_q[w][k] = dq[k];
-    for (int k = 0; k < 4; ++k) s_b[w][k] = db[k];
+    WellTerms& t = A.terms[w];
+    t.mask = mask;
+    for (int k = 0; k < 3; ++k) t.q[k] = dq[k];
+    for (int k = 0; k < 4; ++k) t.b[k] = db[k];
   }
-  __syncthreads();
-  // phase 2: the sums in the reference's well order (one thread), kept on chip
-  __shared__ double s_wq[3 * kMaxWells];
-  for (int t = threadIdx.x; t < 3 * P.nwc; t += blockDim.x) s_wq[t] = 0.0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double b0 = bal[6 + 0], b1 = bal[6 + 1], b3 = bal[6 + 3], b4 = bal[6 + 4];
-    for (int w = 0; w < P.nwells; ++w) {
-      const int slot = s_slot[w], mask = s_mask[w];
-      if (slot < 0) continue;
-      if (mask & 1) s_wq[slot] += s_q[w][0];
-      if (mask & 2) s_wq[P.nwc + slot] += s_q[w][1];
-      if (mask & 4) s_wq[2 * P.nwc + slot] += s_q[w][2];
-      // balance additions in the order the serial loop made them: gas in then
-      // oil in (gas injectors), oil out then gas out (producers)
-      if (mask & 32) b3 += s_b[w][2];
-      if (mask & 8) b0 += s_b[w][0];
-      if (mask & 16) b1 += s_b[w][1];
-      if (mask & 64) b4 += s_b[w][3];
-    }
-    bal[6 + 0] = b0; bal[6 + 1] = b1; bal[6 + 3] = b3; bal[6 + 4] = b4;
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < 3 * P.nwc; t += blockDim.x) wq[t] = s_wq[t];
 }
 
 // K4a: fluxes, divergence, dS and the substep ratio (simulation.py:968-1042, 1351-1379).
 // K4a': water and gas mobilities and densities and the oil-gas capillary pressure
-// of every cell, at the new pressure.
-__global__ void __launch_bounds__(kCells) k_flux_props(
+// of every cell, at the new pressure; one thread a block also forms a well's terms.
+__global__ void __launch_bounds__(kCells, 4) k_flux_props(
     ModelParams P, const double* __restrict__ pvt_g, const double* __restrict__ p, const double* __restrict__ sw,
-    const double* __restrict__ sg, double* __restrict__ mw, double* __restrict__ mg, double* __restrict__ rw,
-    double* __restrict__ rg, double* __restrict__ pcg, const int* pred) {
+    const double* __restrict__ sg, const double* __restrict__ pv, double dt, double* __restrict__ mw,
+    double* __restrict__ mg, double* __restrict__ rw, double* __restrict__ rg, double* __restrict__ pcg, WellArgs A,
+    const int* pred) {
   if (pred && *pred == 0) return;
   __shared__ double s_col[kPvtCols * kMaxPvtRows];
   __shared__ double s_slope[(kPvtCols - 1) * kMaxPvtRows];
   PvtSmem T{P.pvt_rows, s_col, s_slope};
   if (P.pvt_rows > 0) pvt_stage(pvt_g, P.pvt_rows, s_col, s_slope);
+  // (all wells in one block were its critical path: 47 us against 32)
+  if (threadIdx.x == 0)
+    for (int w = blockIdx.x; w < P.nwells; w += gridDim.x) well_source(P, T, A, w, p, sw, sg, pv, dt);
   const bool grav = (P.dz > 0) && (P.nz > 1);
   for (int c = blockIdx.x * kCells + threadIdx.x; c < P.N; c += gridDim.x * kCells) {
     const double p_ = p[c], swc = sw[c], sgc = sg[c];
@@ -686,14 +666,13 @@ __global__ void __launch_bounds__(kCells) k_flux_props(
   }
 }
 
-__global__ void __launch_bounds__(kCells) k_saturation_flux(
+__global__ void __launch_bounds__(kCells, 3) k_saturation_flux(
     ModelParams P, const double* __restrict__ p, const double* __restrict__ mw, const double* __restrict__ mg,
     const double* __restrict__ rw, const double* __restrict__ rg, const double* __restrict__ pcg,
     const double* __restrict__ sw, const double* __restrict__ sg, const double* __restrict__ tx,
     const double* __restrict__ ty, const double* __restrict__ tz, const double* __restrict__ pv,
-    const int* __restrict__ wc_cells, const double* __restrict__ wq, double dt,
-    double* __restrict__ dsw_out, double* __restrict__ dsg_out, double* __restrict__ red,
-    unsigned* __restrict__ counter, int* __restrict__ nsub_out, const int* pred) {
+    WellArgs A, double dt, double* __restrict__ dsw_out, double* __restrict__ dsg_out,
+    double* __restrict__ red, unsigned* __restrict__ counter, int* __restrict__ nsub_out, const int* pred) {
   if (pred && *pred == 0) return;
   __shared__ double s_red[3 * 8];
   __shared__ bool s_last;
@@ -702,7 +681,7 @@ __global__ void __launch_bounds__(kCells) k_saturation_flux(
   const int plane = P.ny * P.nz;
   double rmax = 0.0, rnan = 0.0, rinf = 0.0;
   for (int c0 = blockIdx.x * kCells; c0 < P.N; c0 += gridDim.x * kCells) {
-    const bool has_well = P.nwc > 0 && run_has_well(wc_cells, P.nwc, c0);
+    const bool has_well = P.nwc > 0 && run_has_well(A.wc_cells, P.nwc, c0);
     const int c = c0 + threadIdx.x;
     if (c >= P.N) continue;
     const int i = c / plane, r = c - i * plane, j = r / P.nz, k = r - j * P.nz;
@@ -749,9 +728,15 @@ __global__ void __launch_bounds__(kCells) k_saturation_flux(
       else { dw -= fw; dg -= fg; }
     }
     double qwc = 0.0, qgc = 0.0;
+    int slot = -1;
     if (has_well) {
-      const int slot = well_slot(wc_cells, P.nwc, c);
-      if (slot >= 0) { qwc = wq[slot]; qgc = wq[P.nwc + slot]; }
+      slot = well_slot(A.wc_cells, P.nwc, c);
+      if (slot >= 0)                   // the cell's wells in configuration order
+        for (int q = A.wc_ptr[slot]; q < A.wc_ptr[slot + 1]; ++q) {
+          const WellTerms& t = A.terms[A.wc_wells[q]];
+          if (t.mask & 1) qwc += t.q[0];
+          if (t.mask & 2) qgc += t.q[1];
+        }
     }
     const double f = dt / pv[c];
     const double dSw = f * (qwc - dw);
@@ -759,6 +744,12 @@ __global__ void __launch_bounds__(kCells) k_saturation_flux(
     dsw_out[c] = dSw;
     dsg_out[c] = dSg;
     const double swc = sw[c], sgc = sg[c], eps = 1e-12;
+    if (slot >= 0) {
+      A.state[4 * slot] = swc;
+      A.state[4 * slot + 1] = sgc;
+      A.state[4 * slot + 2] = dSw;
+      A.state[4 * slot + 3] = dSg;
+    }
     const double sw_up = tclamp_min(1.0 - P.so_r - sgc - swc, 0.0);
     const double sw_dn = tclamp_min(swc - P.sw_cr, 0.0);
     const double sg_up = tclamp_min(1.0 - P.so_r - swc - sgc, 0.0);
@@ -815,40 +806,23 @@ __global__ void __launch_bounds__(kCells) k_saturation_flux(
   }
 }
 
-// Per-substep component balance of PVT runs (simulation.py:1396-1505): a thread
-// per (substep, well) replays the substeps at the well's cell, then four threads
-// add the terms in the reference's order.
-constexpr int kContribSmem = 3584;     // doubles of the terms kept in shared memory
-__host__ __device__ inline bool contrib_on_chip(const ModelParams& P) {
-  return 4ll * P.max_substeps * P.nwells <= kContribSmem;
-}
-__global__ void k_well_substeps(ModelParams P, const double* __restrict__ pvt_g,
-                                const WellDev* __restrict__ wells, const double* __restrict__ p_new,
-                                const double* __restrict__ sw, const double* __restrict__ sg,
-                                const double* __restrict__ dsw, const double* __restrict__ dsg,
-                                const int* __restrict__ nsub, double dt, double* contrib, double* bal,
-                                const int* pred) {
-  if (pred && *pred == 0) return;
-  extern __shared__ double s_contrib[];    // contrib on chip when it fits (kContribSmem)
-  if (contrib_on_chip(P)) contrib = s_contrib;
-  // contrib[(s * nwells + w) * 4 + q]: the addend of bal[6 + {0, 1, 3, 4}[q]] for
-  // substep s and well w (never negative), -1 where the reference adds nothing
-  __shared__ double s_col[kPvtCols * kMaxPvtRows];
-  __shared__ double s_slope[(kPvtCols - 1) * kMaxPvtRows];
-  PvtSmem T{P.pvt_rows, s_col, s_slope};
-  pvt_stage(pvt_g, P.pvt_rows, s_col, s_slope);
-  const int N = *nsub;
+// Per-substep component balance of PVT runs (simulation.py:1396-1505): item
+// s * nwells + w replays the substeps up to s at well w's cell.  contrib[4 item + q]:
+// the addend of bal[6 + {0, 1, 3, 4}[q]] (never negative), -1 where the reference
+// adds nothing.
+__device__ __noinline__ void well_replay(const ModelParams& P, const PvtSmem& T, const WellArgs& A, int it, int N,
+                                         const double* __restrict__ p_new, double dt, double* contrib) {
   const double dt_sub = dt / N;
   const double so_r = P.so_r;
-  const int items = N * P.nwells;
-  for (int it = threadIdx.x; it < items; it += blockDim.x) {
+  {
     const int s = it / P.nwells, w = it % P.nwells;
     double add[4] = {-1.0, -1.0, -1.0, -1.0};   // bal[6+0], bal[6+1], bal[6+3], bal[6+4]
-    const WellDev W = wells[w];
+    const WellDev W = A.wells[w];
     const int c = W.cell;
     if (c >= 0) {
-      double swc = sw[c], sgc = sg[c];
-      const double dws = dsw[c] / N, dgs = dsg[c] / N;
+      const double* w0 = A.state + 4 * well_slot(A.wc_cells, P.nwc, c);
+      double swc = w0[0], sgc = w0[1];
+      const double dws = w0[2] / N, dgs = w0[3] / N;
       for (int q = 0; q <= s; ++q) {   // the cell's state after substep s (as K4b)
         swc = swc + dws;
         sgc = sgc + dgs;
@@ -910,32 +884,17 @@ __global__ void k_well_substeps(ModelParams P, const double* __restrict__ pvt_g,
 #pragma unroll
     for (int q = 0; q < 4; ++q) contrib[(size_t)it * 4 + q] = add[q];
   }
-  __syncthreads();
-  // the reference's accumulation order: substeps outer, wells inner (simulation.py:1396-1505)
-  if (threadIdx.x < 4) {
-    const int q = threadIdx.x;
-    const int slot = q == 0 ? 0 : q == 1 ? 1 : q == 2 ? 3 : 4;
-    double acc = bal[6 + slot];
-    for (int i0 = 0; i0 < items; i0 += 8) {      // eight loads ahead of their additions
-      double v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = i0 + u < items ? contrib[(size_t)(i0 + u) * 4 + q] : -1.0;
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (!(v[u] < 0.0)) acc += v[u];   // NaN propagates as before
-    }
-    bal[6 + slot] = acc;
-  }
 }
 
 // K4b: N clamped substeps per cell, So, and the mass balance (simulation.py:1381-1527).
 constexpr int kSatBlock = 256;
-__global__ void __launch_bounds__(kSatBlock) k_saturation_substeps(
+__global__ void __launch_bounds__(kSatBlock, 4) k_saturation_substeps(
     ModelParams P, const double* __restrict__ pvt_g, const double* __restrict__ p_new,
     double* __restrict__ sw, double* __restrict__ sg, double* __restrict__ so,
     const double* __restrict__ dsw, const double* __restrict__ dsg, const double* __restrict__ pv,
-    const int* __restrict__ nsub, double* __restrict__ red, unsigned* __restrict__ counter,
-    double* __restrict__ bal, const int* pred) {
+    const int* __restrict__ nsub, double* __restrict__ red, unsigned* __restrict__ counter, WellArgs A,
+    double dt, double* contrib, const int* pred) {
+  double* bal = A.bal;
   if (pred && *pred == 0) return;
   __shared__ double s_col[kPvtCols * kMaxPvtRows];
   __shared__ double s_slope[(kPvtCols - 1) * kMaxPvtRows];
@@ -946,6 +905,12 @@ __global__ void __launch_bounds__(kSatBlock) k_saturation_substeps(
   const int N = *nsub;
   const double so_r = P.so_r;
   double acc[6] = {0, 0, 0, 0, 0, 0};  // water in/out, oil in/out, gas in/out
+  // the wells' replay items, a warp's first thread each, spread over the blocks
+  // (one block replaying them all was the kernel's critical path: 64 us against 42)
+  const int items = P.pvt_rows > 0 ? N * P.nwells : 0;
+  if ((threadIdx.x & 31) == 0)
+    for (int it = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; it < items; it += (kSatBlock / 32) * gridDim.x)
+      well_replay(P, T, A, it, N, p_new, dt, contrib);
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < P.N;
        c += (long long)gridDim.x * blockDim.x) {
     const double sw0 = sw[c], sg0 = sg[c];
@@ -978,8 +943,9 @@ __global__ void __launch_bounds__(kSatBlock) k_saturation_substeps(
     double v = block_sum<kSatBlock>(acc[q], s_w);
     if (threadIdx.x == 0) red[6 * blockIdx.x + q] = v;
   }
+  __threadfence();
+  __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
     unsigned done = atomicAdd(counter, 1u);
     s_last = (done == gridDim.x - 1);
   }
@@ -987,16 +953,40 @@ __global__ void __launch_bounds__(kSatBlock) k_saturation_substeps(
   if (s_last) {   // the whole last block sums the block partials (fixed order)
     __threadfence();
     double tot[6] = {0, 0, 0, 0, 0, 0};
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
       for (int q = 0; q < 6; ++q) tot[q] += ((volatile double*)red)[6 * b + q];
 #pragma unroll
     for (int q = 0; q < 6; ++q) tot[q] = block_sum<kSatBlock>(tot[q], s_w);
+    // component balance: the wells' terms in configuration order, then the
+    // replayed substeps' (warp q: oil in, oil out, gas in, gas out)
+    __shared__ double s_bal[4];
+    const int wq = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (wq < 4) {
+      double t = 0.0;
+      for (int it = lane; it < items; it += 32) {
+        const double v = __ldcg(contrib + 4 * (size_t)it + wq);
+        if (!(v < 0.0)) t += v;        // NaN propagates
+      }
+      t = warp_sum(t);
+      if (lane == 0) {
+        const int bit = wq == 0 ? 8 : wq == 1 ? 16 : wq == 2 ? 32 : 64;
+        double v = bal[6 + (wq < 2 ? wq : wq + 1)];
+        for (int w = 0; w < P.nwells; ++w)
+          if (A.terms[w].mask & bit) v += A.terms[w].b[wq];
+        s_bal[wq] = v + t;
+      }
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
       // mass_balance[water/oil/gas][in/out] (simulation.py:1521-1526)
       for (int q = 0; q < 6; ++q) bal[q] += tot[q];
       // component accum = in - out (simulation.py:1529-1530)
-      bal[6 + 2] = bal[6 + 0] - bal[6 + 1];
-      bal[6 + 5] = bal[6 + 3] - bal[6 + 4];
+      bal[6 + 0] = s_bal[0];
+      bal[6 + 1] = s_bal[1];
+      bal[6 + 2] = s_bal[0] - s_bal[1];
+      bal[6 + 3] = s_bal[2];
+      bal[6 + 4] = s_bal[3];
+      bal[6 + 5] = s_bal[2] - s_bal[3];
       *counter = 0u;
     }
   }
@@ -1004,10 +994,11 @@ __global__ void __launch_bounds__(kSatBlock) k_saturation_substeps(
 
 }  // namespace
 
-// blocks of the substep kernel: up to eight an SM, each with several cells a
-// thread, so that staging the PVT table and the block sums are paid once for them
-inline unsigned sat_grid(long long n) {
-  return (unsigned)std::max<long long>(1, std::min<long long>((n + kSatBlock - 1) / kSatBlock, (long long)num_sms() * 8));
+// Blocks of a kernel over cells: as many as fit on the SMs at once (per_sm by its
+// registers), each with several runs of cells, so that staging the PVT table and
+// the block sums are paid once for them and no partial wave is left.
+inline unsigned cell_grid(long long n, int per_sm) {
+  return (unsigned)std::max<long long>(1, std::min<long long>((n + kCells - 1) / kCells, (long long)num_sms() * per_sm));
 }
 
 // ---------------------------------------------------------------- host API
@@ -1028,7 +1019,7 @@ void model_build_static(Model& m, const double* kx, const double* ky, const doub
   m.col.alloc(m.nnz);
   k_pattern<<<grid_for(P.N + 1, 256), 256, 0, s>>>(P, m.nnz, m.rowptr.p, m.col.p); ::impes::count_launch();
   IMPES_CHECK_LAUNCH();
-  m.red_blocks = (int)sat_grid(P.N);
+  m.red_blocks = (int)cell_grid(P.N, 4);
   m.props.alloc((size_t)5 * P.N);
   m.red.alloc((size_t)6 * m.red_blocks + 16);
   m.counter.alloc(2);
@@ -1041,7 +1032,8 @@ void model_build_static(Model& m, const double* kx, const double* ky, const doub
     k_pvt_table<<<1, 256, 0, s>>>(P.pvt_rows, m.pvt.p, m.pvt_tab.p); ::impes::count_launch();
     IMPES_CHECK_LAUNCH();
   }
-  m.wq.alloc(std::max(1, 3 * P.nwc));
+  m.wterms.alloc(std::max<size_t>(1, (sizeof(WellTerms) / sizeof(double)) * P.nwells));
+  m.wstate.alloc(std::max(1, 4 * P.nwc));
   m.wsub.alloc(std::max<size_t>(1, (size_t)4 * std::max(P.max_substeps, 1) * std::max(P.nwells, 1)));
 }
 
@@ -1056,9 +1048,8 @@ void model_assemble(Model& m, const double* p, const double* sw, const double* s
   const int tid = timers().begin(IMPES_PH_ASSEMBLE, s);
   const size_t n = m.P.N;
   double *mt = m.props.p, *gs = mt + n, *mo = gs + n, *pc = mo + n, *acc = pc + n;
-  const unsigned g = sat_grid(m.P.N);
-  k_cell_props<<<g, kCells, 0, s>>>(m.P, m.pvt_tab.p, p, sw, sg, m.pv.p, dt, mt, gs, mo, pc, acc);
-  k_assemble<<<g, kCells, 0, s>>>(m.P, p, mt, gs, mo, pc, acc, m.tx.p, m.ty.p, m.tz.p, m.wells.p, m.wc_cells.p,
+  k_cell_props<<<cell_grid(n, 4), kCells, 0, s>>>(m.P, m.pvt_tab.p, p, sw, sg, m.pv.p, dt, mt, gs, mo, pc, acc);
+  k_assemble<<<cell_grid(n, 3), kCells, 0, s>>>(m.P, p, mt, gs, mo, pc, acc, m.tx.p, m.ty.p, m.tz.p, m.wells.p, m.wc_cells.p,
                                   m.wc_ptr.p, m.wc_wells.p, m.well_mode.p, csr_val, rhs);
   ::impes::count_launches(2);
   IMPES_CHECK_LAUNCH();
@@ -1069,29 +1060,19 @@ void model_saturation(Model& m, const double* p_new, double* sw, double* sg, dou
                       cudaStream_t s, const int* pred) {
   const ModelParams& P = m.P;
   const int tid = timers().begin(IMPES_PH_SATURATION, s);
-  if (P.nwells > 0) {
-    k_well_sources<<<1, kMaxWells, 0, s>>>(P, m.pvt_tab.p, m.wells.p, m.wc_cells.p, p_new, sw, sg, m.pv.p,
-                                     dt, m.wq.p, m.balances.p, m.well_q.p, m.well_rates.p, pred); ::impes::count_launch();
-    IMPES_CHECK_LAUNCH();
-  }
-  const unsigned g = sat_grid(P.N);
   const size_t n = P.N;
   double *mw = m.props.p, *mg = mw + n, *rw = mg + n, *rg = rw + n, *pcg = rg + n;
-  k_flux_props<<<g, kCells, 0, s>>>(P, m.pvt_tab.p, p_new, sw, sg, mw, mg, rw, rg, pcg, pred);
-  k_saturation_flux<<<g, kCells, 0, s>>>(P, p_new, mw, mg, rw, rg, pcg, sw, sg, m.tx.p, m.ty.p, m.tz.p, m.pv.p,
-                                         m.wc_cells.p, m.wq.p, dt, m.dsw.p, m.dsg.p, m.red.p, m.counter.p,
-                                         m.nsub.p, pred);
-  ::impes::count_launches(2);
-  IMPES_CHECK_LAUNCH();
-  if (P.pvt_rows > 0 && P.nwells > 0) {
-    const size_t smem = contrib_on_chip(P) ? sizeof(double) * 4 * P.max_substeps * P.nwells : 0;
-    k_well_substeps<<<1, 512, smem, s>>>(P, m.pvt_tab.p, m.wells.p, p_new, sw, sg, m.dsw.p, m.dsg.p,
-                                      m.nsub.p, dt, m.wsub.p, m.balances.p, pred); ::impes::count_launch();
-    IMPES_CHECK_LAUNCH();
-  }
-  k_saturation_substeps<<<g, kSatBlock, 0, s>>>(P, m.pvt_tab.p, p_new, sw, sg, so, m.dsw.p, m.dsg.p,
-                                                m.pv.p, m.nsub.p, m.red.p, m.counter.p + 1,
-                                                m.balances.p, pred); ::impes::count_launch();
+  const WellArgs A{m.wells.p, m.wc_cells.p, m.wc_ptr.p, m.wc_wells.p, reinterpret_cast<WellTerms*>(m.wterms.p),
+                   m.wstate.p, m.balances.p, m.well_q.p, m.well_rates.p};
+  k_flux_props<<<cell_grid(n, 4), kCells, 0, s>>>(P, m.pvt_tab.p, p_new, sw, sg, m.pv.p, dt, mw, mg, rw, rg, pcg, A,
+                                                  pred);
+  k_saturation_flux<<<cell_grid(n, 3), kCells, 0, s>>>(P, p_new, mw, mg, rw, rg, pcg, sw, sg, m.tx.p, m.ty.p, m.tz.p,
+                                                       m.pv.p, A, dt, m.dsw.p, m.dsg.p, m.red.p, m.counter.p,
+                                                       m.nsub.p, pred);
+  k_saturation_substeps<<<cell_grid(n, 4), kSatBlock, 0, s>>>(P, m.pvt_tab.p, p_new, sw, sg, so, m.dsw.p, m.dsg.p,
+                                                              m.pv.p, m.nsub.p, m.red.p, m.counter.p + 1, A, dt,
+                                                              m.wsub.p, pred);
+  ::impes::count_launches(3);
   IMPES_CHECK_LAUNCH();
   timers().end(tid, s, 8.0 * (6.0 * P.N + 0.5 * (double)(m.nnz - P.N)));
 }
