@@ -88,6 +88,37 @@ __device__ __forceinline__ T row_dot8(int a0, int e, int S, const T* __restrict_
   return row_dot(k, e, S, val, col, x, cb, acc);
 }
 
+// U entries k = a0, a0 + S, .. of a row: their values and columns, loaded
+// together (0 past the row's end).  The matrix does not change while a solve
+// runs, so the first batch of a kernel is loaded before griddepcontrol.wait: two
+// of the three dependent loads of a row (row pointer -> column -> x) overlap the
+// tail of the kernel before (pdl_wait_release says why that is safe).
+template <typename T, int U>
+struct RowBatch {
+  T v[U];
+  int c[U];
+};
+template <typename T, typename CT, int U>
+__device__ __forceinline__ void batch_load(RowBatch<T, U>& m, int k, int e, int S, const T* __restrict__ val,
+                                           const CT* __restrict__ col) {
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const bool in = k + u * S < e;
+    m.v[u] = in ? val[k + u * S] : T(0);
+    m.c[u] = in ? (int)col[k + u * S] : -1;
+  }
+}
+// acc + the batch's products in entry order, the gathers of x issued together
+template <typename T, int U, typename XT>
+__device__ __forceinline__ T batch_dot(const RowBatch<T, U>& m, int k, int e, int S, const XT* x, int cb, T acc) {
+  T xv[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) xv[u] = k + u * S < e ? (T)x[cb + m.c[u]] : T(0);
+#pragma unroll
+  for (int u = 0; u < U; ++u) acc += m.v[u] * xv[u];
+  return acc;
+}
+
 template <typename T, typename CT, int LPR, int MODE>
 __global__ void __launch_bounds__(TB) k_csr(int n, const int* __restrict__ rowptr,
                                             const CT* __restrict__ col, const T* __restrict__ val,
@@ -117,57 +148,135 @@ __global__ void __launch_bounds__(TB) k_csr(int n, const int* __restrict__ rowpt
   }
 }
 
+// k_csr for short rows: up to four lanes a row, and the handful of entries of a
+// prolongation row.  There a row is a chain of loads and gains from the early
+// batch: residual and sweep of a 539,534-row level 17.0 -> 13.3 us (fp32, one lane
+// a row), prolongations 10-20 %.  With eight lanes or more a row the warps
+// already cover the chain and the batch's predicated loads cost more than they
+// hide (14,473 rows of 37 entries, 16 lanes: 3.8 us plain, 4.4 us with it).
+// x, b and y carry no __restrict__ here: a load that the compiler takes for
+// invariant could be moved ahead of the wait.
+template <typename T, typename CT, int LPR, int MODE>
+__global__ void __launch_bounds__(TB) k_csr_early(int n, const int* __restrict__ rowptr,
+                                                  const CT* __restrict__ col, const T* __restrict__ val,
+                                                  const T* x, const T* b, const T* __restrict__ inv, T* y, int rel) {
+  const int lane = threadIdx.x % LPR;
+  constexpr int U = 4, RW = 32 / LPR;              // entries a batch, rows a warp
+  // whole warps take RW rows at a time, so that every lane reaches the shuffles
+  const long long warps = (long long)gridDim.x * (TB / 32);
+  long long base = ((long long)blockIdx.x * (TB / 32) + (threadIdx.x >> 5)) * RW;
+  int a = 0, e = 0;
+  RowBatch<T, U> m;
+  auto fetch = [&](long long row) {
+    a = e = 0;
+    if (MODE != Y_SMOOTH0 && row < n) {
+      a = rowptr[row];
+      e = rowptr[row + 1];
+    }
+    batch_load(m, a + lane, e, LPR, val, col);
+  };
+  long long row = base + (threadIdx.x & 31) / LPR;
+  fetch(row);
+  pdl_wait_release();
+  for (; base < n; base += warps * RW) {
+    row = base + (threadIdx.x & 31) / LPR;
+    T acc = T(0);
+    T bi = T(0), wi = T(0), xi = T(0);
+    const bool out = lane == 0 && row < n;
+    if (out) {
+      if (MODE == Y_B_MINUS_AX || MODE == Y_SMOOTH || MODE == Y_SMOOTH0) bi = b[row];
+      if (MODE == Y_SMOOTH || MODE == Y_SMOOTH0 || MODE == Y_W_AX) wi = inv[row];
+      if (MODE == Y_SMOOTH) xi = x[row];
+      if (MODE == Y_ADD_AX) xi = y[row];
+    }
+    if (MODE != Y_SMOOTH0) {
+      const int cb = col_base<CT>(row, rel);
+      acc = batch_dot(m, a + lane, e, LPR, x, cb, acc);
+      acc = row_dot8(a + lane + U * LPR, e, LPR, val, col, x, cb, acc);
+#pragma unroll
+      for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, LPR);
+    }
+    if (out) {
+      if (MODE == Y_AX) y[row] = acc;
+      else if (MODE == Y_B_MINUS_AX) y[row] = bi - acc;
+      else if (MODE == Y_SMOOTH) y[row] = xi + T(kOmega) * wi * (bi - acc);
+      else if (MODE == Y_ADD_AX) y[row] = xi + acc;
+      else if (MODE == Y_SMOOTH0) y[row] = T(kOmega) * wi * bi;
+      else if (MODE == Y_W_AX) y[row] = wi * acc;
+    }
+    fetch(base + warps * RW + (threadIdx.x & 31) / LPR);
+  }
+}
+
 // Wide rows (coarse Galerkin levels, hundreds to thousands of entries per row):
 // WPR warps per row, chosen by the mean row length.  Thread t of the row group
 // takes entries a+t, a+t+G, ... (G = 32*WPR), so each warp's value and column
 // loads are coalesced and its gathers of x hit adjacent columns.  CT and rel as
 // in k_csr (16-bit columns: 6 bytes per fp32 entry instead of 8).  With WPR > 1
 // the row's first warp adds the group's partial sums in a fixed order.  Same
-// epilogues as k_csr.
-template <typename T, typename CT, int MODE, int WPR>
-__global__ void __launch_bounds__(TB) k_csr_rows(int n, const int* __restrict__ rowptr,
-                                                 const CT* __restrict__ col, const T* __restrict__ val,
-                                                 const T* __restrict__ x, const T* __restrict__ b,
-                                                 const T* __restrict__ inv, T* __restrict__ y, int rel) {
-  pdl_wait_release();
+// epilogues as k_csr.  A level of a few thousand rows is one wave of warps, bound
+// by the chain row pointer -> column -> x of its longest rows: U entries a thread
+// are in flight at a time, the first of them (early batch, see k_csr_early) before
+// the wait.  fp64 levels of the 152,969-cell black-oil hierarchy, sweeps on
+// 11,246 rows of 276 entries 18.4 + 9.8 -> 12.1 + 9.0 us, 1,665 rows of 605
+// 10.3 + 5.3 -> 6.9 + 4.4 us; its whole V-cycle 491 -> 408 us.
+template <typename T, typename CT, int MODE, int WPR, int U>
+__global__ void __launch_bounds__(TB, U == 4 ? 8 / (sizeof(T) / 4) : 1)
+    k_csr_rows(int n, const int* __restrict__ rowptr, const CT* __restrict__ col, const T* __restrict__ val,
+               const T* x, const T* b, const T* __restrict__ inv, T* y, int rel) {
   constexpr int kWarps = TB / 32, kRows = kWarps / WPR, G = 32 * WPR;
   __shared__ T part[kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = warp / WPR, sub = warp % WPR;
   const int tid = sub * 32 + lane;
+  int a = 0, e = 0;
+  RowBatch<T, U> m;
+  auto fetch = [&](long long row) {
+    a = e = 0;
+    if (row < n) {
+      a = rowptr[row];
+      e = rowptr[row + 1];
+    }
+    batch_load(m, a + tid, e, G, val, col);
+  };
+  fetch((long long)blockIdx.x * kRows + grp);
+  pdl_wait_release();
   for (long long base = (long long)blockIdx.x * kRows; base < n; base += (long long)gridDim.x * kRows) {
     const long long row = base + grp;
-    T acc = T(0);
-    if (row < n) {
-      const int a = rowptr[row], e = rowptr[row + 1];
-      const int cb = col_base<CT>(row, rel);
-      acc = row_dot(a + tid, e, G, val, col, x, cb, acc);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    const bool out = sub == 0 && lane == 0 && row < n;
+    T bi = T(0), wi = T(0), xi = T(0);
+    if (out) {
+      if (MODE == Y_B_MINUS_AX || MODE == Y_SMOOTH) bi = b[row];
+      if (MODE == Y_SMOOTH || MODE == Y_W_AX) wi = inv[row];
+      if (MODE == Y_SMOOTH) xi = x[row];
+      if (MODE == Y_ADD_AX) xi = y[row];
     }
-    if (WPR == 1) {
-      if (lane == 0 && row < n) {
-        if (MODE == Y_AX) y[row] = acc;
-        else if (MODE == Y_B_MINUS_AX) y[row] = b[row] - acc;
-        else if (MODE == Y_SMOOTH) y[row] = x[row] + T(kOmega) * inv[row] * (b[row] - acc);
-        else if (MODE == Y_ADD_AX) y[row] = y[row] + acc;
-        else if (MODE == Y_W_AX) y[row] = inv[row] * acc;
+    const int cb = col_base<CT>(row, rel);
+    T acc = batch_dot(m, a + tid, e, G, x, cb, T(0));
+    for (int k = a + tid + U * G; k < e; k += U * G) {
+      batch_load(m, k, e, G, val, col);
+      acc = batch_dot(m, k, e, G, x, cb, acc);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (WPR > 1) {
+      if (lane == 0) part[warp] = acc;
+      __syncthreads();
+      if (out) {
+        acc = part[warp];
+#pragma unroll
+        for (int w = 1; w < WPR; ++w) acc += part[warp + w];
       }
-      continue;
     }
-    if (lane == 0) part[warp] = acc;
-    __syncthreads();
-    if (sub == 0 && lane == 0 && row < n) {
-      T t = part[warp];
-#pragma unroll
-      for (int w = 1; w < WPR; ++w) t += part[warp + w];
-      if (MODE == Y_AX) y[row] = t;
-      else if (MODE == Y_B_MINUS_AX) y[row] = b[row] - t;
-      else if (MODE == Y_SMOOTH) y[row] = x[row] + T(kOmega) * inv[row] * (b[row] - t);
-      else if (MODE == Y_ADD_AX) y[row] = y[row] + t;
-      else if (MODE == Y_W_AX) y[row] = inv[row] * t;
+    if (out) {
+      if (MODE == Y_AX) y[row] = acc;
+      else if (MODE == Y_B_MINUS_AX) y[row] = bi - acc;
+      else if (MODE == Y_SMOOTH) y[row] = xi + T(kOmega) * wi * (bi - acc);
+      else if (MODE == Y_ADD_AX) y[row] = xi + acc;
+      else if (MODE == Y_W_AX) y[row] = wi * acc;
     }
-    __syncthreads();
+    if (WPR > 1) __syncthreads();
+    fetch(base + (long long)gridDim.x * kRows + grp);
   }
 }
 
@@ -281,26 +390,45 @@ void launch_wide(int n, int avg, const int* rowptr, const CT* col, const T* val,
       return;
     }
   }
+  auto rows = [&](auto wpr, auto deep, int g) {
+    launch_pdl(k_csr_rows<T, CT, MODE, decltype(wpr)::value, decltype(deep)::value>, grid(g), TB, 0, s, n, rowptr, col,
+               val, x, b, inv, y, rel);
+  };
+  using std::integral_constant;
+  const integral_constant<int, 4> four;
+  const integral_constant<int, 8> eight;
   if (avg <= 512) {
-    launch_pdl(k_csr_rows<T, CT, MODE, 1>, grid(8), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel);
+    // eight entries in flight where a lane has that many, or where the level is at
+    // most one wave of warps; else four, which leaves registers for every warp an
+    // SM can hold (21,022 fp64 rows of 143 entries: 9.9 + 9.8 us at four, 11.0 +
+    // 9.5 at eight; 2,668 rows of 595 and less: eight is the faster throughout)
+    const bool deep = avg > 256 || n <= num_sms() * 64;
+    if (deep) rows(integral_constant<int, 1>{}, eight, 8);
+    else rows(integral_constant<int, 1>{}, four, 8);
   } else if (avg <= 1536) {
-    launch_pdl(k_csr_rows<T, CT, MODE, 2>, grid(4), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel);
+    rows(integral_constant<int, 2>{}, eight, 4);
   } else {
-    launch_pdl(k_csr_rows<T, CT, MODE, 4>, grid(2), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel);
+    rows(integral_constant<int, 4>{}, eight, 2);
   }
 }
 
+// the row kernel for eight lanes or more
+template <typename T, typename CT, int LPR, int MODE>
+constexpr auto csr_lanes() {
+  if constexpr (MODE == Y_ADD_AX) return k_csr_early<T, CT, LPR, MODE>;
+  else return k_csr<T, CT, LPR, MODE>;
+}
 template <typename T, typename CT, int MODE>
 void launch_lanes(int lpr, int n, const int* rowptr, const CT* col, const T* val, const T* x,
                   const T* b, const T* inv, T* y, int rel, cudaStream_t s) {
   auto grid = [&](int l) { return grid_for(((size_t)n * l + TB - 1) / TB * TB, TB, 16); };
   switch (lpr) {
-    case 1: launch_pdl(k_csr<T, CT, 1, MODE>, grid(1), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
-    case 2: launch_pdl(k_csr<T, CT, 2, MODE>, grid(2), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
-    case 4: launch_pdl(k_csr<T, CT, 4, MODE>, grid(4), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
-    case 8: launch_pdl(k_csr<T, CT, 8, MODE>, grid(8), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
-    case 16: launch_pdl(k_csr<T, CT, 16, MODE>, grid(16), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
-    default: launch_pdl(k_csr<T, CT, 32, MODE>, grid(32), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
+    case 1: launch_pdl(k_csr_early<T, CT, 1, MODE>, grid(1), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
+    case 2: launch_pdl(k_csr_early<T, CT, 2, MODE>, grid(2), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
+    case 4: launch_pdl(k_csr_early<T, CT, 4, MODE>, grid(4), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
+    case 8: launch_pdl(csr_lanes<T, CT, 8, MODE>(), grid(8), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
+    case 16: launch_pdl(csr_lanes<T, CT, 16, MODE>(), grid(16), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
+    default: launch_pdl(csr_lanes<T, CT, 32, MODE>(), grid(32), TB, 0, s, n, rowptr, col, val, x, b, inv, y, rel); break;
   }
 }
 
@@ -352,16 +480,54 @@ __global__ void __launch_bounds__(TB) k_restrict_s0(int nc, const int* __restric
   }
 }
 
+// the same with the early batch, for up to eight lanes a row (see k_csr_early):
+// 330,000 -> 177,868 rows 4.4 -> 3.7 us, 1,000,000 -> 539,534 rows 9.5 -> 7.9 us (fp32)
+template <typename T, int LPR>
+__global__ void __launch_bounds__(TB) k_restrict_s0_early(int nc, const int* __restrict__ rowptr,
+                                                    const int* __restrict__ col, const T* __restrict__ val,
+                                                    const T* r, const T* __restrict__ inv_c, T* bc, T* xc) {
+  constexpr int U = 4, RW = 32 / LPR;
+  const int lane = threadIdx.x % LPR;
+  const long long warps = (long long)gridDim.x * (TB / 32);
+  long long base = ((long long)blockIdx.x * (TB / 32) + (threadIdx.x >> 5)) * RW;
+  int a = 0, e = 0;
+  T wi = T(0);
+  RowBatch<T, U> m;
+  auto fetch = [&](long long row) {
+    a = e = 0;
+    if (row < nc) {
+      a = rowptr[row];
+      e = rowptr[row + 1];
+      if (lane == 0) wi = inv_c[row];
+    }
+    batch_load(m, a + lane, e, LPR, val, col);
+  };
+  fetch(base + (threadIdx.x & 31) / LPR);
+  pdl_wait_release();
+  for (; base < nc; base += warps * RW) {
+    const long long row = base + (threadIdx.x & 31) / LPR;
+    T acc = batch_dot(m, a + lane, e, LPR, r, 0, T(0));
+    acc = row_dot8(a + lane + U * LPR, e, LPR, val, col, r, 0, acc);
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, LPR);
+    if (lane == 0 && row < nc) {
+      bc[row] = acc;
+      xc[row] = T(kOmega) * wi * acc;
+    }
+    fetch(base + warps * RW + (threadIdx.x & 31) / LPR);
+  }
+}
+
 template <typename T>
 void launch_restrict_s0(const Level& L, int lpr, const T* rval, const T* r, const T* inv_c, T* bc, T* xc,
                         cudaStream_t s) {
   const int n = L.nc;
   auto grid = [&](int l) { return grid_for(((size_t)n * l + TB - 1) / TB * TB, TB, 16); };
   switch (lpr) {
-    case 1: launch_pdl(k_restrict_s0<T, 1>, grid(1), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
-    case 2: launch_pdl(k_restrict_s0<T, 2>, grid(2), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
-    case 4: launch_pdl(k_restrict_s0<T, 4>, grid(4), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
-    case 8: launch_pdl(k_restrict_s0<T, 8>, grid(8), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
+    case 1: launch_pdl(k_restrict_s0_early<T, 1>, grid(1), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
+    case 2: launch_pdl(k_restrict_s0_early<T, 2>, grid(2), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
+    case 4: launch_pdl(k_restrict_s0_early<T, 4>, grid(4), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
+    case 8: launch_pdl(k_restrict_s0_early<T, 8>, grid(8), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
     case 16: launch_pdl(k_restrict_s0<T, 16>, grid(16), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
     default: launch_pdl(k_restrict_s0<T, 32>, grid(32), TB, 0, s, n, (const int*)L.rrow.p, (const int*)L.rcol.p, rval, r, inv_c, bc, xc); break;
   }

@@ -1937,6 +1937,7 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
     sell_refresh(h, 0, s, true);
     if (h.prm.mixed_precision) sell_refresh(h, 1, s, true);
   }
+  pdl_fence(s);
   amg_autotune(h, s);
   // the SELL copies the tuner did not pick are dropped
   for (auto& L : h.levels) {
@@ -2013,6 +2014,7 @@ void update_fp32_chain(AMG& h, cudaStream_t s) {
   }
   coarse_factor(h, *h.levels.back(), s, true);
   sell_refresh(h, 1, s, false, true);
+  pdl_fence(s);
   h.fp64_stale = true;
 }
 
@@ -2026,6 +2028,7 @@ void amg_ensure_fp64(AMG& h, cudaStream_t s) {
   }
   coarse_factor(h, *h.levels.back(), s);
   sell_refresh(h, 0, s);
+  pdl_fence(s);
   h.fp64_stale = false;
 }
 
@@ -2065,6 +2068,7 @@ void amg_update(AMG& h, const double* val, cudaStream_t s) {
   IMPES_CHECK_LAUNCH();
   sell_refresh(h, 0, s);
   if (h.prm.mixed_precision) sell_refresh(h, 1, s);
+  pdl_fence(s);
   timers().end(tid, s, bytes);
 }
 

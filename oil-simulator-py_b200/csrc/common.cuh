@@ -180,13 +180,20 @@ inline unsigned grid_for(size_t n, int block, int max_per_sm = 8) {
 // without the programmatic attribute), then launch_dependents lets the next
 // kernel of the stream launch at once, so its blocks are scheduled while this
 // grid runs and wait on the device instead of after a launch gap.  Only kernels
-// that begin with this call may be launched through launch_pdl.
+// that begin with this call may be launched through launch_pdl.  The one thing a
+// kernel may do ahead of it is to read the hierarchy (row pointers, columns,
+// values, inverse diagonals): the setup kernels that write it are followed by
+// pdl_fence, so they have completed before any kernel of a chain starts.
 __device__ __forceinline__ void pdl_wait_release() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 // false when the environment sets IMPES_NO_PDL=1 (plain stream order)
 bool pdl_enabled();
+// An empty grid in plain stream order: it starts when everything before it has
+// completed and is visible, so whatever is launched behind it, programmatically
+// or not, sees those writes from its first instruction on.
+void pdl_fence(cudaStream_t s);
 template <typename... P, typename... A>
 void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg = {};
