@@ -148,7 +148,7 @@ bool step_graph_run(Model& m, AMG& a, double* p, double* sw, double* sg, double*
     try {
       model_assemble(m, p, sw, sg, dt, m.csr_val.p, m.rhs.p, cs);
       stage = "AMG update";
-      amg_update(a, m.csr_val.p, cs);
+      amg_update(a, m.csr_val.p, cs, true);
       stage = "FGMRES";
       IMPES_CUDA(cudaMemcpyAsync(m.p_save.p, p, sizeof(double) * m.P.N, cudaMemcpyDeviceToDevice, cs));
       if (quad) {

@@ -167,11 +167,16 @@ struct AMG {
   bool use_dia_tile = false;            // level-0 grid-tile sweeps (IMPES_DIA_TILE=1: on)
   // The V-cycle of levels dense_level and below as one dense operator (row-major,
   // leading dimension dense_ld), per [fp32 values][Krylov mode]; valid while the
-  // values it was formed from are the hierarchy's (amg_dense.cu)
+  // values it was formed from are the hierarchy's (amg_dense.cu).  The flags are the
+  // host's: they stand for kernels in stream order, so nothing recorded into a
+  // graph of the caller's may set or rely on them.  V-cycles recorded there run
+  // level by level (dense_off), and an update recorded there forms the operators
+  // behind its values.
   int dense_level = -1;                 // -1: none
   int dense_ld = 0;
   DBuf<double> dense_op[2][2], dense_work;
   bool dense_valid[2][2] = {{false, false}, {false, false}};
+  bool dense_off = false;
   void dense_invalidate() { for (auto& a : dense_valid) a[0] = a[1] = false; }
   int tail_level = -1;                  // first level of the fused tail, -1: none
   int tail_cluster = 0;                 // CTAs in the tail's cluster (16 or 8)
@@ -202,7 +207,9 @@ struct AMG {
 // amg_setup.cu
 void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const double* val,
                cudaStream_t s);
-void amg_update(AMG& h, const double* val, cudaStream_t s);
+// own_graph: s records the handle's own whole-step graph, which forms the coarse
+// operator it needs itself.
+void amg_update(AMG& h, const double* val, cudaStream_t s, bool own_graph = false);
 // amg_dense.cu: inverses of the coarsest matrix (n <= 500), pinned and unpinned
 void coarse_factor(AMG& h, Level& L, cudaStream_t s, bool from_fp32 = false);
 // The coarse V-cycle's dense operator: which levels (after the tails were chosen),

@@ -1720,7 +1720,7 @@ T* vcycle(AMG& h, int l, bool zero_x, cudaStream_t s, bool first_sweep_done = fa
       return LV<T>::x(L);
     }
   }
-  if (l > 0 && zero_x && l == h.dense_level) {
+  if (l > 0 && zero_x && l == h.dense_level && !h.dense_off) {
     dense_apply<T>(h, h.krylov_mode, LV<T>::b(L), LV<T>::x(L), s);
     return LV<T>::x(L);
   }
@@ -1770,7 +1770,8 @@ T* vcycle(AMG& h, int l, bool zero_x, cudaStream_t s, bool first_sweep_done = fa
   if (!tiled) launch_a<T, Y_B_MINUS_AX>(L, LV<T>::slot, x, LV<T>::b(L), nullptr, LV<T>::r(L), s);
   // the restriction also takes the coarse level's first sweep from zero when
   // that level smooths with l1-Jacobi through the per-level kernels
-  const bool fuse_s0 = !Nc.coarsest && L.r_avg <= 96 && !(l + 1 == h.tail_level) && l + 1 != h.dense_level &&
+  const bool fuse_s0 = !Nc.coarsest && L.r_avg <= 96 && !(l + 1 == h.tail_level) &&
+                       (l + 1 != h.dense_level || h.dense_off) &&
                        !(sizeof(T) == 4 && l + 1 == h.stail_level) &&
                        !(h.prm.smoother == IMPES_SMOOTHER_CHEBYSHEV && Nc.cheb_lmax.p);
   if (fuse_s0) {
@@ -1805,6 +1806,14 @@ void dense_ensure(AMG& h, cudaStream_t s) {
 // LV<T>::x(L0) unless zero_x), replayed from a CUDA graph captured on first use.
 template <typename T>
 T* vcycle_top(AMG& h, bool zero_x, cudaStream_t s) {
+  if (stream_capturing(s)) {       // a graph of the caller's: replayed on whatever values are the levels' then
+    struct Off {
+      AMG& h;
+      explicit Off(AMG& a) : h(a) { h.dense_off = true; }
+      ~Off() { h.dense_off = false; }
+    } off(h);
+    return vcycle<T>(h, 0, zero_x, s);
+  }
   dense_ensure<T>(h, s);
   if (!h.use_graphs) return vcycle<T>(h, 0, zero_x, s);
   PhaseTimers& tm = timers();
@@ -3114,7 +3123,7 @@ void amg_fgmres(AMG& h, const double* b, double* x, const impes_krylov_params& k
   } solve_timer{s, timers().begin(IMPES_PH_SOLVE, s)};
   amg_fgmres_prepare(h, kp);
   AMG::FgGraph* g = nullptr;
-  if (h.use_graphs && h.use_step_graph && !h.fg_graph_failed && !timers().on) {
+  if (h.use_graphs && h.use_step_graph && !h.fg_graph_failed && !timers().on && !stream_capturing(s)) {
     g = fg_graph(h, kp);
     h.fg_graph_failed = g == nullptr;
   }

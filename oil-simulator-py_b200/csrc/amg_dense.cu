@@ -634,7 +634,7 @@ void amg_dense_form(AMG& h, int slot, bool krylov, cudaStream_t s) {
   if (h.dense_level < 0) return;
   if (slot == 0) dense_form<double>(h, krylov ? 1 : 0, s);
   else dense_form<float>(h, krylov ? 1 : 0, s);
-  h.dense_valid[slot][krylov ? 1 : 0] = true;
+  if (!stream_capturing(s)) h.dense_valid[slot][krylov ? 1 : 0] = true;
 }
 
 template <typename T>

@@ -2029,10 +2029,20 @@ void amg_ensure_fp64(AMG& h, cudaStream_t s) {
   coarse_factor(h, *h.levels.back(), s);
   sell_refresh(h, 0, s);
   pdl_fence(s);
+  if (stream_capturing(s)) return;       // recorded, not run
+  h.dense_valid[0][0] = h.dense_valid[0][1] = false;
   h.fp64_stale = false;
 }
 
-void amg_update(AMG& h, const double* val, cudaStream_t s) {
+namespace {
+// The operators of these values, behind an update that a caller records: its
+// replays change the values without the host's knowledge.
+void dense_form_recorded(AMG& h, int slot, cudaStream_t s) {
+  for (int krylov = 0; krylov < 2; ++krylov) amg_dense_form(h, slot, krylov != 0, s);
+}
+}  // namespace
+
+void amg_update(AMG& h, const double* val, cudaStream_t s, bool own_graph) {
   IMPES_REQUIRE(h.built, IMPES_ERR_STATE, "update before setup");
   const int tid = timers().begin(IMPES_PH_GALERKIN, s);
   double bytes = 0.0;
@@ -2042,10 +2052,12 @@ void amg_update(AMG& h, const double* val, cudaStream_t s) {
     bytes += 12.0 * L.nnz + 24.0 * L.pnnz + 8.0 * h.levels[l + 1]->nnz;
     if (!L.coarsest && !L.planned) all_planned = false;
   }
-  h.dense_invalidate();
+  const bool recorded = !own_graph && stream_capturing(s);
+  if (!recorded) h.dense_invalidate();
   equilibrate_level0(h, val, s);
   if (h.prm.mixed_precision && all_planned && h.levels.size() > 1) {
     update_fp32_chain(h, s);
+    if (recorded) dense_form_recorded(h, 1, s);
     timers().end(tid, s, bytes * 0.6);   // 4-byte values instead of 8
     return;
   }
@@ -2069,6 +2081,8 @@ void amg_update(AMG& h, const double* val, cudaStream_t s) {
   sell_refresh(h, 0, s);
   if (h.prm.mixed_precision) sell_refresh(h, 1, s);
   pdl_fence(s);
+  if (recorded) dense_form_recorded(h, 0, s);
+  if (recorded && h.prm.mixed_precision) dense_form_recorded(h, 1, s);
   timers().end(tid, s, bytes);
 }
 

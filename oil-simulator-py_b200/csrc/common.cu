@@ -108,6 +108,15 @@ void Arena::trim() {
 
 const char* last_error_cstr() { return g_last_error.c_str(); }
 
+bool stream_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 bool pdl_enabled() {
   static const bool on = [] {
     const char* ev = getenv("IMPES_NO_PDL");

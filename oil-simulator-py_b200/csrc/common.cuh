@@ -188,6 +188,9 @@ __device__ __forceinline__ void pdl_wait_release() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
+// Whether s records into a graph: what is launched then has not run when the call
+// returns, and may run any number of times later.
+bool stream_capturing(cudaStream_t s);
 // false when the environment sets IMPES_NO_PDL=1 (plain stream order)
 bool pdl_enabled();
 // An empty grid in plain stream order: it starts when everything before it has
