@@ -835,12 +835,7 @@ bool dia_tile_ok(const AMG& h, const Level& L, int slot) {
 template <typename T, bool RES>
 void launch_dia_tile(const Level& L, const T* x0, const T* b, const T* inv, T* xout, T* r, cudaStream_t s) {
   const size_t smem = dia_tile_smem<T, RES>(L);
-  // raise the dynamic shared-memory limit once per instantiation (thread-safe
-  // initialisation: ensemble workers launch concurrently)
-  static const cudaError_t attr = cudaFuncSetAttribute((const void*)k_dia_tile<T, RES>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)kTileSmemMax);
-  IMPES_CUDA(attr);
+  raise_smem_limit((const void*)k_dia_tile<T, RES>, kTileSmemMax);
   DiaGrid g{L.grid_nx, L.grid_ny, L.grid_nz, (L.grid_ny + kTileY - 1) / kTileY, kTileThreads / L.grid_nz};
   const int tiles = ((L.grid_nx + kTileX - 1) / kTileX) * g.tiles_y;
   launch_pdl(k_dia_tile<T, RES>, tiles, kTileThreads, smem, s, g, dia_values<T>(L), x0, b, inv, xout, r);

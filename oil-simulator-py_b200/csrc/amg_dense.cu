@@ -199,11 +199,7 @@ void launch_gj(int n, const GJArgs& args, cudaStream_t s) {
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = CL > 1 ? 1 : 0;
-  if (CL > 8) {
-    static const cudaError_t np =
-        cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    IMPES_CUDA(np);
-  }
+  if (CL > 8) allow_wide_cluster((const void*)kern);
   IMPES_CUDA(cudaLaunchKernelEx(&cfg, kern, n, args));
   count_launch();
 }

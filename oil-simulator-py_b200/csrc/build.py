@@ -33,7 +33,7 @@ SOURCES = {
     "pcg.cu": [],
     "abi.cu": [],
 }
-HEADERS = ["common.cuh", "model.cuh", "amg.cuh", os.path.join(REPO, "include", "impes_b200.h")]
+HEADERS = ["common.cuh", "device_limits.h", "model.cuh", "amg.cuh", os.path.join(REPO, "include", "impes_b200.h")]
 
 
 def _mtime(p):

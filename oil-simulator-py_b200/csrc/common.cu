@@ -1,5 +1,6 @@
 // Shared host utilities: thread-local error text and a device exclusive scan.
 #include "common.cuh"
+#include "device_limits.h"
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
@@ -26,15 +27,36 @@ void count_launches(long long n) {
 unsigned long long launches() { return g_launches.load(std::memory_order_relaxed); }
 unsigned long long thread_launches() { return t_launches; }
 
+namespace {
+int current_device() {
+  int dev = 0;
+  IMPES_CUDA(cudaGetDevice(&dev));
+  return dev;
+}
+}  // namespace
 void raise_smem_limit(const void* kernel, size_t bytes) {
-  static std::mutex mu;
-  static std::map<const void*, size_t> current;
-  std::lock_guard<std::mutex> lock(mu);
-  size_t& c = current[kernel];
-  if (bytes > c) {
-    IMPES_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    c = bytes;
+  static DeviceLimits limits;
+  limits.raise(current_device(), kernel, bytes, [&](size_t v) {
+    IMPES_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v));
+  });
+}
+void allow_wide_cluster(const void* kernel) {
+  static DeviceLimits limits;
+  limits.raise(current_device(), kernel, 1, [&](size_t) {
+    IMPES_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  });
+}
+int num_sms() {
+  constexpr int kDevices = 128;
+  static std::atomic<int> sms[kDevices];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) dev = 0;
+  int n = sms[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    sms[dev].store(n, std::memory_order_relaxed);
   }
+  return n;
 }
 namespace {
 thread_local Arena* t_arena = nullptr;

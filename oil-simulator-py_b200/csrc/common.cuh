@@ -28,10 +28,11 @@ void count_launch();
 void count_launches(long long n);
 unsigned long long launches();
 unsigned long long thread_launches();   // launches issued by the calling host thread
-// Raise a kernel's dynamic shared-memory limit to at least `bytes`; never
-// lowers it, so host threads launching the same kernel with different sizes
-// do not undo each other's setting.
+// Raise a kernel's dynamic shared-memory limit on the current device to at least
+// `bytes`; never lowers it.
 void raise_smem_limit(const void* kernel, size_t bytes);
+// Lets a kernel launch in clusters of more than eight CTAs on the current device.
+void allow_wide_cluster(const void* kernel);
 
 #define IMPES_CUDA(call)                                                        \
   do {                                                                          \
@@ -155,16 +156,7 @@ struct HostPinned {
   HostPinned& operator=(const HostPinned&) = delete;
 };
 
-inline int num_sms() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  return sms;
-}
+int num_sms();                         // of the current device
 
 inline unsigned grid_for(size_t n, int block, int max_per_sm = 8) {
   size_t g = (n + block - 1) / block;
