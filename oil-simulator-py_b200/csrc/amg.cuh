@@ -179,6 +179,7 @@ struct AMG {
   bool dense_off = false;
   void dense_invalidate() { for (auto& a : dense_valid) a[0] = a[1] = false; }
   int tail_level = -1;                  // first level of the fused tail, -1: none
+  int coarse_cluster = 16;              // CTAs that invert a coarsest matrix of more than 256 rows
   int tail_cluster = 0;                 // CTAs in the tail's cluster (16 or 8)
   int stail_level = -1;                 // first level of the shared-memory fp32 tail, -1: none
   size_t stail_smem = 0;                // its shared-memory bytes
@@ -210,7 +211,9 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
 // own_graph: s records the handle's own whole-step graph, which forms the coarse
 // operator it needs itself.
 void amg_update(AMG& h, const double* val, cudaStream_t s, bool own_graph = false);
-// amg_dense.cu: inverses of the coarsest matrix (n <= 500), pinned and unpinned
+// amg_dense.cu: inverses of the coarsest matrix (n <= 500), pinned and unpinned;
+// the CTAs of a cluster that may invert one of more than 256 rows (16, else 8)
+int coarse_cluster_size();
 void coarse_factor(AMG& h, Level& L, cudaStream_t s, bool from_fp32 = false);
 // The coarse V-cycle's dense operator: which levels (after the tails were chosen),
 // forming it from the current values, and x = Op b on level h.dense_level.

@@ -5,6 +5,7 @@
 //   _v_cycle :1037-1106 (coarsest solve with DOF 0 pinned :1045-1069).
 #include "amg.cuh"
 #include <algorithm>
+#include <cstdlib>
 #include <cooperative_groups.h>
 
 namespace cg = cooperative_groups;
@@ -206,6 +207,29 @@ void launch_gj(int n, const GJArgs& args, cudaStream_t s) {
 
 }  // namespace
 
+// Sixteen CTAs need that many free SMs in one GPC, which a part of a GPU may not
+// have; IMPES_COARSE_CLUSTER=8 asks for the narrow form (read at setup).
+int coarse_cluster_size() {
+  const char* ev = getenv("IMPES_COARSE_CLUSTER");
+  if (ev && atoi(ev) == 8) return 8;
+  auto* kern = k_gauss_jordan<16, 1, 32, 16>;
+  allow_wide_cluster((const void*)kern);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * 16);
+  cfg.blockDim = dim3(1024);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 16;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters >= 1) return 16;
+  cudaGetLastError();
+  return 8;
+}
+
 void coarse_factor(AMG& h, Level& L, cudaStream_t s, bool from_fp32) {
   if (L.n > 500 || L.n == 0) return;
   const int n = L.n;
@@ -230,7 +254,8 @@ void coarse_factor(AMG& h, Level& L, cudaStream_t s, bool from_fp32) {
   else if (n <= 96) launch_gj<1, 3, 8, 12>(n, args, s);
   else if (n <= 128) launch_gj<1, 4, 8, 16>(n, args, s);
   else if (n <= 256) launch_gj<8, 1, 32, 8>(n, args, s);
-  else launch_gj<16, 1, 32, 16>(n, args, s);
+  else if (h.coarse_cluster == 16) launch_gj<16, 1, 32, 16>(n, args, s);
+  else launch_gj<8, 2, 16, 32>(n, args, s);
   IMPES_CHECK_LAUNCH();
 }
 

@@ -1681,6 +1681,7 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
     const char* eg = getenv("IMPES_DIA_TILE");
     h.use_dia_tile = eg && eg[0] == '1';
   }
+  h.coarse_cluster = coarse_cluster_size();
   h.levels.clear();
   h.dense_level = -1;
   h.dense_invalidate();
