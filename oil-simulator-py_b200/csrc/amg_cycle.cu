@@ -2363,9 +2363,9 @@ __global__ void k_fg_init(FgState* st, const double* part_b, const double* part_
   t.beta = sqrt(r2);
   t.rel = t.bnorm > 0.0 ? t.beta / t.bnorm : 0.0;
   t.true_rel = t.rel;
-  t.bzero = !(t.bnorm > 0.0);
   t.nan = !(t.beta == t.beta) || !(t.bnorm == t.bnorm);
-  t.converged = t.bzero || t.rel < t.tol;
+  t.bzero = !t.nan && !(t.bnorm > 0.0);
+  t.converged = !t.nan && (t.bzero || t.rel < t.tol);
   t.done = t.bzero || t.nan || t.rel < t.tol || t.max_iters <= 0;
   *st = t;
   g[0] = t.beta;
@@ -2786,8 +2786,10 @@ __global__ void k_fg_restart(const double* partial, int nb, FgState* st, double*
   }
   outer.set(st->done ? 0u : 1u);
 }
+// x stays the caller's when the solve met a NaN
 __global__ void k_fg_final(long long n, const double* dhalf, const double* xs, double* x, const FgState* st) {
   pdl_wait_release();
+  if (st->nan) return;
   const bool zero = st->bzero;
   GRID_LOOP(i, n) x[i] = zero ? 0.0 : dhalf[i] * xs[i];
 }
@@ -2946,7 +2948,7 @@ void fg_prologue(AMG& h, const double* b, const double* x, const impes_krylov_pa
     launch_pdl(k_zero, gn, TB, 0, s, n, h.kx.p);
   launch_pdl(k_fg_params, 1, 1, 0, s, h.fgst.p, kp.tol, kp.max_iters);
 }
-// after them: x = D^-1/2 x_s (zero for a zero right-hand side)
+// after them: x = D^-1/2 x_s (zero for a zero right-hand side, x as it was after a NaN)
 void fg_epilogue(AMG& h, double* x, cudaStream_t s) {
   const long long n = h.levels[0]->n;
   launch_pdl(k_fg_final, grid_for(n, TB), TB, 0, s, n, (const double*)h.dhalf_inv.p, (const double*)h.kx.p, x,
