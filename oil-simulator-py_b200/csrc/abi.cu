@@ -485,6 +485,7 @@ int impes_model_create(impes_model** out, const impes_model_desc* d, const impes
         IMPES_CUDA(cudaMemcpyAsync(m.wc_wells.p, wc_wells.data(), sizeof(int) * nwells, cudaMemcpyHostToDevice, s));
       }
       IMPES_CUDA(cudaMemcpyAsync(m.wc_ptr.p, wc_ptr.data(), sizeof(int) * (P.nwc + 1), cudaMemcpyHostToDevice, s));
+      P.pvt_finite = d->pvt_rows > 0 && pvt_densities_finite(P, pvt) ? 1 : 0;
       m.pvt.alloc(std::max(1, d->pvt_rows * 9));
       if (d->pvt_rows)
         IMPES_CUDA(cudaMemcpyAsync(m.pvt.p, pvt, sizeof(double) * d->pvt_rows * 9, cudaMemcpyHostToDevice, s));

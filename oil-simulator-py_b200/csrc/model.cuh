@@ -23,6 +23,7 @@ struct ModelParams {
   int pvt_rows;
   int nwells;       // wells
   int nwc;          // distinct well cells
+  int pvt_finite;   // the table gives a finite density of every phase at any finite pressure
 };
 
 // Device-side well record (same fields as impes_well_desc + derived).
@@ -85,6 +86,9 @@ void model_assemble(Model& m, const double* p, const double* sw, const double* s
 // pred (device int, may be null): the kernels do nothing unless *pred != 0
 void model_saturation(Model& m, const double* p_new, double* sw, double* sg, double* so,
                       double dt, cudaStream_t s, const int* pred = nullptr);
+
+// Whether a PVT table (host, rows x 9) yields finite densities at every finite pressure.
+bool pvt_densities_finite(const ModelParams& P, const double* pvt);
 
 // Closed-form CSR row pointer of the 7-point pattern (no scan needed) of cell
 // c = (i ny + j) nz + k: the entries of the rows before it, direction by direction.

@@ -929,7 +929,8 @@ __global__ void __launch_bounds__(kSatBlock, 4) k_saturation_substeps(
     so[c] = 1.0 - swc - sgc;
     const double dwe = swc - sw0, dge = sgc - sg0;
     const double p = p_new[c], pvc = pv[c];
-    if (dwe == 0.0 && dge == 0.0 && isfinite(p) && isfinite(pvc)) continue;   // no mass moves
+    // no mass moves; where a density may be NaN or infinite, zero times it is NaN
+    if (dwe == 0.0 && dge == 0.0 && P.pvt_finite && isfinite(p) && isfinite(pvc)) continue;
     Rho r = densities(P, T, p, pvt_at(P, T, p));
     const double mw = dwe * pvc * r.w;
     const double mg = dge * pvc * r.g;
@@ -999,6 +1000,25 @@ __global__ void __launch_bounds__(kSatBlock, 4) k_saturation_substeps(
 // the block sums are paid once for them and no partial wave is left.
 inline unsigned cell_grid(long long n, int per_sm) {
   return (unsigned)std::max<long long>(1, std::min<long long>((n + kCells - 1) / kCells, (long long)num_sms() * per_sm));
+}
+
+// Formation volume factors that are nowhere negative (so that the 1e-12 of the
+// divisors stands above an interpolation's rounding), numbers and slopes that are
+// finite and far from overflow, pressures in ascending order.
+bool pvt_densities_finite(const ModelParams& P, const double* pvt) {
+  const double top = 1e140;             // products and quotients by 1e-12 of such stay finite
+  auto plain = [&](double v) { return v > -top && v < top; };
+  if (!plain(P.rho_w_ref) || !plain(P.rho_o_ref) || !plain(P.rho_g_ref)) return false;
+  for (int r = 0; r < P.pvt_rows; ++r) {
+    const double* a = pvt + (size_t)r * kPvtCols;
+    const double* before = r > 0 ? a - kPvtCols : nullptr;
+    if (!plain(a[0]) || (before && !(a[0] > before[0]))) return false;
+    for (int c : {C_BO, C_BW, C_BG, C_RS, C_RV}) {
+      if (!plain(a[c]) || (before && !plain((a[c] - before[c]) / (a[0] - before[0])))) return false;
+      if (c != C_RS && c != C_RV && a[c] < 0.0) return false;
+    }
+  }
+  return true;
 }
 
 // ---------------------------------------------------------------- host API
