@@ -272,51 +272,75 @@ namespace {
 // from): it holds the coarsest inverse, which stays float64 there too.
 constexpr double kOmega = 0.7;  // classical_amg.py:1022
 
-enum DnMode { DN_AX = 0, DN_RESID = 1, DN_SWEEP = 2, DN_ADD = 3 };
+enum DnMode { DN_AX = 0, DN_RESID = 1, DN_SWEEP = 2, DN_ADD = 3, DN_PLUS = 4 };
 
 // Epilogue of a product acc = (A X)(i, c):
-//  DN_AX: acc;  DN_RESID: I - acc;  DN_SWEEP: x + w (I - acc);  DN_ADD: y + acc
+//  DN_AX: acc;  DN_RESID: I - acc;  DN_SWEEP: x + w (I - acc);  DN_ADD: y + acc;
+//  DN_PLUS: x + acc
+// The kernels of a forming are one chain of programmatic launches (pdl_fence behind
+// it), so matrices that an earlier one writes carry no __restrict__.
 template <int MODE>
 __device__ __forceinline__ double dn_out(double acc, int i, int c, double w, const double* X, const double* Y,
                                          size_t at) {
   if (MODE == DN_RESID) return (i == c ? 1.0 : 0.0) - acc;
   if (MODE == DN_SWEEP) return X[at] + w * ((i == c ? 1.0 : 0.0) - acc);
   if (MODE == DN_ADD) return Y[at] + acc;
+  if (MODE == DN_PLUS) return X[at] + acc;
   return acc;
 }
 
 // Y = epilogue(A X) for a CSR matrix A of `rows` rows and a dense X of n
-// columns (row-major, leading dimension ld): a block takes one row of A and 256
-// columns, two a thread, so every gathered row of X is one contiguous segment.
+// columns (row-major, leading dimension ld): a warp takes 64 columns, two a lane,
+// so every gathered row of X is a contiguous segment.  32 entries of the row are
+// loaded at once and handed round by shuffles.  With W = 4 a block's warps share
+// one row and 64 columns, warp w taking entries w, w + 4, .. (their sums are
+// added in that order): rows of A and R are chains of loads, and some of a capped
+// hierarchy's hold half of the columns (748 rows of 25 entries on average, the
+// longest 406, and the 184 below them: 34 us a product with W = 1, 17 with W = 4).
+// Rows of P are short: W = 1, 256 columns a block (3.6 us, 7.9 with W = 4).
 // Bound by L2 (nnz n reads of 8 bytes): used while rows are short.
-template <typename TV, int MODE>
+template <typename TV, int MODE, int W>
 __global__ void __launch_bounds__(128) k_dn_spmm(int rows, int n, int ld, const int* __restrict__ rowptr,
                                                  const int* __restrict__ col, const TV* __restrict__ val,
-                                                 const TV* __restrict__ inv, const double* __restrict__ X,
-                                                 double* Y) {
-  const int i = blockIdx.x;
-  const int c = (blockIdx.y * 128 + threadIdx.x) * 2;
-  if (c >= n) return;
+                                                 const TV* __restrict__ inv, const double* X, double* Y) {
+  pdl_wait_release();
+  constexpr int U = 8;
+  __shared__ double2 part[3][32];
+  const int i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = ((blockIdx.y * (4 / W) + warp / W) * 32 + lane) * 2;
+  const double* Xc = X + min(c, ld - 2);              // (lanes past the last column load, and store nothing)
+  const int e0 = rowptr[i] + warp % W, e1 = rowptr[i + 1];
   double a0 = 0.0, a1 = 0.0;
-  const int e1 = rowptr[i + 1];
-  int e = rowptr[i];
-  for (; e + 4 <= e1; e += 4) {
-    double2 x[4];
-    double v[4];
+  for (int b = e0; b < e1; b += 32 * W) {             // 32 entries of this warp, one a lane
+    const int e = b + W * lane, have = min(32, (e1 - b + W - 1) / W);
+    const double v = e < e1 ? (double)val[e] : 0.0;
+    const int k = e < e1 ? col[e] : 0;
+    for (int q = 0; q < have; q += U) {
+      double2 x[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      v[u] = (double)val[e + u];
-      x[u] = *reinterpret_cast<const double2*>(X + (size_t)col[e + u] * ld + c);
+      for (int u = 0; u < U; ++u) {
+        const int kq = __shfl_sync(0xffffffffu, k, q + u);
+        x[u] = q + u < have ? *reinterpret_cast<const double2*>(Xc + (size_t)kq * ld) : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const double vq = __shfl_sync(0xffffffffu, v, q + u);
+        a0 += vq * x[u].x;
+        a1 += vq * x[u].y;
+      }
     }
+  }
+  if (W > 1) {
+    if (warp > 0) part[warp - 1][lane] = make_double2(a0, a1);
+    __syncthreads();
+    if (warp > 0) return;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) { a0 += v[u] * x[u].x; a1 += v[u] * x[u].y; }
+    for (int w = 0; w < 3; ++w) {
+      a0 += part[w][lane].x;
+      a1 += part[w][lane].y;
+    }
   }
-  for (; e < e1; ++e) {
-    const double v = (double)val[e];
-    const double2 x = *reinterpret_cast<const double2*>(X + (size_t)col[e] * ld + c);
-    a0 += v * x.x;
-    a1 += v * x.y;
-  }
+  if (c >= n) return;
   const size_t at = (size_t)i * ld + c;
   const double w = MODE == DN_SWEEP ? (double)(TV(kOmega) * inv[i]) : 0.0;
   double2 r;
@@ -326,81 +350,117 @@ __global__ void __launch_bounds__(128) k_dn_spmm(int rows, int n, int ld, const 
 }
 
 // Y = epilogue(A B), A M x K, B K x N, all row-major with leading dimension ld
-// (a multiple of 8): 64 x 64 tiles, 4 x 4 elements a thread, the next 16-deep
-// slice of A and B in registers while the current one is multiplied.  Bound by
-// the FP64 pipe.  DN_SWEEP reads its x from B (X = B there); w = kOmega inv.
+// (a multiple of 8), by FP64 matrix instructions (m8n8k4): 32 x 32 tiles of four
+// warps (2 x 2), 16-deep slices of A and B through a ring of three buffers
+// (cp.async), fragments read from rows padded by four doubles, which keeps the 16
+// lanes of a half warp on distinct banks.  Elements outside the matrices are taken
+// as zero, whatever the padding columns hold.  DN_SWEEP and DN_PLUS read their x
+// from B (X = B there); w = kOmega inv.
+// Bound by the FP64 pipe, and by whole tiles an SM: n = 638 24.7 us (21 TFLOP/s),
+// 771 47 us, 876 62 us; 64 x 64 tiles with four by four elements a thread took 61,
+// 128 and 139 us, bound by shared-memory reads, and 64 x 32 tiles of this kernel
+// 53 and 59 us at 771 and 876.
+constexpr int kGemmTile = 32, kGemmK = 16, kGemmStages = 3;
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int bytes) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(a), "l"(gmem), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
 template <typename TV, int MODE>
-__global__ void __launch_bounds__(256) k_dn_gemm(int M, int N, int K, int ld, const double* __restrict__ A,
-                                                 const double* __restrict__ B, const TV* __restrict__ inv, double* Y) {
-  constexpr int BM = 64, BN = 64, BK = 16;
-  __shared__ __align__(16) double As[2][BK][BM + 2];
-  __shared__ __align__(16) double Bs[2][BK][BN];
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+__global__ void __launch_bounds__(128) k_dn_gemm(int M, int N, int K, int ld, const double* A, const double* B,
+                                                 const TV* __restrict__ inv, double* Y) {
+  pdl_wait_release();
+  constexpr int BM = kGemmTile, BN = kGemmTile, BK = kGemmK, ST = kGemmStages, LA = BK + 4, LB = BN + 4;
+  constexpr int MT = BM / 16, NT = BN / 16;         // 8 x 8 tiles of a warp
+  __shared__ __align__(16) double As[ST][BM][LA];
+  __shared__ __align__(16) double Bs[ST][BK][LB];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  double ra[4], rb[4];
-  // A: rows m0 + t / 4 .. , four consecutive k a thread; B: row t / 16, four columns
-  auto load = [&](int k0) {
-    const int m = m0 + (t >> 2), ka = k0 + (t & 3) * 4;
+  auto fetch = [&](int st, int k0) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) ra[u] = (m < M && ka + u < K) ? A[(size_t)m * ld + ka + u] : 0.0;
-    const int kb = k0 + (t >> 4), nb = n0 + (t & 15) * 4;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) rb[u] = (kb < K && nb + u < N) ? B[(size_t)kb * ld + nb + u] : 0.0;
-  };
-  auto store = [&](int st) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) As[st][(t & 3) * 4 + u][t >> 2] = ra[u];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) Bs[st][t >> 4][(t & 15) * 4 + u] = rb[u];
-  };
-  double acc[4][4] = {};
-  load(0);
-  store(0);
-  __syncthreads();
-  int st = 0;
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    const bool more = k0 + BK < K;
-    if (more) load(k0 + BK);
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      double a[4], b[4];
-#pragma unroll
-      for (int u = 0; u < 4; u += 2) {
-        const double2 va = *reinterpret_cast<const double2*>(&As[st][k][ty * 4 + u]);
-        a[u] = va.x; a[u + 1] = va.y;
-        const double2 vb = *reinterpret_cast<const double2*>(&Bs[st][k][tx * 2 + 16 * u]);
-        b[u] = vb.x; b[u + 1] = vb.y;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] += a[u] * b[v];
+    for (int q = t; q < BM * BK / 2; q += 128) {
+      const int r = q / (BK / 2), k = (q % (BK / 2)) * 2;
+      const int have = m0 + r < M ? min(2, max(0, K - (k0 + k))) : 0;
+      cp_async16(&As[st][r][k], have ? A + (size_t)(m0 + r) * ld + k0 + k : A, 8 * have);
     }
-    if (more) store(st ^ 1);
-    __syncthreads();
-    st ^= 1;
-  }
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int i = m0 + ty * 4 + u;
+    for (int q = t; q < BK * BN / 2; q += 128) {
+      const int k = q / (BN / 2), c = (q % (BN / 2)) * 2;
+      const int have = k0 + k < K ? min(2, max(0, N - (n0 + c))) : 0;
+      cp_async16(&Bs[st][k][c], have ? B + (size_t)(k0 + k) * ld + n0 + c : B, 8 * have);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  double acc[MT][NT][2] = {};
+  const int steps = (K + BK - 1) / BK;
+#pragma unroll
+  for (int q = 0; q < ST - 1; ++q) fetch(q, q * BK);    // (past the end: zeros)
+  const int wm = (warp >> 1) * (BM / 2) + (lane >> 2), wn = (warp & 1) * (BN / 2) + (lane >> 2), kl = lane & 3;
+  for (int q = 0; q < steps; ++q) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2) : "memory");
+    __syncthreads();             // slice q is there, and everyone is done with the buffer filled next
+    fetch((q + ST - 1) % ST, (q + ST - 1) * BK);
+    const int st = q % ST;
+#pragma unroll
+    for (int k = 0; k < BK; k += 4) {
+      double a[MT], b[NT];
+#pragma unroll
+      for (int u = 0; u < MT; ++u) a[u] = As[st][wm + 8 * u][k + kl];
+#pragma unroll
+      for (int v = 0; v < NT; ++v) b[v] = Bs[st][k + kl][wn + 8 * v];
+#pragma unroll
+      for (int u = 0; u < MT; ++u)
+#pragma unroll
+        for (int v = 0; v < NT; ++v) mma_f64(acc[u][v][0], acc[u][v][1], a[u], b[v]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+#pragma unroll
+  for (int u = 0; u < MT; ++u) {
+    const int i = m0 + wm + 8 * u;
     if (i >= M) continue;
     const double w = MODE == DN_SWEEP ? (double)(TV(kOmega) * inv[i]) : 0.0;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = n0 + tx * 2 + 16 * (v & 2) + (v & 1);
-      if (c >= N) continue;
-      const size_t at = (size_t)i * ld + c;
-      Y[at] = dn_out<MODE>(acc[u][v], i, c, w, B, Y, at);
-    }
+    for (int v = 0; v < NT; ++v)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const int c = n0 + (warp & 1) * (BN / 2) + 8 * v + 2 * kl + x;
+        if (c >= N) continue;
+        const size_t at = (size_t)i * ld + c;
+        Y[at] = dn_out<MODE>(acc[u][v][x], i, c, w, B, Y, at);
+      }
   }
 }
 
-// X = diag(kOmega inv) (the first sweep from zero of every column)
+// What follows from A alone, one warp per row (each output may be null): X1 = W =
+// diag(kOmega inv), the first sweep from zero of every column; X2 = W + W (I - A W),
+// the second; R = I - A W, the residual after the first.
 template <typename TV>
-__global__ void k_dn_diag(int n, int ld, const TV* __restrict__ inv, double* __restrict__ X) {
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (size_t)n * ld; q += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(q / ld), c = (int)(q % ld);
-    X[q] = i == c ? (double)(TV(kOmega) * inv[i]) : 0.0;
+__global__ void __launch_bounds__(256) k_dn_first(int n, int ld, const int* __restrict__ rowptr,
+                                                  const int* __restrict__ col, const TV* __restrict__ val,
+                                                  const TV* __restrict__ inv, double* X1, double* X2, double* R) {
+  pdl_wait_release();
+  const int lane = threadIdx.x & 31;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+    const size_t at = (size_t)i * ld;
+    const double w = (double)(TV(kOmega) * inv[i]);
+    for (int j = lane; j < ld; j += 32) {             // (where A holds no entry, A W is 0)
+      const double d = i == j ? 1.0 : 0.0;
+      if (X1) X1[at + j] = d * w;
+      if (X2) X2[at + j] = d * w + w * d;
+      if (R) R[at + j] = d;
+    }
+    __syncwarp();
+    for (int e = rowptr[i] + lane; e < rowptr[i + 1]; e += 32) {
+      const int c = col[e];
+      const double r = (i == c ? 1.0 : 0.0) - (double)val[e] * (double)(TV(kOmega) * inv[c]);
+      if (X2) X2[at + c] = (i == c ? w : 0.0) + w * r;
+      if (R) R[at + c] = r;
+    }
   }
 }
 // dense copy of a CSR matrix, one warp per row
@@ -408,6 +468,7 @@ template <typename TV>
 __global__ void __launch_bounds__(256) k_dn_copy(int n, int ld, const int* __restrict__ rowptr,
                                                  const int* __restrict__ col, const TV* __restrict__ val,
                                                  double* __restrict__ M) {
+  pdl_wait_release();
   const int lane = threadIdx.x & 31;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
     double* m = M + (size_t)i * ld;
@@ -420,6 +481,7 @@ __global__ void __launch_bounds__(256) k_dn_copy(int n, int ld, const int* __res
 // Krylov mode the unpinned one unless it was singular (k_coarse_apply's choice)
 __global__ void k_dn_inverse(int n, int ld, const double* __restrict__ Apin, const double* __restrict__ Afree,
                              const int* __restrict__ free_singular, int krylov, double* __restrict__ E) {
+  pdl_wait_release();
   const bool use_free = krylov && *free_singular == 0;
   const double* A = use_free ? Afree : Apin;
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (size_t)n * ld; q += (size_t)gridDim.x * blockDim.x) {
@@ -427,18 +489,20 @@ __global__ void k_dn_inverse(int n, int ld, const double* __restrict__ Apin, con
     E[q] = (c < n && (use_free || c > 0)) ? A[(size_t)i * n + c] : 0.0;
   }
 }
-// out = I + a (+ b)
-__global__ void k_dn_one_plus(int n, int ld, const double* __restrict__ a, const double* __restrict__ b,
-                              double* __restrict__ out) {
+// sum = a + b, one = I + a + b
+__global__ void k_dn_terms(int n, int ld, const double* a, const double* b, double* sum, double* one) {
+  pdl_wait_release();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (size_t)n * ld; q += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(q / ld), c = (int)(q % ld);
-    out[q] = (i == c ? 1.0 : 0.0) + (b ? a[q] + b[q] : a[q]);
+    const double t = a[q] + b[q];
+    sum[q] = t;
+    one[q] = (i == c ? 1.0 : 0.0) + t;
   }
 }
 // E = diag(kOmega inv) T with column 0 (the pinned right-hand side) zero
 template <typename TV>
-__global__ void k_dn_scale_pin(int n, int ld, const TV* __restrict__ inv, const double* __restrict__ T,
-                               double* __restrict__ E) {
+__global__ void k_dn_scale_pin(int n, int ld, const TV* __restrict__ inv, const double* T, double* E) {
+  pdl_wait_release();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (size_t)n * ld; q += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(q / ld), c = (int)(q % ld);
     E[q] = (c > 0 && c < n) ? (double)(TV(kOmega) * inv[i]) * T[q] : 0.0;
@@ -446,7 +510,8 @@ __global__ void k_dn_scale_pin(int n, int ld, const TV* __restrict__ inv, const 
 }
 
 // the finished operator, its padding columns zero
-__global__ void k_dn_store(int n, int ld, const double* __restrict__ E, double* __restrict__ op) {
+__global__ void k_dn_store(int n, int ld, const double* E, double* op) {
+  pdl_wait_release();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (size_t)n * ld; q += (size_t)gridDim.x * blockDim.x)
     op[q] = (int)(q % ld) < n ? E[q] : 0.0;
 }
@@ -505,18 +570,29 @@ template <> struct DV<float> {
 struct Dense {
   int ld;
   cudaStream_t s;
-  unsigned ew(int n) const { return grid_for((size_t)n * ld, 256, 4); }
-  template <int MODE, typename TV = double>
-  void gemm(int M, int N, int K, const double* A, const double* B, double* Y, const TV* inv = nullptr) const {
-    k_dn_gemm<TV, MODE><<<dim3((N + 63) / 64, (M + 63) / 64), 256, 0, s>>>(M, N, K, ld, A, B, inv, Y);
-    count_launch();
+  // an elementwise kernel over n rows
+  template <typename... P, typename... A>
+  void each(void (*kernel)(int, int, P...), int n, A... args) const {
+    launch_pdl(kernel, grid_for((size_t)n * ld, 256, 4), 256, 0, s, n, ld, args...);
     IMPES_CHECK_LAUNCH();
   }
-  template <int MODE, typename TV>
+  template <typename TV>
+  void first(const Level& L, double* X1, double* X2, double* R) const {
+    launch_pdl(k_dn_first<TV>, (unsigned)((L.n + 7) / 8), 256, 0, s, L.n, ld, (const int*)L.rowptr.p,
+               (const int*)L.col.p, DV<TV>::val(L), DV<TV>::inv(L), X1, X2, R);
+    IMPES_CHECK_LAUNCH();
+  }
+  template <int MODE, typename TV = double>
+  void gemm(int M, int N, int K, const double* A, const double* B, double* Y, const TV* inv = nullptr) const {
+    launch_pdl(k_dn_gemm<TV, MODE>, dim3((N + kGemmTile - 1) / kGemmTile, (M + kGemmTile - 1) / kGemmTile), 128, 0, s,
+               M, N, K, ld, A, B, inv, Y);
+    IMPES_CHECK_LAUNCH();
+  }
+  template <int MODE, typename TV, int W = 4>
   void spmm(int rows, int n, const int* rp, const int* ci, const TV* v, const TV* inv, const double* X,
             double* Y) const {
-    k_dn_spmm<TV, MODE><<<dim3(rows, (n + 255) / 256), 128, 0, s>>>(rows, n, ld, rp, ci, v, inv, X, Y);
-    count_launch();
+    launch_pdl(k_dn_spmm<TV, MODE, W>, dim3(rows, (n + 256 / W - 1) / (256 / W)), 128, 0, s, rows, n, ld, rp, ci, v, inv,
+               X, Y);
     IMPES_CHECK_LAUNCH();
   }
   // Y = epilogue(A X) with the level's A (dense copy Ad when given)
@@ -548,39 +624,28 @@ void dense_form(AMG& h, int krylov, cudaStream_t s) {
     const Level& C = *h.levels.back();
     const int n = C.n;
     if (n <= 500) {
-      k_dn_inverse<<<d.ew(n), 256, 0, s>>>(n, ld, C.lu.p, C.lu_free.p, h.iflag.p + 3, krylov, w[0]);
-      count_launch();
+      d.each(k_dn_inverse, n, (const double*)C.lu.p, (const double*)C.lu_free.p, (const int*)(h.iflag.p + 3), krylov,
+             w[0]);
     } else {
-      // fifty sweeps from zero: W (I + H + ... + H^49), H = I - A W, by doubling
-      // the number of terms: S_2m = S_m + H^m S_m
-      double *H = w[1], *P = w[2], *S = w[3], *Q = w[4], *A = w[5];
-      k_dn_diag<TV><<<d.ew(n), 256, 0, s>>>(n, ld, DV<TV>::inv(C), P);
-      count_launch();
-      if (dense_products(C)) {
-        k_dn_copy<TV><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(n, ld, C.rowptr.p, C.col.p, DV<TV>::val(C), A);
-        count_launch();
-      }
-      d.product<DN_RESID, TV>(C, dense_products(C) ? A : nullptr, P, H);            // H
-      d.gemm<DN_AX>(n, n, n, H, H, P);                                        // H^2
-      k_dn_one_plus<<<d.ew(n), 256, 0, s>>>(n, ld, H, P, S);                  // S_3
-      count_launch();
-      d.gemm<DN_AX>(n, n, n, P, H, Q);                                        // H^3
-      for (int m = 3; m < 24; m *= 2) {
-        IMPES_CUDA(cudaMemcpyAsync(P, S, sz * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        d.gemm<DN_ADD>(n, n, n, Q, P, S);                                     // S_2m
-        d.gemm<DN_AX>(n, n, n, Q, Q, A);                                      // H^2m
-        std::swap(Q, A);
-      }
-      d.gemm<DN_AX>(n, n, n, H, S, P);
-      k_dn_one_plus<<<d.ew(n), 256, 0, s>>>(n, ld, P, nullptr, S);            // S_25 = I + H S_24
-      count_launch();
-      d.gemm<DN_AX>(n, n, n, Q, H, A);                                        // H^25
-      IMPES_CUDA(cudaMemcpyAsync(P, S, sz * sizeof(double), cudaMemcpyDeviceToDevice, s));
-      d.gemm<DN_ADD>(n, n, n, A, P, S);                                       // S_50
-      k_dn_scale_pin<TV><<<d.ew(n), 256, 0, s>>>(n, ld, DV<TV>::inv(C), S, w[0]);
-      count_launch();
+      // fifty sweeps from zero: W (I + H + ... + H^49), H = I - A W, in nine
+      // products as (I + H) s(H^2) s(H^10), s(X) = I + X + X^2 + X^3 + X^4
+      double *H = w[1], *P = w[2], *Q = w[3], *S = w[4], *T = w[5], *Z = w[0];
+      auto five = [&](const double* X, const double* X2, double* sum, double* out) {
+        d.each(k_dn_terms, n, X, X2, sum, out);
+        d.gemm<DN_ADD>(n, n, n, X2, sum, out);                // I + X + X^2 + X^2 (X + X^2)
+      };
+      d.first<TV>(C, nullptr, nullptr, H);
+      d.gemm<DN_AX>(n, n, n, H, H, P);                        // H^2
+      d.gemm<DN_AX>(n, n, n, P, P, Q);                        // H^4
+      five(P, Q, T, S);
+      d.gemm<DN_AX>(n, n, n, Q, Q, T);                        // H^8
+      d.gemm<DN_AX>(n, n, n, T, P, Z);                        // H^10
+      d.gemm<DN_AX>(n, n, n, Z, Z, P);                        // H^20
+      five(Z, P, T, Q);
+      d.gemm<DN_AX>(n, n, n, S, Q, T);
+      d.gemm<DN_PLUS>(n, n, n, H, T, P);
+      d.each(k_dn_scale_pin<TV>, n, DV<TV>::inv(C), (const double*)P, Z);
     }
-    IMPES_CHECK_LAUNCH();
   }
   // each level above it: sweeps on the identity, coarse correction, sweeps
   for (int l = (int)h.levels.size() - 2; l >= dl; --l) {
@@ -590,42 +655,49 @@ void dense_form(AMG& h, int krylov, cudaStream_t s) {
     double *E = w[0], *X = w[1], *Y = w[2], *C = w[3], *F = w[4], *A = nullptr;
     if (dense_products(L)) {
       A = w[5];
-      k_dn_copy<TV><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(n, ld, L.rowptr.p, L.col.p, DV<TV>::val(L), A);
-      count_launch();
+      launch_pdl(k_dn_copy<TV>, (unsigned)((n + 7) / 8), 256, 0, s, n, ld, (const int*)L.rowptr.p,
+                 (const int*)L.col.p, DV<TV>::val(L), A);
+      IMPES_CHECK_LAUNCH();
     }
-    k_dn_diag<TV><<<d.ew(n), 256, 0, s>>>(n, ld, DV<TV>::inv(L), X);
-    count_launch();
-    for (int q = 1; q < (light ? 1 : 3); ++q) {
-      d.product<DN_SWEEP, TV>(L, A, X, Y);
-      std::swap(X, Y);
+    if (light) {
+      d.first<TV>(L, X, nullptr, Y);
+    } else {
+      d.first<TV>(L, nullptr, Y, nullptr);
+      d.product<DN_SWEEP, TV>(L, A, Y, X);
+      d.product<DN_RESID, TV>(L, A, X, Y);
     }
-    d.product<DN_RESID, TV>(L, A, X, Y);
     d.spmm<DN_AX, TV>(nc, n, L.rrow.p, L.rcol.p, DV<TV>::rval(L), nullptr, Y, C);
     d.gemm<DN_AX>(nc, n, nc, E, C, F);
-    d.spmm<DN_ADD, TV>(n, n, L.prow.p, L.pcol.p, DV<TV>::pval(L), nullptr, F, X);
+    d.spmm<DN_ADD, TV, 1>(n, n, L.prow.p, L.pcol.p, DV<TV>::pval(L), nullptr, F, X);
     for (int q = 0; q < (light ? 1 : 2); ++q) {
       d.product<DN_SWEEP, TV>(L, A, X, Y);
       std::swap(X, Y);
     }
     std::swap(w[0], X == w[1] ? w[1] : w[2]);     // this level's operator is the next one's E
   }
-  k_dn_store<<<d.ew(Ld.n), 256, 0, s>>>(Ld.n, ld, w[0], op);
-  count_launch();
-  IMPES_CHECK_LAUNCH();
+  d.each(k_dn_store, Ld.n, (const double*)w[0], op);
+  pdl_fence(s);
 }
 
 }  // namespace
 
 // Levels dense_level and below become one operator: from the coarsest level up,
-// while a level has at most kDenseRows rows and its products on the identity
-// stay below kDenseFlops, so that forming it (at about 9 TFLOP/s) pays after
-// about ten V-cycles (an update is followed by ten to a hundred of them).  A
-// coarsest level of more than 500 rows is taken whatever it costs: it saves
-// fifty sweeps a V-cycle.  Measured against the per-level kernels (B200, all
-// update costs included): 64x64 two-phase step (663 rows down) 7.18 -> 5.67 ms,
-// black-oil 100x100x20 step (coarsest 665 rows) 105.0 -> 73.1 ms, 100 stand-alone
-// V-cycles of a 64x64x8 system (565 rows down) 20.1 -> 15.5 ms, mixed 1e6-cell
-// step (776 rows down, light sweeps) 72.8 -> 70.6 ms.
+// while a level has at most kDenseRows rows and its products with A on the identity
+// stay below kDenseFlops.  A coarsest level of more than 500 rows is taken up to
+// kDenseRows whatever its nine products cost (18 n^3: 4.7 GFLOP at 638 rows, 28 at
+// 1,152): it saves fifty sweeps a V-cycle.  Forming pays from the break-even number
+// of V-cycles after an update on (a solve takes ten to a hundred).  Measured, B200,
+// fp64: the operator's rows, time to form it, V-cycle level by level and with it:
+//   64x64x1 two-phase, 667:     179 us,  72 ->  38 us, break-even  5
+//   47x39x9 two-phase, 523:     318 us, 124 ->  77 us,  7
+//   64x64x8 two-phase, 565:     404 us, 153 -> 104 us,  8
+//   120x110x25 gas, capped, 748: 195 us, 316 -> 287 us, 7; light sweeps 109 us, 8
+//   coarsest of 638 rows, 459 a row:  330 us, 623 -> 489 us, 2.5
+//   coarsest of 947 rows, 544 a row:  756 us, 509 -> 379 us, 6
+//   coarsest of 771 / 1,035 / 1,113 rows, 14 a row: 508 / 902 / 1,072 us, 130 -> 26 us,
+//     5 / 9 / 11, so past kDenseRows a solve of ten V-cycles would lose
+// One to three V-cycles after each update cost up to that forming more than level by
+// level, on these sizes 0.1 to 1 ms.
 constexpr int kDenseRows = 1152;
 constexpr double kDenseFlops = 4e9;
 void amg_dense_setup(AMG& h) {
