@@ -197,6 +197,10 @@ int impes_amg_profile_levels(impes_amg* h, int precision, int reps, double* out_
  * (impes_step from the second FGMRES step on) and whether a capture was
  * refused, after which its steps stay host-driven. */
 int impes_amg_step_graphs(impes_amg* h, int* graphs, int* capture_refused);
+/* Instrumentation: the first of the coarse levels whose V-cycle is applied as one
+ * dense operator (-1: none), its rows, and the device memory that the operators
+ * and the work space for forming them hold. */
+int impes_amg_coarse_operator(impes_amg* h, int* level, int* rows, long long* bytes);
 /* Copy level `lvl` into caller device buffers (any pointer may be NULL). */
 int impes_amg_level_export(impes_amg* h, int lvl, int* A_rowptr, int* A_col, double* A_val,
                            double* inv_relax, int* P_rowptr, int* P_col, double* P_val,

@@ -207,7 +207,7 @@ bool step_graph_run(Model& m, AMG& a, double* p, double* sw, double* sg, double*
   IMPES_CUDA(cudaGraphLaunch(g->exec, s));
   a.fp64_stale = g->fp64_stale_after;
   a.dense_invalidate();
-  a.dense_valid[kp.precision == 1 ? 1 : 0][1] = a.dense_level >= 0;
+  a.dense_valid[kp.precision == 1 ? 1 : 0][a.dense_mode(true)] = a.dense_level >= 0;
   FgState* hs = reinterpret_cast<FgState*>(a.hbuf.p);
   static_assert(sizeof(FgState) <= 64 * sizeof(double), "state must fit the pinned scratch");
   IMPES_CUDA(cudaMemcpyAsync(hs, a.fgst.p, sizeof(FgState), cudaMemcpyDeviceToHost, s));
@@ -376,6 +376,16 @@ int impes_amg_step_graphs(impes_amg* h, int* graphs, int* capture_refused) {
     IMPES_REQUIRE(h && graphs && capture_refused, IMPES_ERR_ARG, "null argument");
     *graphs = (int)h->a.step_graphs.size();
     *capture_refused = h->a.step_graph_failed ? 1 : 0;
+  });
+}
+
+int impes_amg_coarse_operator(impes_amg* h, int* level, int* rows, long long* bytes) {
+  return guarded([&] {
+    IMPES_REQUIRE(h && level && rows && bytes, IMPES_ERR_ARG, "null argument");
+    const AMG& a = h->a;
+    *level = a.dense_level;
+    *rows = a.dense_level >= 0 ? a.levels[a.dense_level]->n : 0;
+    *bytes = (long long)a.dense_bytes();
   });
 }
 

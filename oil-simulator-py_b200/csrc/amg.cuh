@@ -166,7 +166,7 @@ struct AMG {
   bool use_tail = false;                // fused V-cycle tail (IMPES_TAIL=1: on)
   bool use_dia_tile = false;            // level-0 grid-tile sweeps (IMPES_DIA_TILE=1: on)
   // The V-cycle of levels dense_level and below as one dense operator (row-major,
-  // leading dimension dense_ld), per [fp32 values][Krylov mode]; valid while the
+  // leading dimension dense_ld), per [fp32 values][Krylov mode] (dense_mode); valid while the
   // values it was formed from are the hierarchy's (amg_dense.cu).  The flags are the
   // host's: they stand for kernels in stream order, so nothing recorded into a
   // graph of the caller's may set or rely on them.  V-cycles recorded there run
@@ -175,6 +175,14 @@ struct AMG {
   int dense_level = -1;                 // -1: none
   int dense_ld = 0;
   DBuf<double> dense_op[2][2], dense_work;
+  // the modes differ in the coarsest inverse they hold: one where that solve is sweeps
+  int dense_modes = 2;
+  int dense_mode(bool krylov) const { return krylov && dense_modes > 1 ? 1 : 0; }
+  size_t dense_bytes() const {
+    size_t b = dense_work.bytes();
+    for (auto& a : dense_op) b += a[0].bytes() + a[1].bytes();
+    return b;
+  }
   bool dense_valid[2][2] = {{false, false}, {false, false}};
   bool dense_off = false;
   void dense_invalidate() { for (auto& a : dense_valid) a[0] = a[1] = false; }

@@ -1794,7 +1794,8 @@ T* vcycle(AMG& h, int l, bool zero_x, cudaStream_t s, bool first_sweep_done = fa
 // Forms the coarse levels' dense operator where the values changed since.
 template <typename T>
 void dense_ensure(AMG& h, cudaStream_t s) {
-  if (h.dense_level >= 0 && !h.dense_valid[LV<T>::slot][h.krylov_mode]) amg_dense_form(h, LV<T>::slot, h.krylov_mode, s);
+  if (h.dense_level >= 0 && !h.dense_valid[LV<T>::slot][h.dense_mode(h.krylov_mode)])
+    amg_dense_form(h, LV<T>::slot, h.krylov_mode, s);
 }
 
 // One V-cycle from level 0 (input in LV<T>::b(L0), initial iterate in

@@ -607,7 +607,7 @@ struct Dense {
 // of 8 bytes from L2.
 inline bool dense_products(const Level& L) { return L.avg_row >= L.n / 6; }
 
-// Forms h.dense_op[slot][krylov] from the current values of the levels below and at
+// Forms h.dense_op[slot][dense_mode(krylov)] from the current values of the levels below and at
 // h.dense_level (fp64 ones or the fp32 chain's).
 template <typename TV>
 void dense_form(AMG& h, int krylov, cudaStream_t s) {
@@ -618,7 +618,7 @@ void dense_form(AMG& h, int krylov, cudaStream_t s) {
   const size_t sz = (size_t)Ld.n * ld;
   double* w[6];
   for (int q = 0; q < 6; ++q) w[q] = h.dense_work.p + q * sz;
-  double* op = h.dense_op[DV<TV>::slot][krylov].p;
+  double* op = h.dense_op[DV<TV>::slot][h.dense_mode(krylov != 0)].p;
   // the coarsest level's operator, in w[0]
   {
     const Level& C = *h.levels.back();
@@ -698,11 +698,23 @@ void dense_form(AMG& h, int krylov, cudaStream_t s) {
 //     5 / 9 / 11, so past kDenseRows a solve of ten V-cycles would lose
 // One to three V-cycles after each update cost up to that forming more than level by
 // level, on these sizes 0.1 to 1 ms.
+//
+// Six work matrices and the operators stay with the handle (7 to 10 n^2 doubles, 38 to
+// 106 MB at the largest sizes), since every update forms them again, from graphs too.
+// A program with many small hierarchies would run out of device memory by them, so
+// they are taken only while they are at most 1/kDenseShare of what is free; the
+// levels' own kernels serve otherwise.
+constexpr size_t kDenseShare = 64;
 constexpr int kDenseRows = 1152;
 constexpr double kDenseFlops = 4e9;
 void amg_dense_setup(AMG& h) {
   h.dense_level = -1;
   h.dense_invalidate();
+  auto release = [&] {
+    h.dense_work.release();
+    for (auto& a : h.dense_op) for (auto& b : a) b.release();
+  };
+  release();                                 // (of the hierarchy before)
   if (h.prm.smoother != IMPES_SMOOTHER_L1_JACOBI || h.tail_level >= 0 || h.stail_level >= 0) return;
   const Level& C = *h.levels.back();
   int dl = (int)h.levels.size() - 1;
@@ -715,26 +727,38 @@ void amg_dense_setup(AMG& h) {
   }
   const Level& D = *h.levels[dl];
   if (D.coarsest && D.n <= 500) return;      // already one product (k_coarse_apply)
+  const int ld = (D.n + 7) / 8 * 8;
+  const size_t sz = (size_t)D.n * ld;
+  const int modes = C.n > 500 ? 1 : 2, slots = h.prm.mixed_precision ? 2 : 1;
+  size_t free_b = 0, total_b = 0;
+  IMPES_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  if ((6 + (size_t)modes * slots) * sz * sizeof(double) > free_b / kDenseShare) return;
+  try {
+    h.dense_work.alloc(6 * sz);
+    for (int q = 0; q < slots; ++q)
+      for (int k = 0; k < modes; ++k) h.dense_op[q][k].alloc(sz);
+  } catch (const Error&) {                   // taken by someone else since
+    cudaGetLastError();
+    release();
+    return;
+  }
+  h.dense_modes = modes;
+  h.dense_ld = ld;
   h.dense_level = dl;
-  h.dense_ld = (D.n + 7) / 8 * 8;
-  const size_t sz = (size_t)D.n * h.dense_ld;
-  h.dense_work.ensure(6 * sz);
-  for (int q = 0; q < (h.prm.mixed_precision ? 2 : 1); ++q)
-    for (int k = 0; k < 2; ++k) h.dense_op[q][k].ensure(sz);
 }
 
 void amg_dense_form(AMG& h, int slot, bool krylov, cudaStream_t s) {
   if (h.dense_level < 0) return;
   if (slot == 0) dense_form<double>(h, krylov ? 1 : 0, s);
   else dense_form<float>(h, krylov ? 1 : 0, s);
-  if (!stream_capturing(s)) h.dense_valid[slot][krylov ? 1 : 0] = true;
+  if (!stream_capturing(s)) h.dense_valid[slot][h.dense_mode(krylov)] = true;
 }
 
 template <typename T>
 void dense_apply(const AMG& h, bool krylov, const T* b, T* x, cudaStream_t s) {
   const int n = h.levels[h.dense_level]->n;
   launch_pdl(k_dn_apply<T>, (n + 3) / 4, 128, h.dense_ld * sizeof(double), s, n, h.dense_ld,
-             (const double*)h.dense_op[sizeof(T) == 4][krylov ? 1 : 0].p, b, x);
+             (const double*)h.dense_op[sizeof(T) == 4][h.dense_mode(krylov)].p, b, x);
   IMPES_CHECK_LAUNCH();
 }
 template void dense_apply<double>(const AMG&, bool, const double*, double*, cudaStream_t);

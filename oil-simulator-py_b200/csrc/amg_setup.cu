@@ -2039,7 +2039,7 @@ namespace {
 // The operators of these values, behind an update that a caller records: its
 // replays change the values without the host's knowledge.
 void dense_form_recorded(AMG& h, int slot, cudaStream_t s) {
-  for (int krylov = 0; krylov < 2; ++krylov) amg_dense_form(h, slot, krylov != 0, s);
+  for (int krylov = 0; krylov < h.dense_modes; ++krylov) amg_dense_form(h, slot, krylov != 0, s);
 }
 }  // namespace
 

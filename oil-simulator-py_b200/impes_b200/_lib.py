@@ -136,6 +136,7 @@ _SIGNATURES = {
     "impes_amg_num_levels": ([_P, C.POINTER(_I)], _I),
     "impes_amg_level_info": ([_P, _I, C.POINTER(LevelDesc)], _I),
     "impes_amg_profile_levels": ([_P, _I, _I, C.POINTER(C.c_double), _P], _I),
+    "impes_amg_coarse_operator": ([_P, C.POINTER(_I), C.POINTER(_I), C.POINTER(C.c_longlong)], _I),
     "impes_amg_step_graphs": ([_P, C.POINTER(C.c_int), C.POINTER(C.c_int)], _I),
     "impes_amg_level_export": ([_P, _I, _P, _P, _P, _P, _P, _P, _P, _P], _I),
     "impes_amg_equilibration": ([_P, _P, C.POINTER(_I), _P], _I),

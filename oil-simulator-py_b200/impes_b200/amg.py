@@ -245,6 +245,14 @@ class ClassicalAMG:
         return self.Dhalf_inv is not None
 
     @property
+    def coarse_operator(self):
+        """(level, rows, bytes) of the dense operator that applies the V-cycle of the
+        coarse levels from ``level`` down, or None where every level runs by itself."""
+        level, rows, size = C.c_int(0), C.c_int(0), C.c_longlong(0)
+        check(lib.impes_amg_coarse_operator(self._h, C.byref(level), C.byref(rows), C.byref(size)))
+        return None if level.value < 0 else (level.value, rows.value, size.value)
+
+    @property
     def levels(self):
         """List of level dicts with keys A, n, P, inv_relax, diag, is_coarsest, and the
         column storage of the level's sweeps: col_index_bytes (2 or 4) and

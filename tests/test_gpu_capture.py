@@ -1,4 +1,6 @@
 """V-cycles and value updates captured into a caller's own CUDA graph act on the values of the replay."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -94,15 +96,25 @@ def test_capture_does_not_stand_for_running(monkeypatch, dims, precision, graphs
 @pytest.mark.parametrize("dims,precision", CASES)
 def test_failed_capture_leaves_the_solver_usable(dims, precision):
     """A solve cannot be captured (it reads its result on the host): the error leaves the handle as it was."""
+    from impes_b200 import _lib
     make, val, b = _system(dims, precision)
     amg = make()
     amg.fgmres(b, tol=1e-10, precision=precision)
     v = _scaled(val, 1.7)
     amg.update_values(v)
     torch.cuda.synchronize()
-    with pytest.raises(RuntimeError):
-        with torch.cuda.graph(torch.cuda.CUDAGraph(), capture_error_mode="thread_local"):
-            amg.fgmres(b, tol=1e-10, precision=precision)
+    # (by the runtime's own calls: a capture of torch's that fails leaves its allocator on the capture's pool)
+    rt = C.CDLL("libcudart.so.12")
+    side = torch.cuda.Stream()
+    graph = C.c_void_p()
+    assert rt.cudaStreamBeginCapture(C.c_void_p(side.cuda_stream), 2) == 0
+    try:
+        with torch.cuda.stream(side):
+            with pytest.raises(_lib.ImpesError):
+                amg.fgmres(b, tol=1e-10, precision=precision)
+    finally:
+        assert rt.cudaStreamEndCapture(C.c_void_p(side.cuda_stream), C.byref(graph)) != 0
+        rt.cudaGetLastError()
     torch.cuda.synchronize()
     x, st = amg.fgmres(b, tol=1e-10, precision=precision)
     ref = make()
