@@ -33,6 +33,13 @@ def _scaled(val, top):
     return val * torch.linspace(1.0, top, val.numel(), dtype=torch.float64, device=val.device)
 
 
+def _weakened(val):
+    # negative (off-diagonal) values by random factors: an M-matrix whose coarse levels differ from the first's
+    g = torch.Generator(device=val.device).manual_seed(3)
+    f = torch.rand(val.numel(), generator=g, dtype=torch.float64, device=val.device)
+    return torch.where(val < 0, val * f ** 4, val)
+
+
 def _capture(fn):
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g):
@@ -100,7 +107,7 @@ def test_failed_capture_leaves_the_solver_usable(dims, precision):
     make, val, b = _system(dims, precision)
     amg = make()
     amg.fgmres(b, tol=1e-10, precision=precision)
-    v = _scaled(val, 1.7)
+    v = _weakened(val)
     amg.update_values(v)
     torch.cuda.synchronize()
     # (by the runtime's own calls: a capture of torch's that fails leaves its allocator on the capture's pool)
