@@ -124,6 +124,7 @@ struct DBuf {
       cudaError_t e = cudaMalloc(&p, count * sizeof(T));
       if (e != cudaSuccess) {
         p = nullptr; n = 0;
+        cudaGetLastError();              // reported here, not by the next launch's check
         throw Error(IMPES_ERR_OOM, "cudaMalloc of " + std::to_string(count * sizeof(T)) + " bytes: " +
                                        cudaGetErrorString(e));
       }

@@ -51,3 +51,26 @@ def test_operator_gives_way_to_a_full_device(dims, levels, modes, mixed):
     assert float((x - xs).norm()) <= 1e-9 * float(x.norm())
     assert ss["converged"] and abs(ss["iterations"] - st["iterations"]) <= 1
     assert float((y - ys).norm()) <= 1e-7 * float(y.norm())
+
+
+def test_a_refused_allocation_is_reported_once():
+    """The call that finds no memory says so, and the calls after it work."""
+    from impes_b200 import _lib
+    from impes_b200.amg import ClassicalAMG
+    csr, b = _system(45, 45)
+    amg = ClassicalAMG(csr, coarsest_size=60)
+    x = amg.vcycle_scaled(b)
+    large, _ = _system(1000, 1000)             # its hierarchy takes more than the gigabyte left here
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - (1 << 30), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(_lib.ImpesError) as err:
+            ClassicalAMG(large, coarsest_size=60)
+        assert err.value.code == _lib.ERR_OOM
+        again = amg.vcycle_scaled(b)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert torch.equal(again, x)
+    _, st = amg.fgmres(b, tol=1e-10)
+    assert st["converged"]
