@@ -325,6 +325,12 @@ int impes_step(impes_model* m, impes_amg* amg, double* p, double* sw, double* sg
 int impes_pcg_solve(int n, const int* rowptr, const int* col, const double* val, const double* b,
                     double* x, double tol, int max_iter, int* iterations, int* converged,
                     double* rz, void* stream);
+/* The same with a limit of its own on the solve's waits: how often a wait of the
+ * grid-wide barrier looks before the solve gives up with IMPES_ERR_TIMEOUT
+ * (4,194,304, about a second, above; 0: the first wait runs out). */
+int impes_pcg_solve_bounded(int n, const int* rowptr, const int* col, const double* val,
+                            const double* b, double* x, double tol, int max_iter, int polls,
+                            int* iterations, int* converged, double* rz, void* stream);
 
 /* Running balances and per-well diagnostics (host outputs; syncs the stream). */
 int impes_model_balances(impes_model* m, impes_sat_stats* stats, void* stream);

@@ -24,9 +24,10 @@ bool impes_amg_handle_built(impes_amg* h) { return h && h->a.built; }
 impes::AMG* impes_amg_handle_core(impes_amg* h) { return &h->a; }
 
 namespace impes {
+constexpr int kPcgPolls = 4 << 20;       // looks of a barrier's wait, about a second
 void pcg_solve(int n, const int* rowptr, const int* col, const double* val, const double* b,
                double* x, double tol, int max_iter, int& iters, bool& converged, double& rs_out,
-               DBuf<double>& work, cudaStream_t s);
+               DBuf<double>& work, cudaStream_t s, int polls = kPcgPolls);
 void adjoint_check_model(const Model& m);
 int adjoint_num_producers(const Model& m);
 void adjoint_rates(Model& m, AMG& a, double* p, double* sw, int steps, double dt,
@@ -853,13 +854,20 @@ int impes_adjoint_gradient(impes_model* h, impes_amg* amg, const double* p0, con
 int impes_pcg_solve(int n, const int* rowptr, const int* col, const double* val, const double* b,
                     double* x, double tol, int max_iter, int* iterations, int* converged,
                     double* rz, void* stream) {
+  return impes_pcg_solve_bounded(n, rowptr, col, val, b, x, tol, max_iter, kPcgPolls, iterations, converged, rz, stream);
+}
+
+int impes_pcg_solve_bounded(int n, const int* rowptr, const int* col, const double* val, const double* b,
+                            double* x, double tol, int max_iter, int polls, int* iterations,
+                            int* converged, double* rz, void* stream) {
   return guarded([&] {
     IMPES_REQUIRE(rowptr && col && val && b && x, IMPES_ERR_ARG, "null argument");
+    IMPES_REQUIRE(polls >= 0, IMPES_ERR_ARG, "polls must not be negative");
     int it = 0;
     bool conv = false;
     double r = 0.0;
     DBuf<double> work;
-    pcg_solve(n, rowptr, col, val, b, x, tol, max_iter, it, conv, r, work, S(stream));
+    pcg_solve(n, rowptr, col, val, b, x, tol, max_iter, it, conv, r, work, S(stream), polls);
     if (iterations) *iterations = it;
     if (converged) *converged = conv ? 1 : 0;
     if (rz) *rz = r;

@@ -17,7 +17,6 @@ namespace {
 constexpr int TBP = 256;                 // rows of a partial sum
 constexpr int kBlocks = 296;             // 2 x 148 SMs: fixed partial count
 constexpr int kGrid = kBlocks / 2;       // CTAs of two such groups of threads
-constexpr int kSpinLimit = 4 << 20;      // polls of a barrier before it gives up (about a second)
 
 struct PcgOut {
   double rs;                             // last r . z
@@ -26,7 +25,7 @@ struct PcgOut {
 };
 
 // All CTAs of the (cooperative) grid; false when the wait gave up.
-__device__ bool grid_barrier(PcgOut* o, unsigned& target) {
+__device__ bool grid_barrier(PcgOut* o, unsigned& target, int polls) {
   __shared__ int s_ok;
   target += kGrid;
   __syncthreads();
@@ -34,7 +33,7 @@ __device__ bool grid_barrier(PcgOut* o, unsigned& target) {
     __threadfence();
     atomicAdd(&o->arrived, 1u);
     int ok = 0;
-    for (int q = 0; q < kSpinLimit; ++q) {
+    for (int q = 0; q < polls; ++q) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(&o->arrived) : "memory");
       if (v >= target) { ok = 1; break; }
@@ -83,7 +82,7 @@ __global__ void __launch_bounds__(2 * TBP) k_pcg(int n, const int* __restrict__ 
                                                  double* __restrict__ d, double* __restrict__ x,
                                                  double* __restrict__ r, double* z, double* pa, double* pb,
                                                  double* __restrict__ Ap, double* part, double tol, int max_iter,
-                                                 PcgOut* out) {
+                                                 int polls, PcgOut* out) {
   __shared__ double sh[2 * TBP / 32], sh_t;
   unsigned target = 0;
   const long long stride = (long long)kBlocks * TBP;
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(2 * TBP) k_pcg(int n, const int* __restrict__ 
     acc += rv * zv;
   }
   group_partial(acc, sh, part);
-  if (!grid_barrier(out, target)) return;
+  if (!grid_barrier(out, target, polls)) return;
   double rs = all_sum(part, &sh_t), beta = 0.0;
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
   int it = 0, conv = rs < 1e-10, nan = !(rs == rs);   // simulation.py:1680-1681
@@ -129,7 +128,7 @@ __global__ void __launch_bounds__(2 * TBP) k_pcg(int n, const int* __restrict__ 
       acc += pv * sum;
     }
     group_partial(acc, sh, part + kBlocks);
-    if (!grid_barrier(out, target)) return;
+    if (!grid_barrier(out, target, polls)) return;
     const double alpha = rs / all_sum(part + kBlocks, &sh_t);
     // x += alpha p, r -= alpha Ap, z = r / d and the partials of r . z
     acc = 0.0;
@@ -150,7 +149,7 @@ __global__ void __launch_bounds__(2 * TBP) k_pcg(int n, const int* __restrict__ 
       }
     }
     group_partial(acc, sh, part);
-    if (!grid_barrier(out, target)) return;
+    if (!grid_barrier(out, target, polls)) return;
     const double t = all_sum(part, &sh_t);
     beta = t / rs;
     rs = t;
@@ -172,10 +171,11 @@ __global__ void __launch_bounds__(2 * TBP) k_pcg(int n, const int* __restrict__ 
 
 // Solves A x = b (x written); returns the iterations taken and whether the
 // stopping test fired.  rs_out: the last r.z.  work: the solve's vectors, grown to
-// what this size needs.
+// what this size needs.  polls: how often a wait of the grid's barrier looks before it
+// gives up (the default is about a second); every CTA then returns.
 void pcg_solve(int n, const int* rowptr, const int* col, const double* val, const double* b,
                double* x, double tol, int max_iter, int& iters, bool& converged, double& rs_out,
-               DBuf<double>& work, cudaStream_t s) {
+               DBuf<double>& work, cudaStream_t s, int polls) {
   IMPES_REQUIRE(n > 0 && max_iter >= 0, IMPES_ERR_ARG, "pcg: bad size or iteration limit");
   const bool one = n <= kBlocks * TBP;
   const size_t nv = (size_t)n;
@@ -187,7 +187,7 @@ void pcg_solve(int n, const int* rowptr, const int* col, const double* val, cons
   double *pa = z + nv, *pb = pa + nv;
   double *d = one ? nullptr : pb + nv, *r = one ? nullptr : d + nv, *Ap = one ? nullptr : r + nv;
   IMPES_CUDA(cudaMemsetAsync(out, 0, sizeof(PcgOut), s));
-  void* args[] = {&n, &rowptr, &col, &val, &b, &d, &x, &r, &z, &pa, &pb, &Ap, &part, &tol, &max_iter, &out};
+  void* args[] = {&n, &rowptr, &col, &val, &b, &d, &x, &r, &z, &pa, &pb, &Ap, &part, &tol, &max_iter, &polls, &out};
   IMPES_CUDA(cudaLaunchCooperativeKernel(one ? (const void*)k_pcg<true> : (const void*)k_pcg<false>, dim3(kGrid),
                                          dim3(2 * TBP), args, 0, s));
   ::impes::count_launch();
