@@ -96,7 +96,6 @@ struct Level {
 // after the captured solve has run.
 struct FgState {
   int j, total, restarts, converged, done, cycle_end, reorth, bzero, nan;
-  int reorths;                          // second Gram-Schmidt passes taken
   int gs_count;                         // blocks of a Gram-Schmidt launch done (last block reduces)
   int max_iters;                        // limits of the solve (k_fg_params)
   double tol;
@@ -230,7 +229,6 @@ void amg_dense_form(AMG& h, int slot, bool krylov, cudaStream_t s);
 template <typename T>
 void dense_apply(const AMG& h, bool krylov, const T* b, T* x, cudaStream_t s);
 // amg_cycle.cu
-void amg_vcycle(AMG& h, int lvl, bool zero_x, int precision, cudaStream_t s);
 void amg_solve_vcycles(AMG& h, const double* b, double* x, double tol, int max_cycles,
                        int* cycles, double* rel, cudaStream_t s, int norm = IMPES_NORM_EQUILIBRATED);
 void amg_apply(AMG& h, const double* b, double* x, int cycles, double apply_tol,

@@ -28,12 +28,11 @@ namespace {
 constexpr int TB = 256;
 constexpr double kOmega = 0.7;  // classical_amg.py:1022
 
-enum CsrMode { Y_AX = 0, Y_B_MINUS_AX = 1, Y_SMOOTH = 2, Y_ADD_AX = 3, Y_SMOOTH0 = 4, Y_W_AX = 5 };
+enum CsrMode { Y_AX = 0, Y_B_MINUS_AX = 1, Y_SMOOTH = 2, Y_ADD_AX = 3, Y_SMOOTH0 = 4 };
 
 // One group of LPR lanes per row.  MODE selects the fused epilogue:
 //  Y_AX: y = A x;  Y_B_MINUS_AX: y = b - A x;  Y_SMOOTH: y = x + w*inv*(b - A x);
-//  Y_ADD_AX: y += A x (prolongation);  Y_SMOOTH0: y = w*inv*b (x = 0);
-//  Y_W_AX: y = wt .* (A x) (weighted operator of FGMRES, wt passed as inv).
+//  Y_ADD_AX: y += A x (prolongation);  Y_SMOOTH0: y = w*inv*b (x = 0).
 // CT is int, or unsigned short with the column of entry k at
 // col[k] + (rel ? row - 32768 : 0): plain 16-bit indices on levels of at most
 // 65536 rows, row-relative ones on larger levels whose bandwidth fits.
@@ -143,7 +142,6 @@ __global__ void __launch_bounds__(TB) k_csr(int n, const int* __restrict__ rowpt
       else if (MODE == Y_SMOOTH) y[row] = x[row] + T(kOmega) * inv[row] * (b[row] - acc);
       else if (MODE == Y_ADD_AX) y[row] = y[row] + acc;
       else if (MODE == Y_SMOOTH0) y[row] = T(kOmega) * inv[row] * b[row];
-      else if (MODE == Y_W_AX) y[row] = inv[row] * acc;
     }
   }
 }
@@ -185,7 +183,7 @@ __global__ void __launch_bounds__(TB) k_csr_early(int n, const int* __restrict__
     const bool out = lane == 0 && row < n;
     if (out) {
       if (MODE == Y_B_MINUS_AX || MODE == Y_SMOOTH || MODE == Y_SMOOTH0) bi = b[row];
-      if (MODE == Y_SMOOTH || MODE == Y_SMOOTH0 || MODE == Y_W_AX) wi = inv[row];
+      if (MODE == Y_SMOOTH || MODE == Y_SMOOTH0) wi = inv[row];
       if (MODE == Y_SMOOTH) xi = x[row];
       if (MODE == Y_ADD_AX) xi = y[row];
     }
@@ -202,7 +200,6 @@ __global__ void __launch_bounds__(TB) k_csr_early(int n, const int* __restrict__
       else if (MODE == Y_SMOOTH) y[row] = xi + T(kOmega) * wi * (bi - acc);
       else if (MODE == Y_ADD_AX) y[row] = xi + acc;
       else if (MODE == Y_SMOOTH0) y[row] = T(kOmega) * wi * bi;
-      else if (MODE == Y_W_AX) y[row] = wi * acc;
     }
     fetch(base + warps * RW + (threadIdx.x & 31) / LPR);
   }
@@ -247,7 +244,7 @@ __global__ void __launch_bounds__(TB, U == 4 ? 8 / (sizeof(T) / 4) : 1)
     T bi = T(0), wi = T(0), xi = T(0);
     if (out) {
       if (MODE == Y_B_MINUS_AX || MODE == Y_SMOOTH) bi = b[row];
-      if (MODE == Y_SMOOTH || MODE == Y_W_AX) wi = inv[row];
+      if (MODE == Y_SMOOTH) wi = inv[row];
       if (MODE == Y_SMOOTH) xi = x[row];
       if (MODE == Y_ADD_AX) xi = y[row];
     }
@@ -273,7 +270,6 @@ __global__ void __launch_bounds__(TB, U == 4 ? 8 / (sizeof(T) / 4) : 1)
       else if (MODE == Y_B_MINUS_AX) y[row] = bi - acc;
       else if (MODE == Y_SMOOTH) y[row] = xi + T(kOmega) * wi * (bi - acc);
       else if (MODE == Y_ADD_AX) y[row] = xi + acc;
-      else if (MODE == Y_W_AX) y[row] = wi * acc;
     }
     if (WPR > 1) __syncthreads();
     fetch(base + (long long)gridDim.x * kRows + grp);
@@ -360,7 +356,6 @@ __global__ void __launch_bounds__(TB) k_csr_stream(int n, const int* __restrict_
         else if (MODE == Y_B_MINUS_AX) y[row] = b[row] - acc;
         else if (MODE == Y_SMOOTH) y[row] = x[row] + float(kOmega) * inv[row] * (b[row] - acc);
         else if (MODE == Y_ADD_AX) y[row] = y[row] + acc;
-        else if (MODE == Y_W_AX) y[row] = inv[row] * acc;
       }
       acc = 0.0f;
     }
@@ -567,7 +562,6 @@ __global__ void __launch_bounds__(TB) k_sell(int n, int nslices, const int* __re
       else if (MODE == Y_B_MINUS_AX) y[row] = b[row] - acc;
       else if (MODE == Y_SMOOTH) y[row] = x[row] + T(kOmega) * inv[row] * (b[row] - acc);
       else if (MODE == Y_ADD_AX) y[row] = y[row] + acc;
-      else if (MODE == Y_W_AX) y[row] = inv[row] * acc;
     }
   }
 }
@@ -627,7 +621,6 @@ __global__ void __launch_bounds__(TB) k_dia(int n, int nd, DiaOffsets o, const T
     else if (MODE == Y_B_MINUS_AX) y[i] = b[i] - acc;
     else if (MODE == Y_SMOOTH) y[i] = x[i] + T(kOmega) * inv[i] * (b[i] - acc);
     else if (MODE == Y_ADD_AX) y[i] = y[i] + acc;
-    else if (MODE == Y_W_AX) y[i] = inv[i] * acc;
   }
 }
 // ND diagonals known at compile time (the 7-point stencil): every value and x
@@ -666,7 +659,6 @@ __global__ void __launch_bounds__(TB) k_dia_n(int n, DiaOffsets o, const T* __re
       else if (MODE == Y_B_MINUS_AX) y[i] = b[i] - acc;
       else if (MODE == Y_SMOOTH) y[i] = x[i] + T(kOmega) * inv[i] * (b[i] - acc);
       else if (MODE == Y_ADD_AX) y[i] = y[i] + acc;
-      else if (MODE == Y_W_AX) y[i] = inv[i] * acc;
     }
   }
 }
@@ -1009,34 +1001,21 @@ __device__ __forceinline__ double axpy_rows(double v, const double* __restrict__
 
 // ---------------------------------------------------- deterministic dots
 constexpr int kDotBlocks = 592;   // 4 x 148 SMs, fixed so partials have a fixed order
-constexpr int kMD = 8;            // vectors per multi-dot launch
 
-// partial[q * kDotBlocks + block] = sum over the block of V[q] . w   (q < k)
-__global__ void __launch_bounds__(TB) k_multidot(long long n, const double* __restrict__ Vbase,
-                                                 long long ldv, int k, const double* __restrict__ w,
-                                                 double* __restrict__ partial) {
+// partial[block] = sum over the block of a . b
+__global__ void __launch_bounds__(TB) k_dot(long long n, const double* __restrict__ a, const double* __restrict__ b,
+                                            double* __restrict__ partial) {
   pdl_wait_release();
-  __shared__ double s[kMD][TB / 32];
-  double acc[kMD];
-#pragma unroll
-  for (int q = 0; q < kMD; ++q) acc[q] = 0.0;
-  GRID_LOOP(i, n) {
-    const double wi = w[i];
-#pragma unroll
-    for (int q = 0; q < kMD; ++q)
-      if (q < k) acc[q] += Vbase[q * ldv + i] * wi;
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < kMD; ++q) {
-    double v = warp_sum(acc[q]);
-    if (lane == 0) s[q][wid] = v;
-  }
+  __shared__ double s[TB / 32];
+  double acc = 0.0;
+  GRID_LOOP(i, n) acc += a[i] * b[i];
+  acc = warp_sum(acc);
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
   __syncthreads();
-  if (threadIdx.x < kMD && threadIdx.x < k) {
+  if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int u = 0; u < TB / 32; ++u) t += s[threadIdx.x][u];
-    partial[threadIdx.x * kDotBlocks + blockIdx.x] = t;
+    for (int u = 0; u < TB / 32; ++u) t += s[u];
+    partial[blockIdx.x] = t;
   }
 }
 // out[0] = sum of partials, fixed order
@@ -1088,8 +1067,8 @@ void spmv(const Level& L, const double* x, double* y, cudaStream_t s) {
 }
 
 double dot_host(AMG& h, const double* a, const double* b, int n, cudaStream_t s) {
-  h.red.ensure((size_t)kMD * kDotBlocks);
-  launch_pdl(k_multidot, kDotBlocks, TB, 0, s, n, a, 0, 1, b, h.red.p);
+  h.red.ensure(kDotBlocks);
+  launch_pdl(k_dot, kDotBlocks, TB, 0, s, (long long)n, a, b, h.red.p);
   launch_pdl(k_dot_finalize, 1, 32, 0, s, (const double*)h.red.p, h.scal.p);
   IMPES_CHECK_LAUNCH();
   IMPES_CUDA(cudaMemcpyAsync(h.hbuf.p, h.scal.p, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -2420,7 +2399,7 @@ __global__ void k_fg_prec_smooth0(long long n, double* __restrict__ V, const dou
   }
 }
 // Z[j] = z (the preconditioner's output, widened exactly to fp64) and
-// V[j+1] = wt .* (A_s z), LPR lanes per row (the level-0 Y_W_AX product)
+// V[j+1] = wt .* (A_s z), LPR lanes per row
 template <typename XT, typename CT, int LPR>
 __global__ void __launch_bounds__(TB) k_fg_op(int n, const int* __restrict__ rowptr, const CT* __restrict__ col,
                                               const double* __restrict__ val, const XT* __restrict__ x,
@@ -2447,11 +2426,10 @@ __global__ void __launch_bounds__(TB) k_fg_op(int n, const int* __restrict__ row
   }
 }
 // Column j of the Hessenberg matrix, by one block of TB threads: h plus the second
-// pass's terms, h[j+1][j] = ||w||, then on thread 0 the Givens rotation
-// (k_givens) and the estimate |g[j+1]|; the counters, the inner loop's
-// condition and, at a cycle's end, y = R^-1 g column by column.  The column and
-// the rotations are staged in shared memory (sm: 5 * 128 doubles), so the serial
-// part waits on no global load.
+// pass's terms, h[j+1][j] = ||w||, then on thread 0 the Givens rotation and the
+// estimate |g[j+1]|; the counters, the inner loop's condition and, at a cycle's
+// end, y = R^-1 g column by column.  The column and the rotations are staged in
+// shared memory (sm: 5 * 128 doubles), so the serial part waits on no global load.
 __device__ void fg_column(double* H, int ldh, double* cs, double* sn, double* g, double* y, FgState* st, int m,
                           FgCond inner, double* sm) {
   double *hj = sm, *c_ = sm + 128, *s_ = c_ + 128, *gg = s_ + 128, *yy = gg + 128;
@@ -2699,7 +2677,6 @@ __global__ void __launch_bounds__(TB, 2) k_fg_gs(long long n, double* V, double*
         st->wn2 = t;
         if (PASS == 1) {
           st->reorth = t < 0.49 * H[(long long)j * ldh + k];
-          st->reorths += st->reorth;
         }
       }
     }
@@ -3226,7 +3203,7 @@ void solve_vcycles_noalloc(AMG& h, const double* b, double* x, double tol, int m
   const int n = L0.n;
   IMPES_REQUIRE(n <= kNoAllocMaxRows, IMPES_ERR_ARG,
                 "impes_amg_solve_vcycles_noalloc: n exceeds the 262144-row static work space");
-  IMPES_REQUIRE(h.red.n >= (size_t)kMD * kDotBlocks, IMPES_ERR_STATE, "hierarchy not set up");
+  IMPES_REQUIRE(h.red.n >= (size_t)kDotBlocks, IMPES_ERR_STATE, "hierarchy not set up");
   amg_ensure_fp64(h, s);
   double* base = solve_scratch();
   double* bs = base;
