@@ -269,6 +269,15 @@ __global__ void k_pattern(ModelParams P, int nnz, int* rowptr, int* col) {
   }
 }
 
+// Items that wells bring along are dealt over the blocks, then over a block's warps,
+// then over their lanes: items block, block + grid, .. of thread 0, of thread 32, ..
+// and so on, in steps of the launch.  On a large grid a warp has one at most (all of
+// them in one block were its critical path); a grid of one block has its 256 threads
+// work on them (one thread a block took 2.3 ms for 120 wells of a 16 x 16 model).
+__device__ __forceinline__ int dealt_first() {
+  return ((threadIdx.x & 31) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * gridDim.x + blockIdx.x;
+}
+
 // The kernels over cells take them in runs of kCells consecutive ones, a thread
 // each; wells are looked up only in a run that holds a well's cell.
 constexpr int kCells = 256;
@@ -635,7 +644,7 @@ __device__ __noinline__ void well_source(const ModelParams& P, const PvtSmem& T,
 
 // K4a: fluxes, divergence, dS and the substep ratio (simulation.py:968-1042, 1351-1379).
 // K4a': water and gas mobilities and densities and the oil-gas capillary pressure
-// of every cell, at the new pressure; one thread a block also forms a well's terms.
+// of every cell, at the new pressure; and the wells' terms.
 __global__ void __launch_bounds__(kCells, 4) k_flux_props(
     ModelParams P, const double* __restrict__ pvt_g, const double* __restrict__ p, const double* __restrict__ sw,
     const double* __restrict__ sg, const double* __restrict__ pv, double dt, double* __restrict__ mw,
@@ -646,9 +655,8 @@ __global__ void __launch_bounds__(kCells, 4) k_flux_props(
   __shared__ double s_slope[(kPvtCols - 1) * kMaxPvtRows];
   PvtSmem T{P.pvt_rows, s_col, s_slope};
   if (P.pvt_rows > 0) pvt_stage(pvt_g, P.pvt_rows, s_col, s_slope);
-  // (all wells in one block were its critical path: 47 us against 32)
-  if (threadIdx.x == 0)
-    for (int w = blockIdx.x; w < P.nwells; w += gridDim.x) well_source(P, T, A, w, p, sw, sg, pv, dt);
+  for (int w = dealt_first(); w < P.nwells; w += blockDim.x * gridDim.x)
+    well_source(P, T, A, w, p, sw, sg, pv, dt);
   const bool grav = (P.dz > 0) && (P.nz > 1);
   for (int c = blockIdx.x * kCells + threadIdx.x; c < P.N; c += gridDim.x * kCells) {
     const double p_ = p[c], swc = sw[c], sgc = sg[c];
@@ -905,12 +913,8 @@ __global__ void __launch_bounds__(kSatBlock, 4) k_saturation_substeps(
   const int N = *nsub;
   const double so_r = P.so_r;
   double acc[6] = {0, 0, 0, 0, 0, 0};  // water in/out, oil in/out, gas in/out
-  // the wells' replay items, a warp's first thread each, spread over the blocks
-  // (one block replaying them all was the kernel's critical path: 64 us against 42)
   const int items = P.pvt_rows > 0 ? N * P.nwells : 0;
-  if ((threadIdx.x & 31) == 0)
-    for (int it = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; it < items; it += (kSatBlock / 32) * gridDim.x)
-      well_replay(P, T, A, it, N, p_new, dt, contrib);
+  for (int it = dealt_first(); it < items; it += blockDim.x * gridDim.x) well_replay(P, T, A, it, N, p_new, dt, contrib);
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < P.N;
        c += (long long)gridDim.x * blockDim.x) {
     const double sw0 = sw[c], sg0 = sg[c];
@@ -963,19 +967,27 @@ __global__ void __launch_bounds__(kSatBlock, 4) k_saturation_substeps(
     __shared__ double s_bal[4];
     const int wq = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (wq < 4) {
+      constexpr int U = 8;             // loads in flight
       double t = 0.0;
-      for (int it = lane; it < items; it += 32) {
-        const double v = __ldcg(contrib + 4 * (size_t)it + wq);
-        if (!(v < 0.0)) t += v;        // NaN propagates
+      for (int it = lane; it < items; it += 32 * U) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = it + 32 * u < items ? __ldcg(contrib + 4 * (size_t)(it + 32 * u) + wq) : -1.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (!(v[u] < 0.0)) t += v[u];  // NaN propagates
       }
       t = warp_sum(t);
-      if (lane == 0) {
-        const int bit = wq == 0 ? 8 : wq == 1 ? 16 : wq == 2 ? 32 : 64;
-        double v = bal[6 + (wq < 2 ? wq : wq + 1)];
-        for (int w = 0; w < P.nwells; ++w)
-          if (A.terms[w].mask & bit) v += A.terms[w].b[wq];
-        s_bal[wq] = v + t;
+      const int bit = wq == 0 ? 8 : wq == 1 ? 16 : wq == 2 ? 32 : 64;
+      double v = bal[6 + (wq < 2 ? wq : wq + 1)];
+      for (int w0 = 0; w0 < P.nwells; w0 += 32) {   // 32 wells loaded at once, added one after another
+        const int w = w0 + lane;
+        const bool on = w < P.nwells && (A.terms[w].mask & bit);
+        const double mine = on ? A.terms[w].b[wq] : 0.0;
+        for (unsigned m = __ballot_sync(0xffffffffu, on); m; m &= m - 1)
+          v += __shfl_sync(0xffffffffu, mine, __ffs(m) - 1);
       }
+      if (lane == 0) s_bal[wq] = v + t;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
