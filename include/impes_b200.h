@@ -154,9 +154,10 @@ int impes_amg_solve_vcycles(impes_amg* h, const double* b, double* x, double tol
  * device memory during a solve -- for example a host that reserves the GPU's
  * memory up front for its own pool, or one that cannot afford the device-wide
  * synchronisation that cudaFree implies.  (No counterpart in the reference.)
- * impes_amg_solve_vcycles allocates and frees three n-vectors on every call;
- * this variant keeps them in a 6 MiB static device array instead and makes no
- * allocation, so n is limited to 262144 rows (larger n returns IMPES_ERR_ARG).
+ * impes_amg_solve_vcycles allocates three n-vectors on its first call, which the
+ * handle keeps; this variant has them in a 6 MiB static device array instead and
+ * makes no allocation, so n is limited to 262144 rows (larger n returns
+ * IMPES_ERR_ARG).
  * Every GPU that loads the library holds that array until the process exits.
  * Every call on a device shares it: calls that overlap on the GPU (several
  * streams or threads) race, so serialise them.  Nothing in the array needs to
@@ -173,7 +174,12 @@ int impes_amg_solve_vcycles_noalloc(impes_amg* h, const double* b, double* x, do
 int impes_amg_apply(impes_amg* h, const double* b, double* x, int cycles, double apply_tol,
                     int apply_max_cycles, void* stream);
 
-/* One V-cycle on the equilibrated system: x = V(0, b_s) (classical_amg.py:1037). */
+/* One V-cycle on the equilibrated system: x = V(0, b_s) (classical_amg.py:1037).
+ * Asynchronous; on a capturing stream it is recorded as plain launches that act
+ * on the values the hierarchy has at each replay.  impes_amg_update can be
+ * recorded too (a mixed hierarchy's fp64 levels then follow at the first fp64
+ * call the host makes after the recording); the solves cannot, since they read
+ * their result on the host. */
 int impes_amg_vcycle_scaled(impes_amg* h, const double* b_scaled, double* x_scaled,
                             int precision, void* stream);
 
@@ -326,8 +332,8 @@ int impes_pcg_solve(int n, const int* rowptr, const int* col, const double* val,
                     double* x, double tol, int max_iter, int* iterations, int* converged,
                     double* rz, void* stream);
 /* The same with a limit of its own on the solve's waits: how often a wait of the
- * grid-wide barrier looks before the solve gives up with IMPES_ERR_TIMEOUT
- * (4,194,304, about a second, above; 0: the first wait runs out). */
+ * grid-wide barrier looks, in steps of 1,024, before the solve gives up with
+ * IMPES_ERR_TIMEOUT (4,194,304, about a second, above; 0: the first wait runs out). */
 int impes_pcg_solve_bounded(int n, const int* rowptr, const int* col, const double* val,
                             const double* b, double* x, double tol, int max_iter, int polls,
                             int* iterations, int* converged, double* rz, void* stream);
