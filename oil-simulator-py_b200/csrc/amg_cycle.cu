@@ -2497,8 +2497,9 @@ __device__ void fg_column(double* H, int ldh, double* cs, double* sn, double* g,
 // parts of V h in shared memory; the dots stay in registers over the block's
 // tiles.  The last block to finish sums the blocks' partials in block order.
 //
-// Bound by HBM, (j + 2) n 8 bytes a launch: at n = 1e6 and 60 vectors passes 0
-// and 1 take 91 and 105 us (5.4 and 4.7 TB/s of 6.45 measured).  A thread per
+// Bound by HBM, (j + 2) n 8 bytes a launch and n 8 more where w is written: at
+// n = 1e6 and 59 vectors the passes take 93, 121 and 110 us (5.2, 4.0 and 4.4 TB/s
+// of 6.45 measured), at n = 330,000 44, 63 and 55 us (3.6, 2.6 and 2.9).  A thread per
 // element with eight vectors' loads in flight read the basis four times at
 // 3.6 TB/s; tiles in shared memory (cp.async, two buffers) took 57 / 83 us a
 // pass at 30 vectors, their update bound by shared-memory reads.

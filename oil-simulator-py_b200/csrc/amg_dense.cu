@@ -54,9 +54,11 @@ __global__ void __launch_bounds__(256) k_dense_pair(int n, const int* __restrict
 // that hold them), and the owner of column k + 1 publishes it.  Two block
 // barriers a step (one of them the cluster's when CL > 1).  Each element gets
 // the operations of the textbook in-place elimination with row swaps, in that
-// order.  Measured (B200, both matrices): 110 rows 922 -> 226 us, 124 rows 1169
-// -> 252 us against a one-CTA elimination in shared memory with four barriers a
-// step; about 200 rows 1462 -> 404 us against one in global memory.
+// order.  Measured (B200, both matrices): 32 / 64 / 96 rows 18 / 54 / 121 us, 110
+// rows 922 -> 226 us and 124 rows 1169 -> 251 us against a one-CTA elimination in
+// shared memory with four barriers a step; in clusters, 200 / 256 rows 486 / 627 us
+// (2.4 us a step), 300 / 500 rows 1.33 / 2.33 ms (4.5 us), a matrix in global memory
+// having taken 28 ms at 431 rows.
 struct GJArgs {
   double* M[2];
   int* singular[2];
@@ -208,7 +210,9 @@ void launch_gj(int n, const GJArgs& args, cudaStream_t s) {
 }  // namespace
 
 // Sixteen CTAs need that many free SMs in one GPC, which a part of a GPU may not
-// have; IMPES_COARSE_CLUSTER=8 asks for the narrow form (read at setup).
+// have; IMPES_COARSE_CLUSTER=8 asks for the narrow form (read at setup).  That one
+// holds 32 doubles a thread, most of them in local memory: 9.5 / 15.9 ms at 300 / 500
+// rows.
 int coarse_cluster_size() {
   const char* ev = getenv("IMPES_COARSE_CLUSTER");
   if (ev && atoi(ev) == 8) return 8;
@@ -246,9 +250,8 @@ void coarse_factor(AMG& h, Level& L, cudaStream_t s, bool from_fp32) {
   IMPES_CHECK_LAUNCH();
   IMPES_CUDA(cudaMemsetAsync(h.iflag.p + 2, 0, 2 * sizeof(int), s));
   const GJArgs args{{L.lu.p, L.lu_free.p}, {h.iflag.p + 2, h.iflag.p + 3}};
-  // one CTA while 128 columns fit its registers (16 doubles a thread), then 32
-  // columns a CTA in a cluster of 8 or 16 (2.1 us a pivot step in one CTA, about
-  // as much in a cluster of 8)
+  // one CTA while 128 columns fit its registers (16 doubles a thread: 2.0 us a pivot
+  // step), then 32 columns a CTA in a cluster of 8 (2.4 us) or 16 (4.5 us)
   if (n <= 32) launch_gj<1, 1, 8, 4>(n, args, s);
   else if (n <= 64) launch_gj<1, 2, 8, 8>(n, args, s);
   else if (n <= 96) launch_gj<1, 3, 8, 12>(n, args, s);
@@ -699,8 +702,8 @@ void dense_form(AMG& h, int krylov, cudaStream_t s) {
 // One to three V-cycles after each update cost up to that forming more than level by
 // level, on these sizes 0.1 to 1 ms.
 //
-// Six work matrices and the operators stay with the handle (7 to 10 n^2 doubles, 38 to
-// 106 MB at the largest sizes), since every update forms them again, from graphs too.
+// Six work matrices and the operators stay with the handle (7 to 10 n^2 doubles: 33 MB at
+// 771 rows, up to 106 MB at 1,152), since every update forms them again, from graphs too.
 // A program with many small hierarchies would run out of device memory by them, so
 // they are taken only while they are at most 1/kDenseShare of what is free; the
 // levels' own kernels serve otherwise.

@@ -51,8 +51,8 @@ void allow_wide_cluster(const void* kernel);
 
 // ------------------------------------------------------------------- arena
 // Device memory of one handle (an AMG hierarchy, a model), taken from the driver
-// in chunks and handed out in 512-byte pieces: building a hierarchy makes some
-// 750 allocations, at 25-80 us each from the driver (60 of 71 ms at 16,497 rows).
+// in chunks and handed out in 512-byte pieces: building a hierarchy of 16,497 rows
+// allocates and frees 789 times, 54 ms when each is the driver's.
 // While a Scope is open on a thread, DBufs of at most kPieceMax bytes allocated
 // there come from its arena; larger ones, and all others, from the driver.  A
 // piece given back is handed out again without waiting for the device, so one
