@@ -177,9 +177,9 @@ int impes_amg_apply(impes_amg* h, const double* b, double* x, int cycles, double
 /* One V-cycle on the equilibrated system: x = V(0, b_s) (classical_amg.py:1037).
  * Asynchronous; on a capturing stream it is recorded as plain launches that act
  * on the values the hierarchy has at each replay.  impes_amg_update can be
- * recorded too (a mixed hierarchy's fp64 levels then follow at the first fp64
- * call the host makes after the recording); the solves cannot, since they read
- * their result on the host. */
+ * recorded too (a mixed hierarchy then rebuilds its fp64 levels at every fp64
+ * call the host makes); the solves cannot, since they read their result on the
+ * host. */
 int impes_amg_vcycle_scaled(impes_amg* h, const double* b_scaled, double* x_scaled,
                             int precision, void* stream);
 

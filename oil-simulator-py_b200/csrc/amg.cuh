@@ -111,6 +111,7 @@ struct AMG {
   // mixed AMG: update_matrix runs the Galerkin chain in fp32 (all the V-cycle
   // of the mixed path reads); the fp64 coarse levels are rebuilt on demand
   bool fp64_stale = false;
+  bool fp64_unknown = false;       // a recorded update may have run since: rebuild at every fp64 call
   DBuf<double> dhalf_inv;          // D^-1/2 when equilibrated
   DBuf<double> jac_w;              // Jacobi weights in the scaled space
   DBuf<double> diag_tmp;

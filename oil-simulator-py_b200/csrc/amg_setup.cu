@@ -1687,6 +1687,7 @@ void amg_setup(AMG& h, int n, int nnz, const int* rowptr, const int* col, const 
   h.dense_invalidate();
   h.built = false;
   h.fp64_stale = false;
+  h.fp64_unknown = false;
   h.iflag.ensure(8);
   h.red.ensure(4096);
   h.scal.ensure(256);
@@ -2020,7 +2021,7 @@ void update_fp32_chain(AMG& h, cudaStream_t s) {
 }
 
 void amg_ensure_fp64(AMG& h, cudaStream_t s) {
-  if (!h.fp64_stale) return;
+  if (!h.fp64_stale && !h.fp64_unknown) return;
   for (size_t l = 0; l < h.levels.size(); ++l) {
     Level& L = *h.levels[l];
     compute_inv_relax(h, L, s);
@@ -2058,7 +2059,10 @@ void amg_update(AMG& h, const double* val, cudaStream_t s, bool own_graph) {
   equilibrate_level0(h, val, s);
   if (h.prm.mixed_precision && all_planned && h.levels.size() > 1) {
     update_fp32_chain(h, s);
-    if (recorded) dense_form_recorded(h, 1, s);
+    if (recorded) {
+      dense_form_recorded(h, 1, s);
+      h.fp64_unknown = true;
+    }
     timers().end(tid, s, bytes * 0.6);   // 4-byte values instead of 8
     return;
   }

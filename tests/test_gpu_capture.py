@@ -173,3 +173,9 @@ def test_captured_mixed_update_reaches_the_next_fp64_call():
     torch.cuda.synchronize()
     _capture(lambda: amg.vcycle_scaled(b, precision="fp64"))
     assert _close(amg.vcycle_scaled(b, precision="fp64"), _fresh(make, v, b, "fp64"), "fp64")
+    for top in (0.4, 2.5):          # and at every later replay
+        v = _scaled(val, top)
+        buf.copy_(v)
+        g.replay()
+        assert _close(amg.vcycle_scaled(b, precision="fp64"), _fresh(make, v, b, "fp64"), "fp64")
+        assert _close(amg.vcycle_scaled(b, precision="mixed"), _fresh(make, v, b, "mixed"), "mixed")
